@@ -46,6 +46,7 @@ struct DevStats {
   unsigned int nrank_dense;               // re-sort: source cells left to k_rank_dense
   unsigned int vmax_lo_bits[3];           // coarse kick: max of certified lower bounds of |v + vfield|
   unsigned long long pp_active;           // PP prefilter: particles with a neighbour besides themselves
+  double sums[3];                         // update_x: the sigma_v sums (update_particle.f90:172-196)
 };
 
 // share of the last step's vmax above which the coarse kick evaluates a

@@ -14,6 +14,7 @@
 //                       frame's visit order, assign ranks, accumulate vfield;
 //   scan                new spine (cell starts);
 //   U3 (per particle)   write the re-encoded particle at start+rank.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -765,7 +766,10 @@ __device__ __forceinline__ void ff_add(float& hi, float& lo, float x, float xlo)
 }
 
 // sigma_v sums of the new state (update_particle.f90:172-196): per-block FP64
-// partials in a fixed partition, summed in block order on the host.
+// partials in a fixed partition, summed in a fixed order by k_sigma_final.
+// Each block ends in FP64 shuffles on the narrow FP64 pipe, so small states
+// take fewer blocks (sigma_blocks): 2048 blocks for every size took 27 us for
+// 64^3 particles, 10 us with a block per 1024.
 __global__ void k_sigma(const void* __restrict__ vp, const int32_t* __restrict__ pcell, const float* __restrict__ vfield,
                         int64_t np, int64_t ncells, const float2* __restrict__ dech, int nvbin, int izipv,
                         double* __restrict__ part) {
@@ -815,14 +819,31 @@ __global__ void k_sigma(const void* __restrict__ vp, const int32_t* __restrict__
   }
 }
 
-// graph mode: sigma_vi_new from the block partials on the device, with the
-// host path's arithmetic (the same summation order, correctly rounded sqrt
-// and division), its vcoef for the encode estimate, and the sums for the host
-__global__ void k_sigma_final(const double* __restrict__ part, int nb, double npg, StepDev* sd, StepOut* so) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+// The sums over the block partials: thread t adds partials t, t + 256, ...,
+// the warps' lanes and then the warps' sums are added in order.  One thread
+// adding all 3 x 2048 from global memory took 364 us, most of a small box's
+// step in a captured graph; 3.7 us this way.  In graph mode (sd set) also
+// sigma_vi_new with the host path's arithmetic (correctly rounded sqrt and
+// division) and its vcoef for the encode estimate.
+constexpr int SF_THREADS = 256;
+__global__ void __launch_bounds__(SF_THREADS) k_sigma_final(const double* __restrict__ part, int nb, DevStats* st,
+                                                            double npg, StepDev* sd, StepOut* so) {
+  __shared__ double w[3][SF_THREADS / 32];
   double s[3] = {0.0, 0.0, 0.0};
-  for (int b = 0; b < nb; b++)
+  for (int b = threadIdx.x; b < nb; b += SF_THREADS)
     for (int t = 0; t < 3; t++) s[t] += part[3 * b + t];
+  for (int t = 0; t < 3; t++) {
+    for (int o = 16; o > 0; o >>= 1) s[t] += __shfl_xor_sync(0xffffffffu, s[t], o);
+    if ((threadIdx.x & 31) == 0) w[t][threadIdx.x >> 5] = s[t];
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int t = 0; t < 3; t++) {
+    s[t] = 0.0;
+    for (int i = 0; i < SF_THREADS / 32; i++) s[t] += w[t][i];
+    st->sums[t] = s[t];
+  }
+  if (!sd) return;
   const double std_res = sqrt(s[1] / npg);
   const float sn = (float)(std_res / (double)sqrtf(3.0f));  // update_particle.f90:224
   sd->sigma_new = sn;
@@ -831,6 +852,11 @@ __global__ void k_sigma_final(const double* __restrict__ part, int nb, double np
     for (int t = 0; t < 3; t++) so->sums[t] = s[t];
     so->sigma_new = sn;
   }
+}
+
+int sigma_blocks(const cube_ctx* c, int64_t np) {
+  const int64_t n = (std::max(np, c->ncells) + 1023) / 1024;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(n, c->red_blocks));
 }
 
 }  // namespace
@@ -898,11 +924,11 @@ static int update_x_graph(cube_ctx* c) {
   k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 16), 128, 0, s>>>(a);
   k_scatter<<<cube_grid(c->np, B), B, 0, s>>>(a);
   k_scatter_xtra<<<cube_grid(c->xtra_cap, B, 2), B, 0, s>>>(a);
-  const int nb = c->red_blocks;
+  const int nb = sigma_blocks(c, c->np);
   k_sigma<<<nb, 256, 0, s>>>(c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, cv.dech, c->nvbin, c->p.izipv,
                              c->red_tmp);
   const double npg = (double)(c->npglobal > 0 ? c->npglobal : c->np);
-  k_sigma_final<<<1, 32, 0, s>>>(c->red_tmp, nb, npg, c->sd, c->sout);
+  k_sigma_final<<<1, SF_THREADS, 0, s>>>(c->red_tmp, nb, c->dstats, npg, c->sd, c->sout);
   CUBE_CUDA(c, cudaGetLastError());
   CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->upd, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, s));
   r = cube_codec_build_dev(c, 1, &c->sd->sigma_new);
@@ -1071,22 +1097,18 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   cube_phase_end(c, PH_UPD_SCATTER);
   CUBE_CUDA(c, cudaGetLastError());
   // sigma statistics of the new state (decoded with sigma_vi)
-  int nb = c->red_blocks;
+  const int nb = sigma_blocks(c, np_new);
   cube_phase_begin(c, PH_UPD_SIGMA);
   k_sigma<<<nb, 256, 0, c->stream>>>(c->vp[kn], c->pcell[kn], c->vfield[kn], np_new, c->ncells, cv.dech,
                                       c->nvbin, c->p.izipv, c->red_tmp);
+  k_sigma_final<<<1, SF_THREADS, 0, c->stream>>>(c->red_tmp, nb, c->dstats, 0.0, nullptr, nullptr);
   cube_phase_end(c, PH_UPD_SIGMA);
   CUBE_CUDA(c, cudaGetLastError());
-  std::vector<double> part(3 * (size_t)nb);
-  CUBE_CUDA(c, cudaMemcpyAsync(part.data(), c->red_tmp, 8 * part.size(), cudaMemcpyDeviceToHost, c->stream));
-  CUBE_CUDA(c, cudaStreamSynchronize(c->stream));
   r = cube_stats_fetch(c);
   if (r) return r;
   if (c->hstats->flags & 2)
     return cube_fail(c, CUBE_ERR_COUNT_MISMATCH, "a re-sorted particle had no rank in its destination cell");
-  double sums[3] = {0, 0, 0};
-  for (int b = 0; b < nb; b++)
-    for (int t = 0; t < 3; t++) sums[t] += part[3 * b + t];
+  const double* sums = c->hstats->sums;
   c->cur = kn;
   c->np = np_new;
   double npg = (double)(c->npglobal > 0 ? c->npglobal : np_new);
