@@ -144,6 +144,8 @@ int capture(cube_batch* b, int parity) {
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(c->codec[0].dech, c->codec[1].dech, 8 * nv, cudaMemcpyDeviceToDevice, c->stream);
     if (e == cudaSuccess)
+      e = cudaMemcpyAsync(c->codec[0].decf, c->codec[1].decf, 4 * (nv / 2 + 1), cudaMemcpyDeviceToDevice, c->stream);
+    if (e == cudaSuccess)
       e = cudaMemcpyAsync(c->codec[0].bnd, c->codec[1].bnd, 8 * (nv / 2 + 1), cudaMemcpyDeviceToDevice, c->stream);
     if (e != cudaSuccess) break;
     k_batch_tail<<<1, 32, 0, c->stream>>>(c->sd, c->sout, b->hist, b->nbox, i, b->nsteps);

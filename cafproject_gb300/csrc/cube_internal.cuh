@@ -135,8 +135,11 @@ struct cube_ctx {
     float sigma = -1.f;
     double* dec = nullptr;     // dec[v+nvbin/2] = tan code / vcoef(sigma), real(8)
     float2* dech = nullptr;    // the same split into float hi + lo
+    float* decf = nullptr;     // decf[|v|] = the float hi of |dec| (odd in v; decf[nvbin/2] from v = -nvbin/2)
     long long* bnd = nullptr;  // bnd[n] = bits of the smallest |v| that encodes to n (n=1..nvbin/2-1)
-    int32_t* rt = nullptr;     // rt[v+nvbin/2] = the code of dec[v+nvbin/2] (a kick by zero)
+    // rt[v+nvbin/2] = the code of dec[v+nvbin/2] (a kick by zero); then one
+    // more entry, the number of codes above -nvbin/2 that it changes
+    int32_t* rt = nullptr;
   } codec[2];
   int codec_next = 0;
   float sigma_vi = 0.f, sigma_vi_new = 0.f;
@@ -315,6 +318,22 @@ __host__ __device__ inline void cell_coords(const Geo& g, int64_t cid, int& gx, 
   gy = ty * g.nt + iy;
   gz = tz * g.nt + iz;
 }
+// the same cell's tile indices and tile-local coordinates (0-based)
+__host__ __device__ __forceinline__ void cell_tile(const Geo& g, int64_t cid, int T[3], int l[3]) {
+  uint32_t c = (uint32_t)cid, q;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    q = fdiv(c, g.dnt);
+    l[d] = (int)(c - q * (uint32_t)g.nt);
+    c = q;
+  }
+  q = fdiv(c, g.dnnt);
+  T[0] = (int)(c - q * (uint32_t)g.nnt);
+  c = q;
+  q = fdiv(c, g.dnnt);
+  T[1] = (int)(c - q * (uint32_t)g.nnt);
+  T[2] = (int)q;
+}
 // tile index and 1-based tile-local coordinate of a global coarse coordinate
 __host__ __device__ __forceinline__ void tile_local(const Geo& g, int gc, int& T, int& L) {
   T = (int)fdiv((uint32_t)gc, g.dnt);
@@ -334,6 +353,12 @@ __device__ __forceinline__ void store_code(void* a, int64_t i, int nbytes, long 
     ((int8_t*)a)[i] = (int8_t)(uint8_t)(unsigned long long)v;
   else
     ((int16_t*)a)[i] = (int16_t)(uint16_t)(unsigned long long)v;
+}
+__device__ __forceinline__ void store_code_i(void* a, int64_t i, int nbytes, int v) {
+  if (nbytes == 1)
+    ((int8_t*)a)[i] = (int8_t)(uint8_t)(unsigned)v;
+  else
+    ((int16_t*)a)[i] = (int16_t)(uint16_t)(unsigned)v;
 }
 // int(xp+ishift,izipx)+rshift == unsigned(xp)+0.5 (update_particle.f90:66)
 __device__ __forceinline__ double pos_off(int code, int izipx) {
@@ -404,16 +429,24 @@ __device__ __forceinline__ long long v_encode_tab(double v, const long long* __r
 struct CodecView {
   const double* dec;
   const float2* dech;  // dec split into float hi + lo (hi = fl32(dec))
+  const float* decf;   // hi alone, by |code|
   const long long* bnd;
   int half, nmax;  // nvbin/2, nvbin/2-1
   float cf, amp;   // vcoef(sigma) and (nvbin-1)/pi as floats (estimate only)
   const float* cfp;  // when set, cf is read from the device (graph mode)
-  const int32_t* rt;  // code of a zero kick: encode(decode(code)) (may be null)
+  const int32_t* rt;  // code of a zero kick: encode(decode(code)) (may be null); rt[2 half] counts the codes it changes
 };
 __device__ __forceinline__ float codec_cf(const CodecView& k) { return k.cfp ? __ldg(k.cfp) : k.cf; }
 __device__ __forceinline__ double codec_decode(const CodecView& k, int code) { return __ldg(k.dec + code + k.half); }
 __device__ __forceinline__ float2 codec_decode_ff(const CodecView& k, int code) {
   return __ldg(k.dech + code + k.half);
+}
+// The float hi of the decoded value.  A table of 4 bytes per |code|: most
+// lanes' entries (|v| within a few sigma) fit a quarter of the L1, where the
+// 8-byte pairs of dech for both signs took 512 KB and missed it
+__device__ __forceinline__ float codec_decode_f(const CodecView& k, int code) {
+  const float m = __ldg(k.decf + abs(code));
+  return code < 0 ? -m : m;
 }
 __device__ __forceinline__ long long codec_encode(const CodecView& k, double v) {
   return v_encode_tab(v, k.bnd, k.nmax, codec_cf(k), k.amp);
@@ -428,76 +461,33 @@ __device__ __forceinline__ long long codec_encode(const CodecView& k, double v) 
 // stored result is therefore the reference's bit for bit.
 constexpr float kU24 = 5.9604645e-8f;  // 2^-24
 
-// exact float -> double bit pattern with integer operations (subnormals -> +-0)
-__device__ __forceinline__ long long f2d_bits(float f) {
-  unsigned int u = __float_as_uint(f);
-  unsigned int ex = (u >> 23) & 0xffu;
-  unsigned long long s = (unsigned long long)(u >> 31) << 63;
-  if (ex == 0u) return (long long)s;
-  unsigned long long e64 = ex == 0xffu ? 0x7ffull : (unsigned long long)(ex - 127u + 1023u);
-  return (long long)(s | (e64 << 52) | ((unsigned long long)(u & 0x7fffffu) << 29));
-}
-
-// The velocity code of any |V| in [ab - E, ab + E] (ab = bit pattern of a
-// non-negative double, E >= 0) is n: returns true and n when the whole
-// interval lies in one code bin.  Distances are counted in ulps of ab's binade;
-// an edge in another binade is at least as far as that binade's end.
-// the three parts of certify_abs: the FP32 estimate of the bin, the probe of
-// its two edges, and the check on the edges the probe (or a walk) found
-__device__ __forceinline__ long long certify_estimate(long long ab, const CodecView& k) {
-  float af = approx_float_pos(ab);
-  float u0 = k.amp * atanf(codec_cf(k) * af);
-  int m = (int)(u0 + 0.5f);
-  return m < 0 ? 0 : (m > k.nmax ? k.nmax : m);
-}
-__device__ __forceinline__ void certify_probe(long long n, const CodecView& k, long long& lb, long long& ub) {
-  lb = n > 0 ? __ldg(k.bnd + n) : 0;
-  ub = n < k.nmax ? __ldg(k.bnd + n + 1) : 0x7fffffffffffffffLL;
-}
-__device__ __forceinline__ bool certify_finish(long long ab, float E, const CodecView& k, long long n, long long lb,
-                                               long long ub, long long* n_out) {
-  if (ab < lb || ab >= ub) {
-    while (n < k.nmax && __ldg(k.bnd + n + 1) <= ab) n++;
-    while (n > 0 && __ldg(k.bnd + n) > ab) n--;
-    certify_probe(n, k, lb, ub);
-  }
-  *n_out = n;
-  int e = (int)((ab >> 52) & 0x7ff);
-  if (e == 0 || e >= 0x7fe) return n == 0 && e == 0;  // subnormal |V| is deep inside code 0
-  int sh = 1075 - e;                                   // E in ulps of this binade: E * 2^sh
-  float kf = (sh >= -126 && sh <= 127) ? __fmul_rn(E, __int_as_float((127 + sh) << 23)) : ldexpf(E, sh);
-  if (!(kf < 4.0e15f)) return false;
-  long long kk = (kf < 2147483648.0f ? (long long)(unsigned int)kf : (long long)kf) + 1;
-  long long blo = (long long)e << 52, bhi = (long long)(e + 1) << 52;
-  if (n > 0) {
-    long long lx = lb > blo ? lb : blo;
-    if (ab - lx <= kk) return false;
-  }
-  if (n < k.nmax) {
-    long long ux = ub < bhi ? ub : bhi;
-    if (ux - ab <= kk) return false;
-  }
-  return true;
-}
-__device__ __forceinline__ bool certify_abs(long long ab, float E, const CodecView& k, long long* n_out) {
-  // the FP32 estimate is within a few hundredths of a code: probe its bin with
-  // two independent loads, walk only when it fell on the wrong side of an edge
-  const long long n = certify_estimate(ab, k);
-  long long lb, ub;
-  certify_probe(n, k, lb, ub);
-  return certify_finish(ab, E, k, n, lb, ub, n_out);
-}
-// certify_abs of three values with the table probes of all three issued
-// together, so no value's loads wait for another's
-__device__ __forceinline__ void certify_abs3(const long long ab[3], const float E[3], const CodecView& k,
-                                             long long n_out[3], bool ok[3]) {
-  long long n[3], lb[3], ub[3];
-#pragma unroll
-  for (int d = 0; d < 3; d++) n[d] = certify_estimate(ab[d], k);
-#pragma unroll
-  for (int d = 0; d < 3; d++) certify_probe(n[d], k, lb[d], ub[d]);
-#pragma unroll
-  for (int d = 0; d < 3; d++) ok[d] = certify_finish(ab[d], E[d], k, n[d], lb[d], ub[d], &n_out[d]);
+// The velocity code of every |V| in [A - E, A + E] (floats A, E >= 0) is n:
+// true and n when the whole interval lies in one code bin.  The code is the
+// nearest integer to u(V) = (nvbin-1)/pi_f * atan(vcoef V), so no table is
+// needed: u(A) in FP32 is off by at most
+//   2^-23 (vcoef as a float, its product; atan(x) grows no faster than x)
+// + 2^-22 (atanf: 2 ulp, its documented bound)
+// + 2^-23 (amp as a float, its product)          = 4.8e-7, taken as 5.5e-7,
+// relative, u moves by at most amp*vcoef*E over the interval (atan' <= 1), and
+// the reference's own FP64 roundings are below 1e-14.  Where the sum of both
+// does not reach the nearest half-integer the code is certain; a code above 0
+// also has the sign of V then, for u(A) >= 1/2 + u(E).  One lane in fifty or
+// so at |V| of a few sigma stays undecided (u ~ 10^4: 5.5e-7 of it is half a
+// percent of a bin, and E adds as much) and takes the exact chain.  The bins'
+// edges from a table (two 8-byte gathers) left one in a few hundred undecided,
+// but the gathers and 64-bit compares were most of the kicks' instructions and
+// L1 misses.  At 512^3 particles, with the 4-byte decode table: fine kick 6.74
+// -> 4.38 ms, coarse kick 6.43 -> 3.70, scatter 4.05 -> 3.17, PP's kick of its
+// active particles 0.80 -> 0.44.
+__device__ __forceinline__ bool certify_code(float A, float E, const CodecView& k, int* n_out) {
+  const float cf = codec_cf(k);
+  const float u = __fmul_rn(k.amp, atanf(__fmul_rn(cf, A)));
+  const float r = rintf(u);
+  *n_out = (int)r;
+  const float tol = __fmaf_rn(E, __fmul_rn(__fmul_rn(k.amp, cf), 1.00001f), __fmul_rn(u, 5.5e-7f));
+  // 0.5 less the rounding of this sum; an E of NaN or inf, or a code beyond
+  // the last, fails the comparisons
+  return __fadd_rn(fabsf(__fsub_rn(u, r)), tol) < 0.499999f && r <= (float)k.nmax;
 }
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
@@ -517,27 +507,20 @@ static __device__ __noinline__ long long pp_kick_exact(CodecView cv, int code, f
 // The PP kick of one particle's three velocity codes: v = decode(code) +
 // F*kick, encoded with the same sigma.  The FP32 sum of the decode's float
 // hi and the FP32 kick product is certified against its bound (the
-// product's two roundings, the hi split and the sum's rounding) with the
-// three table probes issued together; undecided lanes take the FP64
-// expression.  code[] is updated in place.
+// product's two roundings, the hi split and the sum's rounding); undecided
+// lanes take the FP64 expression.  code[] is updated in place.
 __device__ __forceinline__ void pp_kick3(const CodecView& cv, int code[3], const float F[3], float kick_f,
                                          double kick_d, int exact_only) {
-  float E[3], vf[3];
-  long long ab[3], n[3];
-  bool ok[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    const float dh = codec_decode_ff(cv, code[d]).x;
+    const float dh = codec_decode_f(cv, code[d]);
     const float kf = __fmul_rn(F[d], kick_f);
-    vf[d] = __fadd_rn(dh, kf);
-    E[d] = 1.25f * (fabsf(kf) * 1.3e-7f + (2.f * fabsf(dh) + fabsf(vf[d])) * 6.0e-8f);
-    ab[d] = f2d_bits(vf[d]) & 0x7fffffffffffffffLL;
+    const float vf = __fadd_rn(dh, kf);
+    const float E = 1.25f * (fabsf(kf) * 1.3e-7f + (2.f * fabsf(dh) + fabsf(vf)) * 6.0e-8f);
+    int n;
+    const bool ok = certify_code(fabsf(vf), E, cv, &n) && !exact_only;
+    code[d] = ok ? (vf < 0.f ? -n : n) : (int)pp_kick_exact(cv, code[d], F[d], kick_d);
   }
-  certify_abs3(ab, E, cv, n, ok);
-#pragma unroll
-  for (int d = 0; d < 3; d++)
-    code[d] = (!exact_only && ok[d]) ? (int)(vf[d] < 0.f ? -n[d] : n[d])
-                                     : (int)pp_kick_exact(cv, code[d], F[d], kick_d);
 }
 
 // Nearest float to the real t + lo, certified when every real within margin

@@ -314,6 +314,9 @@ __device__ __forceinline__ float f2sum(float a, float b, float c) {
   return __fadd_rn(__fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b)), __fmul_rn(c, c));
 }
 // kPre: then rewrite each force value as its kick factor force*a_mid*dt/6/pi
+// (repeating a row's first value in its padding, to spare the kicks the wrap in
+// x, took 6.5 ms instead of 4.6 at 1024^3: the padding shares its sector with
+// the next row's start, whose load another block has pending)
 template <bool kPre>
 __global__ void k_f2max(float* __restrict__ f0, float* __restrict__ f1, float* __restrict__ f2, int n,
                         unsigned int* __restrict__ out, float a_mid, float dt, const StepDev* sd) {
@@ -394,103 +397,118 @@ __device__ __forceinline__ float kick_tau(const KickArgs& a, int d) {
 // bounded by
 //   gamma_7 sum|t_i| + 2^-24 (|decode| + |V_f|) + 9*2^-53 (|decode| + sum|t_i| + |V_f|)
 // (recursive-summation bound, gamma_7 = 7u/(1-7u), u = 2^-24; the decode table's
-// float hi is within half an ulp).  certify_abs keeps the code only when every
+// float hi is within half an ulp).  certify_code keeps the code only when every
 // double inside that bound encodes to it; otherwise the lane runs the exact
 // chain, so the stored code is always the reference's.
 //
 // The exact chain (and, in the coarse kick, the exact |v + vfield| of lanes
-// that may set vmax) is needed by a few components in a thousand, but a warp
-// runs it whenever one of its 32 lanes needs it, on the FP64 pipe.  So each
+// that may set vmax) is needed by a few components in a hundred, but a warp
+// would run it whenever one of its 32 lanes needs it, on the FP64 pipe.  So each
 // warp queues those (particle, component, code) entries in shared memory and
 // runs the chain 32 entries at a time, each lane recomputing its entry's CIC
 // corners and terms (the same arithmetic, the same bits).  An entry packs
 // the particle index (bits 18 and up), the 16-bit code and the component.
+//
+// Bound by the L1: the force gathers are 8 corners x 3 components of 4 bytes
+// (a warp's 32 particles spread over four or so cells, so about ten sectors a
+// gather) plus what the velocity codec gathers, and by issue slots.  Hence the
+// table-free certificate and the 4-byte decode table (one table gather a
+// component instead of five), one row address per pair of x corners, and every
+// component unrolled (indexing the codes in a loop had put them in local
+// memory): 6.74 -> 4.38 ms fine and 6.43 -> 3.70 ms coarse at 512^3 particles,
+// 63 % of the L1's wavefront rate now.
 constexpr int KICK_Q = 64;  // queue entries per warp: at most 31 pending + 32 from one component
 __device__ __forceinline__ unsigned long long kick_qkey(int64_t p, int d, int code) {
   return ((unsigned long long)p << 18) | ((unsigned long long)(code & 0xffff) << 2) | (unsigned long long)d;
 }
 
-// a corner's mesh index is xo[i] + yo[j] + zo[k] (i, j, k = 0 for the lower
-// corner, 1 for the upper; x and y parts in 32 bits)
+// A stencil's lower x, its upper x relative to it, and the row y + n*z of its
+// four corners (lower and upper y, lower and upper z).
 struct KickCorners {
-  int xo[2], yo[2];
-  int64_t zo[2];
+  int x, dx;
+  uint32_t row[2][2];  // [z][y]
   float d1[3], d2[3];
-  int64_t cell;
+  int cell;
 };
 
 template <bool kFine>
 __device__ __forceinline__ void kick_corners(const KickArgs& a, int64_t p, KickCorners& k) {
   const Geo& g = a.g;
   k.cell = a.pcell[p];
-  int gc[3];
-  cell_coords(g, k.cell, gc[0], gc[1], gc[2]);
-  int i1[3], i2[3];
+  int T[3], l[3], i1[3], i2[3];
+  cell_tile(g, k.cell, T, l);
   const int n = kFine ? g.nf : g.nc;
+#pragma unroll
   for (int d = 0; d < 3; d++) {
-    int T, L;
-    tile_local(g, gc[d], T, L);
-    int code = load_code(a.xp, 3 * p + d, g.izipx);
-    float tx;
+    const int code = load_code(a.xp, 3 * p + d, g.izipx);
+    float tx, fl;
     int base;
     if (kFine) {
-      tx = fine_tempx(g.ncell, L, code, g.izipx);  // tile-local frame (pm.f90:138)
-      base = T * g.nt * g.ncell + (int)floorf(tx);
+      tx = fine_tempx(g.ncell, l[d] + 1, code, g.izipx);  // tile-local frame (pm.f90:138)
+      fl = floorf(tx);
+      base = T[d] * g.nt * g.ncell + (int)fl;
     } else {
-      tx = coarse_tempx(gc[d] + 1, code, g.izipx);  // global frame (pm.f90:335)
-      base = (int)floorf(tx);
+      tx = coarse_tempx(T[d] * g.nt + l[d] + 1, code, g.izipx);  // global frame (pm.f90:335)
+      fl = floorf(tx);
+      base = (int)fl;
     }
-    float fl = floorf(tx);
     k.d1[d] = __fsub_rn(__fadd_rn(fl, 1.0f), tx);
     k.d2[d] = __fsub_rn(1.0f, k.d1[d]);
     i1[d] = wrap1(base, n);
     i2[d] = wrap1(base + 1, n);
   }
-  // mesh_idx(n, x, y, z) = x + (n+2)*(y + n*z)
-  k.xo[0] = i1[0];
-  k.xo[1] = i2[0];
-  k.yo[0] = (n + 2) * i1[1];
-  k.yo[1] = (n + 2) * i2[1];
-  k.zo[0] = (int64_t)(n + 2) * n * i1[2];
-  k.zo[1] = (int64_t)(n + 2) * n * i2[2];
+  k.x = i1[0];
+  k.dx = i2[0] - i1[0];
+  k.row[0][0] = (uint32_t)i1[1] + (uint32_t)n * (uint32_t)i1[2];
+  k.row[0][1] = (uint32_t)i2[1] + (uint32_t)n * (uint32_t)i1[2];
+  k.row[1][0] = (uint32_t)i1[1] + (uint32_t)n * (uint32_t)i2[2];
+  k.row[1][1] = (uint32_t)i2[1] + (uint32_t)n * (uint32_t)i2[2];
 }
 
-// the eight real(4) CIC terms of component d, in the reference's order
-template <bool kPre>
-__device__ __forceinline__ void kick_terms(const KickArgs& a, const KickCorners& k, int d, float t[8]) {
-  const float* F = a.f[d];
-  const float* d1 = k.d1;
-  const float* d2 = k.d2;
-#define KT(c, wa, wb, wc) (kPre ? kick_w(__ldg(F + (c)), wa, wb, wc) : kick_term(__ldg(F + (c)), kick_amid(a), kick_dt(a), wa, wb, wc))
-  // corners c111, c211, c121, c112, c122, c212, c221, c222
-  const float* F0 = F + k.zo[0];
-  const float* F1 = F + k.zo[1];
-  t[0] = KT(k.xo[0] + k.yo[0] + (F0 - F), d1[0], d1[1], d1[2]);
-  t[1] = KT(k.xo[1] + k.yo[0] + (F0 - F), d2[0], d1[1], d1[2]);
-  t[2] = KT(k.xo[0] + k.yo[1] + (F0 - F), d1[0], d2[1], d1[2]);
-  t[3] = KT(k.xo[0] + k.yo[0] + (F1 - F), d1[0], d1[1], d2[2]);
-  t[4] = KT(k.xo[0] + k.yo[1] + (F1 - F), d1[0], d2[1], d2[2]);
-  t[5] = KT(k.xo[1] + k.yo[0] + (F1 - F), d2[0], d1[1], d2[2]);
-  t[6] = KT(k.xo[1] + k.yo[1] + (F0 - F), d2[0], d2[1], d1[2]);
-  t[7] = KT(k.xo[1] + k.yo[1] + (F1 - F), d2[0], d2[1], d2[2]);
-#undef KT
+// the eight real(4) CIC terms of the component whose mesh is F, in the
+// reference's order: corners c111, c211, c121, c112, c122, c212, c221, c222
+template <bool kFine, bool kPre>
+__device__ __forceinline__ void kick_terms(const KickArgs& a, const KickCorners& k, const float* F, float t[8]) {
+  const uint32_t stride = (uint32_t)((kFine ? a.g.nf : a.g.nc) + 2) * 4u;  // bytes of a padded row
+  const char* base = reinterpret_cast<const char*>(F + k.x);
+  float v[2][2][2];  // [z][y][x]
+#pragma unroll
+  for (int z = 0; z < 2; z++)
+#pragma unroll
+    for (int y = 0; y < 2; y++) {
+      const float* r = reinterpret_cast<const float*>(base + (uint64_t)k.row[z][y] * stride);
+      v[z][y][0] = __ldg(r);
+      v[z][y][1] = __ldg(r + k.dx);
+    }
+  auto term = [&](int x, int y, int z) {
+    const float wx = x ? k.d2[0] : k.d1[0], wy = y ? k.d2[1] : k.d1[1], wz = z ? k.d2[2] : k.d1[2];
+    return kPre ? kick_w(v[z][y][x], wx, wy, wz) : kick_term(v[z][y][x], kick_amid(a), kick_dt(a), wx, wy, wz);
+  };
+  t[0] = term(0, 0, 0);
+  t[1] = term(1, 0, 0);
+  t[2] = term(0, 1, 0);
+  t[3] = term(0, 0, 1);
+  t[4] = term(0, 1, 1);
+  t[5] = term(1, 0, 1);
+  t[6] = term(1, 1, 0);
+  t[7] = term(1, 1, 1);
 }
 
 // one queued component on the reference's FP64 chain: its code, and in the
 // coarse kick vmax=max(vmax,abs(vreal+vfield)) (pm.f90:349) as real(4)
 template <bool kFine, bool kPre>
-__device__ __forceinline__ void kick_exact_entry(const KickArgs& a, unsigned long long key, float vm[3]) {
+__device__ __noinline__ void kick_exact_entry(const KickArgs& a, unsigned long long key, float vm[3]) {
   const int64_t p = (int64_t)(key >> 18);
   const int d = (int)(key & 3ull);
   const int code = (int)(int16_t)(uint16_t)((key >> 2) & 0xffffull);
   KickCorners k;
   kick_corners<kFine>(a, p, k);
   float t[8];
-  kick_terms<kPre>(a, k, d, t);
+  kick_terms<kFine, kPre>(a, k, d == 0 ? a.f[0] : (d == 1 ? a.f[1] : a.f[2]), t);
   double v = codec_decode(a.cin, code);
   for (int i = 0; i < 8; i++) v = __dadd_rn(v, (double)t[i]);
   if (!kFine) {
-    const double w = fabs(__dadd_rn(v, (double)a.vfield[3 * k.cell + d]));
+    const double w = fabs(__dadd_rn(v, (double)a.vfield[3 * (int64_t)k.cell + d]));
     const float wf = __double2float_rn(w);
     vm[0] = d == 0 ? fmaxf(vm[0], wf) : vm[0];
     vm[1] = d == 1 ? fmaxf(vm[1], wf) : vm[1];
@@ -515,6 +533,9 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
   float vm[3] = {0.f, 0.f, 0.f};  // coarse: exact vmax; fine: the FP32 estimate
   float vlo[3] = {0.f, 0.f, 0.f};  // coarse: lower bounds of |v + vfield|
   unsigned long long nex = 0;
+  // the zero-kick codes are the codes themselves, but for -nvbin/2, when the
+  // table's count says so
+  const bool rt_same = kFine && a.pp_act && __ldg(a.cin.rt + 2 * a.cin.half) == 0;
   // whole warps iterate together (the queue's ballots); lanes past the end
   // compute on the last particle and store nothing
   for (int64_t p0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p0 - lane < a.np;
@@ -532,50 +553,46 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
       // others' force is zero, their PP code the zero-kick code of theirs
       const bool on = (__ldg(a.pp_act + (p >> 5)) >> (p & 31)) & 1u;
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        const int z = __ldg(a.cin.rt + codes[d] + a.cin.half);
-        codes[d] = on ? codes[d] : z;
-      }
+      for (int d = 0; d < 3; d++)
+        if (!on && (!rt_same || codes[d] == -a.cin.half)) codes[d] = __ldg(a.cin.rt + codes[d] + a.cin.half);
     } else if (kFine && a.fpp) {
       // ext_pp_force's kick before the fine kick, both in this pass: the PP
       // code (decoded and encoded with sigma_vi) is the one the fine kick decodes
       const float F[3] = {a.fpp[3 * p], a.fpp[3 * p + 1], a.fpp[3 * p + 2]};
       pp_kick3(a.cin, codes, F, a.pp_kf, a.pp_kd, a.exact_only);
     }
+#pragma unroll
     for (int d = 0; d < 3; d++) {
       float t[8];
-      kick_terms<kPre>(a, k, d, t);
-      const int code = codes[d];
-      float dh = codec_decode_ff(a.cin, code).x;
+      kick_terms<kFine, kPre>(a, k, a.f[d], t);
+      const float dh = codec_decode_f(a.cin, codes[d]);
       float S = t[0], T = fabsf(t[0]);
+#pragma unroll
       for (int i = 1; i < 8; i++) {
         S = __fadd_rn(S, t[i]);
         T = __fadd_rn(T, fabsf(t[i]));
       }
-      float vf = __fadd_rn(dh, S);
-      long long vb = f2d_bits(vf), ab = vb & 0x7fffffffffffffffLL;
-      float E = 1.25f * (T * 4.76837158e-7f + (fabsf(dh) + fabsf(vf)) * 6.0e-8f + T * 1.0e-15f);
-      long long nc_ = 0;
-      bool ok = !a.exact_only && certify_abs(ab, E, a.cout, &nc_);
-      bool need_vmax = false;
+      const float vf = __fadd_rn(dh, S);
+      const float E = 1.25f * (T * 4.76837158e-7f + (fabsf(dh) + fabsf(vf)) * 6.0e-8f + T * 1.0e-15f);
+      int n;
+      bool fast = certify_code(fabsf(vf), E, a.cout, &n) && !a.exact_only;
       if (!kFine) {
-        const float vfd = a.vfield[3 * k.cell + d];
+        const float vfd = a.vfield[3 * (int64_t)k.cell + d];
         // |v + vfield| of the reference's FP64 v lies in [lo, ub]
-        float ub = (fabsf(vf) + E + fabsf(vfd)) * 1.000001f;
-        float lo = __fmul_rn(__fsub_rn(fabsf(__fadd_rn(vf, vfd)), E), 0.99999f);
+        const float ub = (fabsf(vf) + E + fabsf(vfd)) * 1.000001f;
+        const float lo = __fmul_rn(__fsub_rn(fabsf(__fadd_rn(vf, vfd)), E), 0.99999f);
         if (valid) vlo[d] = fmaxf(vlo[d], lo);
         // the first pass: lanes that may reach tau; the rerun: lanes that may
         // reach the largest lower bound, which the maximum does
-        need_vmax = ub >= (a.vmax_only ? __uint_as_float(__ldg(&a.vmax_lo[d])) : kick_tau(a, d));
+        if (ub >= (a.vmax_only ? __uint_as_float(__ldg(&a.vmax_lo[d])) : kick_tau(a, d))) fast = false;
       } else if (a.vmax_est && valid) {
-        vm[d] = fmaxf(vm[d], fabsf(__fadd_rn(vf, a.vfield[3 * k.cell + d])));
+        vm[d] = fmaxf(vm[d], fabsf(__fadd_rn(vf, a.vfield[3 * (int64_t)k.cell + d])));
       }
-      const bool fast = ok && !need_vmax;
-      if (fast && valid && !a.vmax_only) store_code(a.vp_out, 3 * p + d, g.izipv, vb < 0 ? -nc_ : nc_);
+      if (fast && valid && !a.vmax_only) store_code_i(a.vp_out, 3 * p + d, g.izipv, vf < 0.f ? -n : n);
       const bool defer = valid && !fast;
       const unsigned m = __ballot_sync(0xffffffffu, defer);
       if (m) {
-        if (defer) s_q[wq][qn + __popc(m & ((1u << lane) - 1u))] = kick_qkey(p, d, code);
+        if (defer) s_q[wq][qn + __popc(m & ((1u << lane) - 1u))] = kick_qkey(p, d, codes[d]);
         qn += __popc(m);
         // the chain for 32 queued entries at a time, one per lane
         if (qn >= 32) {

@@ -286,15 +286,19 @@ int cube_build_tables(cube_ctx* c) {
 }
 
 // sigp, when set, supplies sigma from the device (graph mode)
+// decf and rt may be null; the count behind rt starts at zero here
 __global__ void k_decode_table(const float* __restrict__ tan_tab, int nv, float sigma, const float* sigp,
-                               double* __restrict__ dec, float2* __restrict__ dech) {
+                               double* __restrict__ dec, float2* __restrict__ dech, float* __restrict__ decf,
+                               int32_t* __restrict__ rt) {
   if (sigp) sigma = *sigp;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0 && rt) rt[nv] = 0;
   if (i < nv) {
     double d = __ddiv_rn((double)tan_tab[i], vcoef(sigma));
     dec[i] = d;
     float hi = __double2float_rn(d);
     dech[i] = make_float2(hi, __double2float_rn(__dsub_rn(d, (double)hi)));
+    if (decf && i <= nv / 2) decf[nv / 2 - i] = -hi;  // tan is odd, to the bit
   }
 }
 
@@ -367,12 +371,16 @@ __global__ void k_reencode(CodecView k, const float* sigp, float sigma, int nvbi
   k.cf = (float)vcoef(sigma);
   k.cfp = nullptr;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nvbin) rt[i] = (int32_t)codec_encode(k, codec_decode(k, i - k.half));
+  if (i >= nvbin) return;
+  const int32_t n = (int32_t)codec_encode(k, codec_decode(k, i - k.half));
+  rt[i] = n;
+  if (i > 0 && n != i - k.half) atomicAdd(rt + nvbin, 1);
 }
 
 static void view_of(const cube_ctx* c, const cube_ctx::Codec& k, CodecView* v) {
   v->dec = k.dec;
   v->dech = k.dech;
+  v->decf = k.decf;
   v->bnd = k.bnd;
   v->half = c->nvbin / 2;
   v->nmax = c->nvbin / 2 - 1;
@@ -384,7 +392,8 @@ static void view_of(const cube_ctx* c, const cube_ctx::Codec& k, CodecView* v) {
 
 static int build_codec(cube_ctx* c, int slot, float sigma, const float* sigp = nullptr) {
   cube_ctx::Codec& k = c->codec[slot];
-  k_decode_table<<<(c->nvbin + 255) / 256, 256, 0, c->stream>>>(c->tan_tab, c->nvbin, sigma, sigp, k.dec, k.dech);
+  k_decode_table<<<(c->nvbin + 255) / 256, 256, 0, c->stream>>>(c->tan_tab, c->nvbin, sigma, sigp, k.dec, k.dech,
+                                                                  k.decf, k.rt);
   int nmax = c->nvbin / 2 - 1;
   k_encode_bounds<<<(nmax + 127) / 128, 128, 0, c->stream>>>(sigma, sigp, c->nvbin, k.bnd);
   if (k.rt) {
@@ -443,11 +452,11 @@ __global__ void k_codec_check(const double* __restrict__ v, int64_t n, double c,
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     direct[i] = (int32_t)v_encode(v[i], c, nvbin);
     int32_t t = (int32_t)codec_encode(k, v[i]);
-    // the kernels' certified encode (its table-free test first): when it
+    // the kernels' certified encode, for the float nearest v: when it
     // certifies a code, that code must be the table's; INT32_MIN marks a miss
-    const long long bits = __double_as_longlong(v[i]);
-    long long nq;
-    if (certify_abs(bits & 0x7fffffffffffffffLL, 0.f, k, &nq) && (bits < 0 ? -nq : nq) != (long long)t) t = INT32_MIN;
+    const float A = fabsf(__double2float_rn(v[i]));
+    int nq;
+    if (certify_code(A, __fmul_rn(A, 6.0e-8f), k, &nq) && (v[i] < 0.0 ? -nq : nq) != t) t = INT32_MIN;
     table[i] = t;
   }
 }
@@ -588,7 +597,7 @@ extern "C" int cube_codec_check_static(cube_ctx* c, float sigma, const double* v
   // released with work on the shared array still in flight
   const int nmax = c->nvbin / 2 - 1;
   k_decode_table<<<(c->nvbin + 255) / 256, 256, 0, c->stream>>>(c->tan_tab, c->nvbin, sigma, nullptr, tab.dec,
-                                                                  tab.dech);
+                                                                  tab.dech, nullptr, nullptr);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
     k_encode_bounds<<<(nmax + 127) / 128, 128, 0, c->stream>>>(sigma, nullptr, c->nvbin, tab.bnd);

@@ -122,7 +122,7 @@ __global__ void k_dest(UpdArgs a) {
       int vcode = load_code(a.vp, 3 * p + d, g.izipv);
       float vfd = a.vfield[3 * cell + d];
       // fast path: v = dec+vfield, P = dt_mid*v, deltax = P/4 in FP32 with bound Edx
-      float dh = codec_decode_ff(a.cv, vcode).x;
+      float dh = codec_decode_f(a.cv, vcode);
       float vfa = __fadd_rn(dh, vfd);
       float Pf = __fmul_rn(dtm(a), vfa);
       float dxf = __fmul_rn(Pf, 0.25f);
@@ -601,53 +601,102 @@ __global__ void k_rank(UpdArgs a) {
   }
 }
 
-// particle p, landed in cell D, written at index idx of the new arrays
-__device__ __forceinline__ void write_particle_at(const UpdArgs& a, int64_t p, int32_t D, int64_t idx) {
+// vp = code of vreal - vfield_new (update_particle.f90:116-117), the FP64 chain
+__device__ __forceinline__ int recode_exact(const UpdArgs& a, int vcode, float vfd, float vbar) {
+  const double v = __dadd_rn(codec_decode(a.cv, vcode), (double)vfd);
+  return (int)codec_encode(a.cv, __dsub_rn(v, (double)vbar));
+}
+
+// particle p, landed in cell D, written at index idx of the new arrays;
+// returns the components (bit d) whose new velocity code the FP32 test left
+// undecided, for recode_exact
+__device__ __forceinline__ unsigned write_particle_at(const UpdArgs& a, int64_t p, int32_t D, int64_t idx) {
   const Geo& g = a.g;
-  int64_t cell = a.pcell[p];
+  const int64_t cell = a.pcell[p];
+  unsigned open = 0;
   // nint(dt_mid*vreal/(x_resolution*ncell)): the divisor is a power of two
-  float scale = g.izipx == 1 ? 64.0f : 16384.0f;
+  const float scale = g.izipx == 1 ? 64.0f : 16384.0f;
+#pragma unroll
   for (int d = 0; d < 3; d++) {
-    int vcode = load_code(a.vp, 3 * p + d, g.izipv);
-    float vfd = a.vfield[3 * cell + d];
-    float vbar = a.vfield_new[3 * (int64_t)D + d];
-    float2 dd = codec_decode_ff(a.cv, vcode);
+    const int vcode = load_code(a.vp, 3 * p + d, g.izipv);
+    const float vfd = a.vfield[3 * cell + d];
+    const float vbar = a.vfield_new[3 * (int64_t)D + d];
+    const float dh = codec_decode_f(a.cv, vcode);
     // drift in code units: FP32 estimate of dt_mid*(dec+vfield)*scale with its bound
-    float vfa = __fadd_rn(dd.x, vfd);
-    float Pf = __fmul_rn(dtm(a), vfa);
-    float EP = scale * 1.25f * (fabsf(dtm(a)) * (fabsf(dd.x) + fabsf(vfa)) * 1.2e-7f + fabsf(Pf) * 6.0e-8f);
+    const float vfa = __fadd_rn(dh, vfd);
+    const float Pf = __fmul_rn(dtm(a), vfa);
+    const float EP = scale * 1.25f * (fabsf(dtm(a)) * (fabsf(dh) + fabsf(vfa)) * 1.2e-7f + fabsf(Pf) * 6.0e-8f);
     long long dx;
     if (a.exact_only || !nint_certified(__fmul_rn(Pf, scale), EP, &dx)) {
       double v = __dadd_rn(codec_decode(a.cv, vcode), (double)vfd);
       dx = llround(__dmul_rn(__dmul_rn((double)dtm(a), v), (double)scale));
     }
-    long long x = load_code(a.xp, 3 * p + d, g.izipx);
+    const long long x = load_code(a.xp, 3 * p + d, g.izipx);
     store_code(a.xp_new, 3 * idx + d, g.izipx, x + dx);
-    // vp = code of vreal - vfield_new (update_particle.f90:116-117)
     float w, ew;
     two_sum(vfd, -vbar, w, ew);
-    float Vf = __fadd_rn(dd.x, w);
-    float E = 1.25f * ((fabsf(dd.x) + fabsf(Vf)) * 6.0e-8f + fabsf(ew) +
-                       (fabsf(dd.x) + fabsf(vfd) + fabsf(vbar)) * 2.3e-16f);
-    long long ab = f2d_bits(Vf) & 0x7fffffffffffffffLL, n = 0, code;
-    if (!a.exact_only && certify_abs(ab, E, a.cv, &n)) {
-      code = Vf < 0.f ? -n : n;
-    } else {
-      double v = __dadd_rn(codec_decode(a.cv, vcode), (double)vfd);
-      code = codec_encode(a.cv, __dsub_rn(v, (double)vbar));
-    }
-    store_code(a.vp_new, 3 * idx + d, g.izipv, code);
+    const float Vf = __fadd_rn(dh, w);
+    const float E = 1.25f * ((fabsf(dh) + fabsf(Vf)) * 6.0e-8f + fabsf(ew) +
+                             (fabsf(dh) + fabsf(vfd) + fabsf(vbar)) * 2.3e-16f);
+    int n;
+    if (certify_code(fabsf(Vf), E, a.cv, &n) && !a.exact_only)
+      store_code_i(a.vp_new, 3 * idx + d, g.izipv, Vf < 0.f ? -n : n);
+    else
+      open |= 1u << d;
   }
   a.pid_new[idx] = a.pid[p];
   a.pcell_new[idx] = D;
+  return open;
 }
 
-__device__ __forceinline__ void write_particle(const UpdArgs& a, int64_t p, int32_t D, uint32_t r) {
-  if (D < 0 || (int64_t)D >= a.ncells || r >= (uint32_t)a.cnt_new[D]) {
-    atomicOr(&a.st->flags, 2);  // rank not assigned: never write outside the new arrays
-    return;
+// The undecided components of a warp's particles, queued in shared memory and
+// taken through the FP64 chain 32 at a time, one per lane: a few in a hundred
+// need it, so nearly every warp would run it, mostly idle, at each of them
+// (k_scatter of 512^3 particles: 4.05 -> 3.17 ms with the queue and the
+// table-free test together).  An entry holds the particle and its new index (31 bits
+// each: the permutation is int32) and the component.
+constexpr int SC_Q = 128;  // entries per warp: at most 31 pending + 96 of one pass
+struct RecodeQueue {
+  unsigned long long* q;
+  int n;  // warp-uniform
+};
+__device__ __forceinline__ void recode_entry(const UpdArgs& a, unsigned long long e) {
+  const int d = (int)(e & 3ull);
+  const int64_t p = (int64_t)(e >> 33), idx = (int64_t)((e >> 2) & 0x7fffffffull);
+  const int64_t D = *(volatile const int32_t*)(a.pcell_new + idx);
+  store_code_i(a.vp_new, 3 * idx + d, a.g.izipv,
+               recode_exact(a, load_code(a.vp, 3 * p + d, a.g.izipv), a.vfield[3 * (int64_t)a.pcell[p] + d],
+                            a.vfield_new[3 * D + d]));
+}
+// called by whole warps; open = the lane's undecided components of (p, idx)
+__device__ __forceinline__ void recode_push(const UpdArgs& a, RecodeQueue& rq, unsigned open, int64_t p, int64_t idx) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const bool mine = (open >> d) & 1u;
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (mine)
+      rq.q[rq.n + __popc(m & ((1u << lane) - 1u))] =
+          ((unsigned long long)p << 33) | ((unsigned long long)idx << 2) | (unsigned long long)d;
+    rq.n += __popc(m);
   }
-  write_particle_at(a, p, D, a.cstart_new[D] + r);
+  __syncwarp();  // the entries and the pcell_new they name are visible to the warp
+  while (rq.n >= 32) {
+    recode_entry(a, rq.q[rq.n - 32 + lane]);
+    rq.n -= 32;
+    __syncwarp();
+  }
+}
+__device__ __forceinline__ void recode_rest(const UpdArgs& a, RecodeQueue& rq) {
+  __syncwarp();
+  if ((int)(threadIdx.x & 31) < rq.n) recode_entry(a, rq.q[threadIdx.x & 31]);
+}
+
+// rank r of a landing in D checked before anything is written
+__device__ __forceinline__ bool rank_ok(const UpdArgs& a, int32_t D, uint32_t r) {
+  if (D >= 0 && (int64_t)D < a.ncells && r < (uint32_t)a.cnt_new[D]) return true;
+  atomicOr(&a.st->flags, 2);  // rank not assigned: never write outside the new arrays
+  return false;
 }
 
 // U2, general path: the rank of a landing (a particle's primary destination,
@@ -732,30 +781,66 @@ __global__ void k_sort_place(UpdArgs a, const int32_t* __restrict__ vals, int64_
 // U3 on the sort path: one thread per new index writes the particle that
 // lands there (coalesced writes; the reads stay within a few cells of the
 // destination, which L2 holds)
-__global__ void k_sort_gather(UpdArgs a, const uint64_t* __restrict__ keys, int64_t n_new, int shift) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_new; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t D = (int64_t)(keys[i] >> shift);
-    if (D >= a.ncells || i < a.cstart_new[D] || i >= a.cstart_new[D + 1]) {
-      atomicOr(&a.st->flags, 2);
-      continue;
+__global__ void __launch_bounds__(256) k_sort_gather(UpdArgs a, const uint64_t* __restrict__ keys, int64_t n_new,
+                                                     int shift) {
+  __shared__ unsigned long long s_q[8][SC_Q];
+  RecodeQueue rq{s_q[threadIdx.x >> 5], 0};
+  const int lane = threadIdx.x & 31;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i - lane < n_new;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    unsigned open = 0;
+    int64_t p = 0;
+    if (i < n_new) {
+      const int64_t D = (int64_t)(keys[i] >> shift);
+      if (D >= a.ncells || i < a.cstart_new[D] || i >= a.cstart_new[D + 1]) {
+        atomicOr(&a.st->flags, 2);
+      } else {
+        p = a.perm[i];
+        open = write_particle_at(a, p, (int32_t)D, i);
+      }
     }
-    write_particle_at(a, a.perm[i], (int32_t)D, i);
+    recode_push(a, rq, open, p, i);
   }
+  recode_rest(a, rq);
 }
 
 // U3: scatter every primary copy to its place in the new disjoint order.
-__global__ void k_scatter(UpdArgs a) {
-  int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.np; p += stride) {
-    int32_t D = a.dest[p];
-    if (D >= 0) write_particle(a, p, D, a.rank[p]);
+__global__ void __launch_bounds__(256) k_scatter(UpdArgs a) {
+  __shared__ unsigned long long s_q[8][SC_Q];
+  RecodeQueue rq{s_q[threadIdx.x >> 5], 0};
+  const int lane = threadIdx.x & 31;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p - lane < a.np; p += stride) {
+    unsigned open = 0;
+    int64_t idx = 0;
+    if (p < a.np) {
+      const int32_t D = a.dest[p];
+      const uint32_t r = D >= 0 ? a.rank[p] : 0u;
+      if (D >= 0 && rank_ok(a, D, r)) {
+        idx = a.cstart_new[D] + r;
+        open = write_particle_at(a, p, D, idx);
+      }
+    }
+    recode_push(a, rq, open, p, idx);
   }
+  recode_rest(a, rq);
 }
 
 __global__ void k_scatter_xtra(UpdArgs a) {
   int64_t nx = (int64_t)(a.st->ndup_list < (unsigned long long)a.xtra_cap ? a.st->ndup_list : (unsigned long long)a.xtra_cap);
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nx; e += (int64_t)gridDim.x * blockDim.x)
-    write_particle(a, a.xtra[e].x, a.xtra[e].y, (uint32_t)a.xtra[e].z);
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nx; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = a.xtra[e].x;
+    const int32_t D = a.xtra[e].y;
+    const uint32_t r = (uint32_t)a.xtra[e].z;
+    if (!rank_ok(a, D, r)) continue;
+    const int64_t idx = a.cstart_new[D] + r;
+    const unsigned open = write_particle_at(a, p, D, idx);
+    for (int d = 0; d < 3; d++)
+      if ((open >> d) & 1u)
+        store_code_i(a.vp_new, 3 * idx + d, a.g.izipv,
+                     recode_exact(a, load_code(a.vp, 3 * p + d, a.g.izipv), a.vfield[3 * (int64_t)a.pcell[p] + d],
+                                  a.vfield_new[3 * (int64_t)D + d]));
+  }
 }
 
 __device__ __forceinline__ void ff_add(float& hi, float& lo, float x, float xlo) {
