@@ -54,6 +54,12 @@ static void release(cube_ctx* c) {
     cudaEventDestroy(c->ev_pid);
   }
   cube_timers_free(c);
+  if (c->stream_aux) {
+    cudaStreamSynchronize(c->stream_aux);
+    cudaStreamDestroy(c->stream_aux);
+  }
+  if (c->ev_aux) cudaEventDestroy(c->ev_aux);
+  if (c->ev_codec) cudaEventDestroy(c->ev_codec);
   if (c->owner) {  // meshes, kernels, plans, work area and stream belong to the owner
     if (c->owner->linked == c) c->owner->linked = nullptr;
     c->rho_f = c->kern_f = c->kern_f_raw = c->rho_c = c->kern_c = nullptr;
@@ -167,6 +173,12 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
   } else {
     CUBE_CUDA(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   }
+  // the highest priority: its few small kernels take SM slots as they come free
+  int aux_lo = 0, aux_hi = 0;
+  CUBE_CUDA(c, cudaDeviceGetStreamPriorityRange(&aux_lo, &aux_hi));
+  CUBE_CUDA(c, cudaStreamCreateWithPriority(&c->stream_aux, cudaStreamNonBlocking, aux_hi));
+  CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_aux, cudaEventDisableTiming));
+  CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_codec, cudaEventDisableTiming));
   int64_t np = p->np_max;
   for (int k = 0; k < 2; k++) {
     ALLOC(c->xp[k], 3 * np * p->izipx);

@@ -12,10 +12,9 @@
 //   step    update_x with the rank-path choice, the extra-copy count and
 //           sigma_vi_new resolved on the device, PP, particle_mesh;
 //   tail    k_batch_tail: vmax / vz_max / sigma carried to the next step, the
-//           step's stats appended to a device history; codec slot 1
-//           (sigma_vi_new) copied to slot 0.
-// The state buffers of a context alternate between steps, so two graphs are
-// captured (even and odd steps).  No host synchronisation happens between
+//           step's stats appended to a device history.
+// The state buffers and codec slots of a context alternate between steps, so
+// two graphs are captured (even and odd steps).  No host synchronisation happens between
 // steps; the host reads the history when it asks for it.  Serial mode runs the
 // same schedule through the eager entry points, one box after another -- the
 // plain form run in sequence, which graph mode must reproduce bit for bit.
@@ -132,6 +131,7 @@ int capture(cube_batch* b, int parity) {
   cudaError_t e = cudaEventRecord(b->fork, b->s0);
   for (int i = 0; i < b->nbox && !r && e == cudaSuccess; i++) {
     cube_ctx* c = b->box[i];
+    c->graph_slot = parity;
     e = cudaStreamWaitEvent(c->stream, b->fork, 0);
     if (e != cudaSuccess) break;
     r = box_step(c, c->p.ncell, b->sched + (size_t)i * b->nsteps, b->nsteps);
@@ -139,15 +139,6 @@ int capture(cube_batch* b, int parity) {
       b->err = "box " + std::to_string(i) + ": " + c->err;
       break;
     }
-    const size_t nv = (size_t)c->nvbin;
-    e = cudaMemcpyAsync(c->codec[0].dec, c->codec[1].dec, 8 * nv, cudaMemcpyDeviceToDevice, c->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(c->codec[0].dech, c->codec[1].dech, 8 * nv, cudaMemcpyDeviceToDevice, c->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(c->codec[0].decf, c->codec[1].decf, 4 * (nv / 2 + 1), cudaMemcpyDeviceToDevice, c->stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(c->codec[0].bnd, c->codec[1].bnd, 8 * (nv / 2 + 1), cudaMemcpyDeviceToDevice, c->stream);
-    if (e != cudaSuccess) break;
     k_batch_tail<<<1, 32, 0, c->stream>>>(c->sd, c->sout, b->hist, b->nbox, i, b->nsteps);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaEventRecord(b->join[i], c->stream);
@@ -293,14 +284,17 @@ int check_stats(cube_batch* b, int i, int k, const cube_batch_stats& s) {
 }
 
 int graph_steps(cube_batch* b, int n) {
+  // codec slot k0 & 1 holds the tables of the state's sigma before the first
+  // graph step, and before any later one that an eager call's tables came between
+  for (int i = 0; i < b->nbox; i++) {
+    cube_ctx* c = b->box[i];
+    const int slot = (int)(b->steps_done & 1);
+    if (b->g[0] && c->codec[slot].sigma == c->sigma_vi) continue;
+    int r = cube_codec_build_dev(c, slot, &c->sd->sigma_vi);
+    if (r) return bfail(b, r, c->err);
+    BCUDA(b, cudaStreamSynchronize(c->stream));
+  }
   if (!b->g[0]) {
-    for (int i = 0; i < b->nbox; i++) {
-      cube_ctx* c = b->box[i];
-      // codec slot 0 holds the tables of the state's sigma before the first graph step
-      int r = cube_codec_build_dev(c, 0, &c->sd->sigma_vi);
-      if (r) return bfail(b, r, c->err);
-      BCUDA(b, cudaStreamSynchronize(c->stream));
-    }
     for (int p = 0; p < 2; p++) {
       for (cube_ctx* c : b->box) c->graph_mode = true;
       int r = capture(b, p);
@@ -341,7 +335,12 @@ int graph_steps(cube_batch* b, int n) {
     restore(c, b->snap[last][i]);
     c->sigma_vi = c->sigma_vi_new = hs[i].sigma_vi;
     for (int d = 0; d < 3; d++) c->vmax_prev[d] = hs[i].vmax_prev[d];
-    c->codec[0].sigma = c->codec[1].sigma = hs[i].sigma_vi;
+    // the step's own sigma_vi tables are the other slot's
+    const int slot = (int)(b->steps_done & 1);
+    c->codec[slot].sigma = hs[i].sigma_vi;
+    c->codec[1 - slot].sigma = -1.f;
+    c->codec_next = 1 - slot;
+    c->codec_ahead = -1;
   }
   std::vector<StepOut> ho((size_t)n * b->nbox);
   BCUDA(b, cudaMemcpy(ho.data(), b->hist + (size_t)k0 * b->nbox, sizeof(StepOut) * ho.size(),

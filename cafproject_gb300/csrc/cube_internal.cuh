@@ -142,11 +142,18 @@ struct cube_ctx {
     int32_t* rt = nullptr;
   } codec[2];
   int codec_next = 0;
+  // the tables of the next sigma built beside the step, on a stream of their
+  // own (cube_codec_prefetch, and update_x of a captured step); slot, or -1
+  int codec_ahead = -1;
+  cudaStream_t stream_aux = nullptr;
+  cudaEvent_t ev_aux = nullptr, ev_codec = nullptr;
   float sigma_vi = 0.f, sigma_vi_new = 0.f;
   float vmax_prev[3] = {0.f, 0.f, 0.f};  // last coarse-kick vmax (0: unknown)
-  // graph mode (cube_batch_*): step scalars on the device, codec slot 0 holds
-  // sigma_vi and slot 1 sigma_vi_new, no host synchronisation inside a step
+  // graph mode (cube_batch_*): step scalars on the device, codec slot
+  // graph_slot holds sigma_vi and the other sigma_vi_new (they change places
+  // from step to step), no host synchronisation inside a step
   bool graph_mode = false;
+  int graph_slot = 0;
   StepDev* sd = nullptr;    // device
   StepOut* sout = nullptr;  // device (owned by the batch)
   unsigned long long kick_exact_lanes = 0;
@@ -695,6 +702,9 @@ __device__ __forceinline__ void for_box_particles(const int* pref, const long lo
 int cube_build_tables(cube_ctx* c);
 // decode/encode tables for up to two sigma values at once (built on demand)
 int cube_codec_pair(cube_ctx* c, float s1, float s2, CodecView* v1, CodecView* v2);
+// start building the tables of sigma on the auxiliary stream (the caller has
+// drained the context's streams); keep's slot stays
+int cube_codec_prefetch(cube_ctx* c, float sigma, float keep);
 // graph mode: tables of a slot from a device sigma; a view reading cf from the device
 int cube_codec_build_dev(cube_ctx* c, int slot, const float* sigp);
 void cube_codec_view_dev(const cube_ctx* c, int slot, const float* cfp, CodecView* v);

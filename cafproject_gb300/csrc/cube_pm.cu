@@ -839,9 +839,10 @@ int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool pre, bool with_
     k.pp_kd = (((double)a_mid * (double)dt) / 6.0) / (double)CUBE_PI_F;
     k.pp_kf = (float)k.pp_kd;
   }
-  if (c->graph_mode) {  // decode with sigma_vi (slot 0), encode with sigma_vi_new (slot 1)
-    cube_codec_view_dev(c, 0, &c->sd->h.cf_vi, &k.cin);
-    cube_codec_view_dev(c, 1, &c->sd->cf_new, &k.cout);
+  if (c->graph_mode) {  // decode with sigma_vi, encode with sigma_vi_new
+    CUBE_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_codec, 0));
+    cube_codec_view_dev(c, c->graph_slot, &c->sd->h.cf_vi, &k.cin);
+    cube_codec_view_dev(c, 1 - c->graph_slot, &c->sd->cf_new, &k.cout);
     k.sd = c->sd;
   } else {
     int r = cube_codec_pair(c, c->sigma_vi, c->sigma_vi_new, &k.cin, &k.cout);
@@ -949,9 +950,9 @@ int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
 int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool pre) {
   KickArgs k{};
   int r;
-  if (c->graph_mode) {  // sigma_vi is now sigma_vi_new (slot 1) for both
-    cube_codec_view_dev(c, 1, &c->sd->cf_new, &k.cin);
-    cube_codec_view_dev(c, 1, &c->sd->cf_new, &k.cout);
+  if (c->graph_mode) {  // sigma_vi is now sigma_vi_new for both
+    cube_codec_view_dev(c, 1 - c->graph_slot, &c->sd->cf_new, &k.cin);
+    cube_codec_view_dev(c, 1 - c->graph_slot, &c->sd->cf_new, &k.cout);
     k.sd = c->sd;
   } else {
     r = cube_codec_pair(c, c->sigma_vi, c->sigma_vi, &k.cin, &k.cout);
@@ -1036,6 +1037,7 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
   }
   r = cube_stats_fetch(c);
   if (r) return r;
+  c->codec_ahead = -1;  // the kicks waited for the tables and are done
   float vm[3];
   bool rerun = false;
   for (int d = 0; d < 3; d++) {

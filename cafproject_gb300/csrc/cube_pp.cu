@@ -922,7 +922,7 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
   PPArgs a{};
   int r;
   if (c->graph_mode) {
-    cube_codec_view_dev(c, 0, &c->sd->h.cf_vi, &a.cv);
+    cube_codec_view_dev(c, c->graph_slot, &c->sd->h.cf_vi, &a.cv);
     a.sd = c->sd;
   } else {
     r = cube_codec_pair(c, c->sigma_vi, c->sigma_vi, &a.cv, nullptr);

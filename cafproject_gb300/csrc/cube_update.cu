@@ -926,7 +926,7 @@ __global__ void __launch_bounds__(SF_THREADS) k_sigma_final(const double* __rest
   for (int t = 0; t < 3; t++) {
     s[t] = 0.0;
     for (int i = 0; i < SF_THREADS / 32; i++) s[t] += w[t][i];
-    st->sums[t] = s[t];
+    if (st) st->sums[t] = s[t];
   }
   if (!sd) return;
   const double std_res = sqrt(s[1] / npg);
@@ -957,7 +957,7 @@ static int update_x_graph(cube_ctx* c) {
   Geo g = make_geo(c);
   int k = c->cur, kn = 1 - k;
   CodecView cv;
-  cube_codec_view_dev(c, 0, &c->sd->h.cf_vi, &cv);
+  cube_codec_view_dev(c, c->graph_slot, &c->sd->h.cf_vi, &cv);
   CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), c->stream));
   UpdArgs a{};
   a.g = g;
@@ -1009,15 +1009,22 @@ static int update_x_graph(cube_ctx* c) {
   k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 16), 128, 0, s>>>(a);
   k_scatter<<<cube_grid(c->np, B), B, 0, s>>>(a);
   k_scatter_xtra<<<cube_grid(c->xtra_cap, B, 2), B, 0, s>>>(a);
-  const int nb = sigma_blocks(c, c->np);
-  k_sigma<<<nb, 256, 0, s>>>(c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, cv.dech, c->nvbin, c->p.izipv,
-                             c->red_tmp);
-  const double npg = (double)(c->npglobal > 0 ? c->npglobal : c->np);
-  k_sigma_final<<<1, SF_THREADS, 0, s>>>(c->red_tmp, nb, c->dstats, npg, c->sd, c->sout);
-  CUBE_CUDA(c, cudaGetLastError());
   CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->upd, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, s));
-  r = cube_codec_build_dev(c, 1, &c->sd->sigma_new);
+  // sigma_vi_new and its codec tables beside the densities and transforms: the
+  // fine kick is the first to need them (it waits for ev_codec)
+  CUBE_CUDA(c, cudaEventRecord(c->ev_aux, s));
+  CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_aux, c->ev_aux, 0));
+  const int nb = sigma_blocks(c, c->np);
+  k_sigma<<<nb, 256, 0, c->stream_aux>>>(c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, cv.dech, c->nvbin,
+                                         c->p.izipv, c->red_tmp);
+  const double npg = (double)(c->npglobal > 0 ? c->npglobal : c->np);
+  k_sigma_final<<<1, SF_THREADS, 0, c->stream_aux>>>(c->red_tmp, nb, nullptr, npg, c->sd, c->sout);
+  CUBE_CUDA(c, cudaGetLastError());
+  c->stream = c->stream_aux;
+  r = cube_codec_build_dev(c, 1 - c->graph_slot, &c->sd->sigma_new);
+  c->stream = s;
   if (r) return r;
+  CUBE_CUDA(c, cudaEventRecord(c->ev_codec, c->stream_aux));
   c->cur = kn;
   c->rank_walked = 0;
   return CUBE_OK;
@@ -1199,6 +1206,8 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   double npg = (double)(c->npglobal > 0 ? c->npglobal : np_new);
   double std_res = std::sqrt(sums[1] / npg);
   c->sigma_vi_new = (float)(std_res / (double)std::sqrt(3.0f));  // update_particle.f90:224
+  // its tables are built while PP and the transforms run; the fine kick needs them
+  if ((r = cube_codec_prefetch(c, c->sigma_vi_new, c->sigma_vi))) return r;
   if (st) {
     st->nplocal = np_new;
     st->max_tile_np = 0;
