@@ -68,6 +68,8 @@ static void release(cube_ctx* c) {
     c->plan_f_r2c = c->plan_f_c2r = c->plan_c_r2c = c->plan_c_c2r = 0;
     c->stream = nullptr;
   }
+  // the three force meshes are one allocation each
+  for (int d = 1; d < 3; d++) c->force_f[d] = c->force_c[d] = nullptr;
   void* bufs[] = {c->xp[0], c->xp[1], c->vp[0], c->vp[1], c->pid[0], c->pid[1], c->pcell[0], c->pcell[1],
                   c->rhoc[0], c->rhoc[1],
                   c->vfield[0], c->vfield[1], c->cstart[0], c->cstart[1], c->dest, c->dframe, c->doff, c->lrank, c->offc, c->perm, c->vdense, c->rank, c->xtra,
@@ -109,9 +111,26 @@ static int make_plans(cube_ctx* c) {
   for (cufftHandle h : {c->plan_f_r2c, c->plan_f_c2r, c->plan_c_r2c, c->plan_c_c2r})
     CUBE_FFT(c, cufftSetAutoAllocation(h, 0));
   CUBE_FFT(c, cufftMakePlan3d(c->plan_f_r2c, nf, nf, nf, CUFFT_R2C, &wf1));
-  CUBE_FFT(c, cufftMakePlan3d(c->plan_f_c2r, nf, nf, nf, CUFFT_C2R, &wf2));
   CUBE_FFT(c, cufftMakePlan3d(c->plan_c_r2c, nc, nc, nc, CUFFT_R2C, &wc1));
-  CUBE_FFT(c, cufftMakePlan3d(c->plan_c_c2r, nc, nc, nc, CUFFT_C2R, &wc2));
+  // Up to 224 points a dimension the three force components go through one
+  // batched plan: a third of the launches, and more blocks in each (64: 37 ->
+  // 19 us, 128: 62 -> 41, 200: 240 -> 222).  From 232 on the batch is no faster
+  // and sometimes slower (232: 407 -> 425, 264: 518 -> 586).  The same bits for
+  // every size compared (16 to 640).  Odd extents keep the single plan, whose
+  // default in-place layout differs there.
+  auto inverse = [&](cufftHandle h, int n, int* batch, size_t* w) -> int {
+    if (n > 224 || n % 2) {
+      CUBE_FFT(c, cufftMakePlan3d(h, n, n, n, CUFFT_C2R, w));
+      return CUBE_OK;
+    }
+    int dims[3] = {n, n, n}, in[3] = {n, n, n / 2 + 1}, out[3] = {n, n, n + 2};
+    const int pad = (n + 2) * n * n;
+    CUBE_FFT(c, cufftMakePlanMany(h, 3, dims, in, 1, pad / 2, out, 1, pad, CUFFT_C2R, 3, w));
+    *batch = 3;
+    return CUBE_OK;
+  };
+  if (int r = inverse(c->plan_f_c2r, nf, &c->f_c2r_batch, &wf2)) return r;
+  if (int r = inverse(c->plan_c_c2r, nc, &c->c_c2r_batch, &wc2)) return r;
   size_t w = wf1;
   for (size_t x : {wf2, wc1, wc2})
     if (x > w) w = x;
@@ -225,12 +244,14 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
     int64_t nfh = (int64_t)(c->nf / 2 + 1);
     int64_t fpad = 2 * nfh * c->nf * (int64_t)c->nf;  // floats of a padded fine mesh
     ALLOC(c->rho_f, 4 * fpad);
-    for (int d = 0; d < 3; d++) ALLOC(c->force_f[d], 4 * fpad);
+    ALLOC(c->force_f[0], 3 * 4 * fpad);  // one after another, for the batched transform
+    for (int d = 1; d < 3; d++) c->force_f[d] = c->force_f[0] + d * fpad;
     ALLOC(c->kern_f, 4 * 3 * nfh * c->nf * (int64_t)c->nf);
     int64_t nch = (int64_t)(p->nc / 2 + 1);
-    int64_t cpad = 2 * nch * p->nc * (int64_t)p->nc;
+    int64_t cpad = (int64_t)(p->nc + 2) * p->nc * (int64_t)p->nc;  // the kernels' row stride, for odd nc too
     ALLOC(c->rho_c, 4 * cpad);
-    for (int d = 0; d < 3; d++) ALLOC(c->force_c[d], 4 * cpad);
+    ALLOC(c->force_c[0], 3 * 4 * cpad);
+    for (int d = 1; d < 3; d++) c->force_c[d] = c->force_c[0] + d * cpad;
     ALLOC(c->kern_c, 4 * 3 * nch * p->nc * (int64_t)p->nc);
   }
   if (p->pp_on) {
@@ -281,6 +302,8 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
     c->plan_f_c2r = owner->plan_f_c2r;
     c->plan_c_r2c = owner->plan_c_r2c;
     c->plan_c_c2r = owner->plan_c_c2r;
+    c->f_c2r_batch = owner->f_c2r_batch;
+    c->c_c2r_batch = owner->c_c2r_batch;
     c->cufft_work = owner->cufft_work;
     c->cufft_work_bytes = owner->cufft_work_bytes;
   } else {

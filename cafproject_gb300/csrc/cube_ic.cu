@@ -512,13 +512,18 @@ static int ic_impl(cube_ctx* c, const cube_cosmology* cs, float z_init, uint32_t
   sa.ck = (float2*)c->rho_f;
   k_ic_scale<<<cube_grid(nspec, 256), 256, 0, s>>>(sa);
   CUBE_CUDA(c, cudaGetLastError());
-  CUBE_FFT(c, cufftExecC2R(c->plan_f_c2r, (cufftComplex*)c->rho_f, c->rho_f));
+  float* phi = c->rho_f;
+  if (c->f_c2r_batch > 1) {  // a batched plan takes the force planes; what the other two hold is done with
+    phi = c->force_f[0];
+    CUBE_CUDA(c, cudaMemcpyAsync(phi, c->rho_f, 8 * (size_t)nspec, cudaMemcpyDeviceToDevice, s));
+  }
+  CUBE_FFT(c, cufftExecC2R(c->plan_f_c2r, (cufftComplex*)phi, phi));
   // 4. particles on the Lagrangian grid
   int32_t* cid = c->dest;
   double* vel = fits ? reinterpret_cast<double*>(c->force_f[1]) : static_cast<double*>(own.p);
   CUBE_CUDA(c, cudaMemsetAsync(c->rhoc[k], 0, 4 * (size_t)c->ncells, s));
   CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), s));
-  PartArgs pa{c->rho_f, nf, nc, c->nt, p.nnt, cs->np_nc, p.ncell / cs->np_nc, p.ncell, p.izipx,
+  PartArgs pa{phi, nf, nc, c->nt, p.nnt, cs->np_nc, p.ncell / cs->np_nc, p.ncell, p.izipx,
               1.0f / ((float)nf * nf * nf), vfactor(a, cs->omega_m, cs->omega_l), cid, c->xp[alt], vel, c->rhoc[k],
               c->dstats->vmax_bits};
   k_ic_particles<<<cube_grid(n, 256), 256, 0, s>>>(pa, make_geo(c));

@@ -163,11 +163,12 @@ struct cube_ctx {
   int opt_pp_level = 0;  // first PP level (0-5)
   int opt_pp_heavy = 0;  // PP: entries from which a crowded block walks a particle with a warp (0: default)
   int opt_pp_parts = 0;  // PP: most parts a dense item is split into (0: default, 255)
-  int opt_dep_fine = 0, opt_dep_coarse = 0;  // deposit brick shapes (0-3)
+  int opt_dep_fine = -1, opt_dep_coarse = -1;  // deposit brick shapes (0-3; -1: by the mesh)
   int fail_alloc = 0;    // host fault injection: the n-th lazy allocation fails (0: off)
   cube_ctx* linked = nullptr;  // the second species linked to this context, if any
   // fine PM
   cufftHandle plan_f_r2c = 0, plan_f_c2r = 0;
+  int f_c2r_batch = 1, c_c2r_batch = 1;  // meshes an inverse plan takes at once: 1, or (small meshes) the three forces
   float* rho_f = nullptr;       // padded real / complex in place
   float* force_f[3] = {nullptr, nullptr, nullptr};
   float* kern_f = nullptr;      // 3 planes of (nf/2+1)*nf*nf, scaled by 1/nf^3

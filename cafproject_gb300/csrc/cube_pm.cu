@@ -277,9 +277,22 @@ int launch_deposit(cube_ctx* c, const DepArgs& a) {
 // The deposits' brick shapes (cube_set_option CUBE_OPT_DEPOSIT_FINE / _COARSE):
 // larger bricks re-read fewer neighbour particles, smaller ones hold less
 // shared memory per CTA (more CTAs per SM) and give small meshes more CTAs.
-// Every shape writes the same exact fixed-point sums.
+// Every shape writes the same exact fixed-point sums.  Unless one is set, the
+// number of 8x4x4 (8x8x8) bricks decides: below one a multiprocessor the smallest
+// bricks fill the chip (nc 24: 16 against 24 us fine, 22 against 53 coarse), above
+// it they re-read too many neighbours (nc 64: 105 against 83, 92 against 77).  The
+// fine deposit then takes the half-high brick (nc 48: 45 against 48 us, nc 256:
+// 4.53 against 4.58 ms); the coarse one takes it up to three bricks a
+// multiprocessor (nc 48: 52 against 72, nc 64: 76.5 against 78.6, nc 96: 189
+// against 173).
+int default_bricks(const cube_ctx* c, int bx, int by, int bz) {
+  const int nc = c->p.nc;
+  return ((nc + bx - 1) / bx) * ((nc + by - 1) / by) * ((nc + bz - 1) / bz);
+}
 int launch_fine_deposit(cube_ctx* c, const DepArgs& a) {
-  switch (c->opt_dep_fine) {
+  int shape = c->opt_dep_fine;
+  if (shape < 0) shape = default_bricks(c, 8, 4, 4) < 152 ? 3 : 2;
+  switch (shape) {
     case 1: return launch_deposit<4, 4, 4, 4, 1, 0>(c, a);  // 16^3 fine cells, 32 KB
     case 2: return launch_deposit<4, 8, 4, 2, 1, 0>(c, a);  // 32x16x8, 32 KB
     case 3: return launch_deposit<4, 4, 4, 2, 1, 0>(c, a);  // 16x16x8, 16 KB
@@ -287,7 +300,12 @@ int launch_fine_deposit(cube_ctx* c, const DepArgs& a) {
   }
 }
 int launch_coarse_deposit(cube_ctx* c, const DepArgs& a) {
-  switch (c->opt_dep_coarse) {
+  int shape = c->opt_dep_coarse;
+  if (shape < 0) {
+    const int nb = default_bricks(c, 8, 8, 8);
+    shape = nb < 152 ? 3 : (nb < 3 * 152 ? 2 : 0);
+  }
+  switch (shape) {
     case 1: return launch_deposit<1, 16, 8, 8, 1, 1>(c, a);
     case 2: return launch_deposit<1, 8, 8, 4, 1, 1>(c, a);
     case 3: return launch_deposit<1, 4, 4, 4, 1, 1>(c, a);
@@ -308,8 +326,10 @@ __global__ void k_green3(const float2* __restrict__ rk, const float* __restrict_
   }
 }
 
-// maxval(sum(force**2,1)) over the mesh (pm.f90:126, 315): one block per row
-// (y, z) at a time, float2 loads along x (rows start 8-byte aligned: stride n+2)
+// maxval(sum(force**2,1)) over the mesh (pm.f90:126, 315): float2 loads along x
+// (rows start 8-byte aligned: stride n+2), blockDim.y rows (y, z) at a time, as
+// many as fill a block of 256 threads (a row a block left three quarters of the
+// threads of a 128^3 mesh idle: 12.6 -> 8.1 us)
 __device__ __forceinline__ float f2sum(float a, float b, float c) {
   return __fadd_rn(__fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b)), __fmul_rn(c, c));
 }
@@ -327,7 +347,7 @@ __global__ void k_f2max(float* __restrict__ f0, float* __restrict__ f1, float* _
   const int64_t rows = (int64_t)n * n;
   const int h = n >> 1;
   float m = 0.f;
-  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+  for (int64_t r = blockIdx.x * (int64_t)blockDim.y + threadIdx.y; r < rows; r += (int64_t)gridDim.x * blockDim.y) {
     const int64_t o = r * (n + 2);
     float2* a = reinterpret_cast<float2*>(f0 + o);
     float2* b = reinterpret_cast<float2*>(f1 + o);
@@ -352,7 +372,17 @@ __global__ void k_f2max(float* __restrict__ f0, float* __restrict__ f1, float* _
     }
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomic_max_pos(out, m);
+  if ((threadIdx.x & 31) == 0 && m > 0.f) atomic_max_pos(out, m);
+}
+
+// the maxima pass over n^3 cells of three padded meshes
+template <bool kPre>
+void launch_f2max(cube_ctx* c, float* const f[3], int n, unsigned int* out, const float* pre) {
+  int bx = 32;
+  while (bx < 256 && bx < n / 2) bx *= 2;
+  const dim3 block(bx, 256 / bx);
+  k_f2max<kPre><<<cube_grid((int64_t)n * n, (int)block.y, 8), block, 0, c->stream>>>(
+      f[0], f[1], f[2], n, out, kPre ? pre[0] : 0.f, kPre ? pre[1] : 0.f, kPre && c->graph_mode ? c->sd : nullptr);
 }
 
 // ------------------------------------------------------------------- kicks
@@ -807,16 +837,14 @@ int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
                                                   (float2*)c->force_f[1], (float2*)c->force_f[2]);
   cube_phase_end(c, PH_F_GREEN);
   cube_phase_begin(c, PH_F_C2R);
-  for (int d = 0; d < 3; d++)
+  for (int d = 0; d < 3; d += c->f_c2r_batch)
     CUBE_FFT(c, cufftExecC2R(c->plan_f_c2r, (cufftComplex*)c->force_f[d], c->force_f[d]));
   cube_phase_end(c, PH_F_C2R);
   cube_phase_begin(c, PH_F_F2MAX);
   if (pre)
-    k_f2max<true><<<cube_grid((int64_t)c->nf * c->nf, 1, 8), 256, 0, s>>>(
-        c->force_f[0], c->force_f[1], c->force_f[2], c->nf, &c->dstats->f2_fine_bits, pre[0], pre[1], c->graph_mode ? c->sd : nullptr);
+    launch_f2max<true>(c, c->force_f, c->nf, &c->dstats->f2_fine_bits, pre);
   else
-    k_f2max<false><<<cube_grid((int64_t)c->nf * c->nf, 1, 8), 256, 0, s>>>(
-        c->force_f[0], c->force_f[1], c->force_f[2], c->nf, &c->dstats->f2_fine_bits, 0.f, 0.f, nullptr);
+    launch_f2max<false>(c, c->force_f, c->nf, &c->dstats->f2_fine_bits, nullptr);
   cube_phase_end(c, PH_F_F2MAX);
   CUBE_CUDA(c, cudaGetLastError());
   if (st) {
@@ -928,14 +956,12 @@ int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
   CUBE_FFT(c, cufftExecR2C(c->plan_c_r2c, c->rho_c, (cufftComplex*)c->rho_c));
   k_green3<<<cube_grid(cspec, 256), 256, 0, s>>>((const float2*)c->rho_c, c->kern_c, cspec, (float2*)c->force_c[0],
                                                   (float2*)c->force_c[1], (float2*)c->force_c[2]);
-  for (int d = 0; d < 3; d++)
+  for (int d = 0; d < 3; d += c->c_c2r_batch)
     CUBE_FFT(c, cufftExecC2R(c->plan_c_c2r, (cufftComplex*)c->force_c[d], c->force_c[d]));
   if (pre)
-    k_f2max<true><<<cube_grid((int64_t)nc * nc, 1, 8), 256, 0, s>>>(c->force_c[0], c->force_c[1], c->force_c[2], nc,
-                                                                    &c->dstats->f2_coarse_bits, pre[0], pre[1], c->graph_mode ? c->sd : nullptr);
+    launch_f2max<true>(c, c->force_c, nc, &c->dstats->f2_coarse_bits, pre);
   else
-    k_f2max<false><<<cube_grid((int64_t)nc * nc, 1, 8), 256, 0, s>>>(c->force_c[0], c->force_c[1], c->force_c[2], nc,
-                                                                     &c->dstats->f2_coarse_bits, 0.f, 0.f, nullptr);
+    launch_f2max<false>(c, c->force_c, nc, &c->dstats->f2_coarse_bits, nullptr);
   cube_phase_end(c, PH_C_FFT);
   CUBE_CUDA(c, cudaGetLastError());
   if (st) {
