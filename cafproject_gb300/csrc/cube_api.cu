@@ -76,7 +76,7 @@ static void release(cube_ctx* c) {
                   c->scan_tmp, c->red_tmp, c->tan_tab, c->codec[0].dec, c->codec[1].dec, c->codec[0].bnd, c->codec[1].bnd, c->codec[0].dech, c->codec[1].dech, c->codec[0].decf, c->codec[1].decf, c->codec[0].rt, c->codec[1].rt, c->rho_f, c->force_f[0],
                   c->force_f[1], c->force_f[2], c->kern_f, c->kern_f_raw, c->rho_c, c->force_c[0],
                   c->force_c[1], c->force_c[2], c->kern_c, c->fpp, c->pp_list[0], c->pp_list[1], c->pp_list[2], c->pp_list[3], c->pp_list[4], c->pp_scr_pts,
-                  c->pp_lpart[0], c->pp_lpart[1], c->pp_lpart[2], c->pp_lpart[3], c->pp_lpart[4], c->pp_nlist, c->dstats,
+                  c->pp_lpart[0], c->pp_lpart[1], c->pp_lpart[2], c->pp_lpart[3], c->pp_lpart[4], c->red_count, c->dstats,
                   c->pp_occ, c->pp_act, c->pp_wcnt, c->pp_wstart, c->pp_arhoc, c->pp_acstart, c->pp_aidx,
                   c->cufft_work};
   for (void* b : bufs)
@@ -92,7 +92,6 @@ static void release(cube_ctx* c) {
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_pp) cudaEventDestroy(c->ev_pp);
   if (c->stream_pp) cudaStreamDestroy(c->stream_pp);
-  if (c->pp_nlist_host) cudaFreeHost(c->pp_nlist_host);
   if (c->plan_f_r2c) cufftDestroy(c->plan_f_r2c);
   if (c->plan_f_c2r) cufftDestroy(c->plan_f_c2r);
   if (c->plan_c_r2c) cufftDestroy(c->plan_c_r2c);
@@ -223,6 +222,8 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
   ALLOC(c->scan_tmp, c->scan_tmp_bytes);
   c->red_blocks = 2048;
   ALLOC(c->red_tmp, sizeof(double) * 4 * c->red_blocks);
+  ALLOC(c->red_count, sizeof(unsigned));
+  CUBE_CUDA(c, cudaMemsetAsync(c->red_count, 0, sizeof(unsigned), c->stream));
   ALLOC(c->tan_tab, 4 * c->nvbin);
   for (int k = 0; k < 2; k++) {
     ALLOC(c->codec[k].dec, 8 * c->nvbin);
@@ -290,9 +291,6 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
       ALLOC(c->pp_list[l], 4 * cap);
       ALLOC(c->pp_lpart[l], 4 * cap);
     }
-    ALLOC(c->pp_nlist, 64);
-    CUBE_CUDA(c, cudaMallocHost((void**)&c->pp_nlist_host, 32));
-    for (int l = 0; l < 5; l++) c->pp_nlist_host[l] = 0;
   }
   ALLOC(c->dstats, sizeof(DevStats));
   CUBE_CUDA(c, cudaMallocHost((void**)&c->hstats, sizeof(DevStats)));
@@ -456,8 +454,8 @@ extern "C" int cube_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_stats
   if ((r = cube_fine_forces_impl(c, st, pre))) return r;
   if ((r = cube_fine_kick_impl(c, a_mid, dt, true))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
-  if ((r = cube_coarse_forces_impl(c, st, pre))) return r;
-  return cube_coarse_kick_impl(c, a_mid, dt, st, true);
+  if ((r = cube_coarse_forces_impl(c, st, pre, true))) return r;
+  return cube_coarse_kick_impl(c, a_mid, dt, st, true, true);
 }
 
 // ext_pp_force followed by particle_mesh (main.f90:113-116) with PP on a
@@ -486,12 +484,12 @@ extern "C" int cube_pp_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_st
     if (r) return r;
   }
   if ((r = cube_fine_forces_impl(c, st_pm, pre))) return r;
-  if ((r = cube_coarse_forces_impl(c, st_pm, pre))) return r;
+  if ((r = cube_coarse_forces_impl(c, st_pm, pre, true))) return r;
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_pp, 0));
   // the fine kick applies PP's kick first (ext_pp_force.f90:116-121), then its own
   if ((r = cube_fine_kick_impl(c, a_mid, dt, true, /*with_pp=*/true))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
-  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st_pm, true))) return r;
+  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st_pm, true, true))) return r;
   {  // PP's stats (its stream is done: the kicks waited for it)
     cudaStream_t s0 = c->stream;
     DevStats *d0 = c->dstats, *h0 = c->hstats;
@@ -524,11 +522,11 @@ extern "C" int cube_particle_mesh2(cube_ctx* c, cube_ctx* nu, float a_mid, float
   if ((r = cube_fine_kick_impl(nu, a_mid, dt, true))) return cube_fail(c, r, nu->err);
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193-194
   nu->sigma_vi = nu->sigma_vi_new;
-  if ((r = cube_coarse_density_impl(c, nullptr, false))) return r;
-  if ((r = cube_coarse_density_impl(nu, nullptr, true))) return cube_fail(c, r, nu->err);
+  if ((r = cube_coarse_density_impl(c, nullptr, false, true))) return r;
+  if ((r = cube_coarse_density_impl(nu, nullptr, true, true))) return cube_fail(c, r, nu->err);
   if ((r = cube_coarse_spectral_impl(c, st, pre))) return r;
-  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true))) return r;
-  if ((r = cube_coarse_kick_impl(nu, a_mid, dt, st_nu, true))) return cube_fail(c, r, nu->err);
+  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true, true))) return r;
+  if ((r = cube_coarse_kick_impl(nu, a_mid, dt, st_nu, true, true))) return cube_fail(c, r, nu->err);
   // testrhof / testrhoc sum both species' mass (pm.f90:108, 258); the coarse
   // kick left the second species' deposited masses in its host stats
   if (st) {

@@ -120,8 +120,8 @@ int box_step(cube_ctx* c, int ncell, const float2* sched, int nsteps) {
   const float pre[2] = {0.f, 0.f};
   if ((r = cube_fine_forces_impl(c, nullptr, pre))) return r;
   if ((r = cube_fine_kick_impl(c, 0.f, 0.f, true))) return r;
-  if ((r = cube_coarse_forces_impl(c, nullptr, pre))) return r;
-  return cube_coarse_kick_impl(c, 0.f, 0.f, nullptr, true);
+  if ((r = cube_coarse_forces_impl(c, nullptr, pre, true))) return r;
+  return cube_coarse_kick_impl(c, 0.f, 0.f, nullptr, true, true);
 }
 
 int capture(cube_batch* b, int parity) {

@@ -38,7 +38,6 @@ struct DevStats {
   unsigned long long npairs, itest1;
   unsigned long long ndup_list;  // entries in the extra-copy list
   unsigned int ndense;           // destination cells left to the warp-per-cell vfield pass
-  unsigned long long nexact;     // kick lanes evaluated on the exact FP64 chain
   unsigned int vmax_est_bits[3]; // fine kick: max |v + vfield| in FP32, when the last vmax is unknown
   double testrhof, testrhoc;
   unsigned long long rhof_fix, rhoc_fix;  // deposited mass in 2^-32 fixed point
@@ -47,6 +46,7 @@ struct DevStats {
   unsigned int vmax_lo_bits[3];           // coarse kick: max of certified lower bounds of |v + vfield|
   unsigned long long pp_active;           // PP prefilter: particles with a neighbour besides themselves
   double sums[3];                         // update_x: the sigma_v sums (update_particle.f90:172-196)
+  int pp_nlist[11];  // PP: lengths of the levels' lists (5), then each level's next-item counter (6)
 };
 
 // share of the last step's vmax above which the coarse kick evaluates a
@@ -128,6 +128,7 @@ struct cube_ctx {
   void* scan_tmp = nullptr;
   size_t scan_tmp_bytes = 0;
   double* red_tmp = nullptr;    // block partial sums for sigma statistics
+  unsigned* red_count = nullptr;  // blocks of k_sigma done (zero between launches)
   int red_blocks = 0;
   // velocity code tables
   float* tan_tab = nullptr;     // float(tan(pi*v/(nvbin-1))) for v in [-nvbin/2, nvbin/2)
@@ -156,7 +157,6 @@ struct cube_ctx {
   int graph_slot = 0;
   StepDev* sd = nullptr;    // device
   StepOut* sout = nullptr;  // device (owned by the batch)
-  unsigned long long kick_exact_lanes = 0;
   int opt_exact_kicks = 0;
   int opt_rank_walk = 0;   // ranks: 0 counting path (sort when it does not apply), 1 walker, 2 sort
   int rank_walked = 0;     // the last update used the walker
@@ -184,8 +184,6 @@ struct cube_ctx {
   int* pp_lpart[5] = {nullptr, nullptr, nullptr, nullptr, nullptr}; // their items' parts and claims
   float4* pp_scr_pts = nullptr;  // PP global staging (levels 4-5): pp_scr_cap float4, then 2 x pp_scr_cap uint32
   int64_t pp_scr_cap = 0;
-  int* pp_nlist = nullptr;          // their lengths
-  int* pp_nlist_host = nullptr;     // pinned copy of the last call's lengths
   int pp_brick_cap = 0;             // ceil(nc/4)^3
   // PP's prefilter (cube_pp.cu): a particle whose 27 neighbouring fine cells
   // hold no other particle has a zero pair force and a one-entry list; the
@@ -719,7 +717,8 @@ int cube_pp_init(cube_ctx* c);  // once per context: the staging kernels' shared
 int cube_pp_finish(cube_ctx* c, cube_stats* st);
 // density deposits; accumulate: add to the mesh (the linked species) instead of writing it
 int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false);
-int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false);
+// fresh (the coarse stages): the stats were zeroed by this step's fine density
+int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false, bool fresh = false);
 // pre (a_mid, dt) non-null: after the maxima, the force meshes are rewritten
 // as the mesh part of the kick term, force*a_mid*dt/6/pi, and the kick that
 // follows is given pre=true (fused step only; the stage calls keep forces)
@@ -727,8 +726,8 @@ int cube_fine_forces_impl(cube_ctx* c, cube_stats* st, const float* pre = nullpt
 // with_pp: first apply the PP kick that cube_pp_launch(.., defer_kick) left
 // to the fine kick (eager mode)
 int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool pre = false, bool with_pp = false);
-int cube_coarse_forces_impl(cube_ctx* c, cube_stats* st, const float* pre = nullptr);
-int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool pre = false);
+int cube_coarse_forces_impl(cube_ctx* c, cube_stats* st, const float* pre = nullptr, bool fresh = false);
+int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool pre = false, bool fresh = false);
 int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre);
 int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre);
 int cube_pk_deposit(cube_ctx* c, int ng, float* rho, unsigned long long* total);

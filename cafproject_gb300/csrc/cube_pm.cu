@@ -404,7 +404,6 @@ struct KickArgs {
   unsigned int* vmax_lo;   // coarse kick: the largest lower bound of |v+vfield| (certain to be <= vmax)
   int vmax_only;           // rerun for the exact vmax (write nothing): lanes whose bound reaches vmax_lo
   int exact_only;          // skip the certified fast path
-  unsigned long long* nexact;
   const StepDev* sd;       // graph mode: a_mid, dt, tau from the device
   unsigned int* vmax_est;        // fine kick: record max |v + vfield| (FP32) here when set
   const unsigned int* tau_est;   // coarse kick: tau = 0.7 of this estimate when set
@@ -562,7 +561,6 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
   int qn = 0;                      // queued entries of this warp (warp-uniform)
   float vm[3] = {0.f, 0.f, 0.f};  // coarse: exact vmax; fine: the FP32 estimate
   float vlo[3] = {0.f, 0.f, 0.f};  // coarse: lower bounds of |v + vfield|
-  unsigned long long nex = 0;
   // the zero-kick codes are the codes themselves, but for -nvbin/2, when the
   // table's count says so
   const bool rt_same = kFine && a.pp_act && __ldg(a.cin.rt + 2 * a.cin.half) == 0;
@@ -628,7 +626,6 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
         if (qn >= 32) {
           __syncwarp();
           kick_exact_entry<kFine, kPre>(a, s_q[wq][qn - 32 + lane], vm);
-          nex++;
           qn -= 32;
           __syncwarp();
         }
@@ -638,7 +635,6 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
   __syncwarp();
   if (lane < qn) {
     kick_exact_entry<kFine, kPre>(a, s_q[wq][lane], vm);
-    nex++;
   }
   if (!kFine || a.vmax_est) {
     for (int d = 0; d < 3; d++) {
@@ -654,8 +650,6 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
       if ((threadIdx.x & 31) == 0 && m > 0.f) atomic_max_pos(&a.vmax_lo[d], m);
     }
   }
-  for (int o = 16; o > 0; o >>= 1) nex += __shfl_xor_sync(0xffffffffu, nex, o);
-  if ((threadIdx.x & 31) == 0 && a.nexact) atomicAdd(a.nexact, nex);
 }
 
 }  // namespace
@@ -889,7 +883,6 @@ int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool pre, bool with_
   k.a_mid = a_mid;
   k.dt = dt;
   k.vmax_bits = nullptr;
-  k.nexact = &c->dstats->nexact;
   k.exact_only = c->opt_exact_kicks;
   // after an upload or initial conditions the last vmax is unknown: the fine
   // kick then records the velocities' maxima for the coarse kick's threshold
@@ -921,10 +914,12 @@ int cube_pk_deposit(cube_ctx* c, int ng, float* rho, unsigned long long* total) 
 }
 
 // --------------------------------------------------------------- coarse
-int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate) {
+int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate, bool fresh) {
   Geo g = make_geo(c);
-  CUBE_CUDA(c, cudaMemsetAsync(&c->dstats->f2_coarse_bits, 0, 4, c->stream));
-  CUBE_CUDA(c, cudaMemsetAsync(&c->dstats->rhoc_fix, 0, 8, c->stream));
+  if (!fresh) {
+    CUBE_CUDA(c, cudaMemsetAsync(&c->dstats->f2_coarse_bits, 0, 4, c->stream));
+    CUBE_CUDA(c, cudaMemsetAsync(&c->dstats->rhoc_fix, 0, 8, c->stream));
+  }
   const int sh = dep_shift(c->p.mass_p);
   DepArgs a{g, c->xp[c->cur], c->rhoc[c->cur], c->cstart[c->cur], c->p.mass_p, c->rho_c, &c->dstats->rhoc_fix, 0,
             std::ldexp(1.0f, sh), std::ldexp(1.0f, -sh), accumulate ? 1 : 0};
@@ -940,8 +935,8 @@ int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate) {
   return CUBE_OK;
 }
 
-int cube_coarse_forces_impl(cube_ctx* c, cube_stats* st, const float* pre) {
-  int r0 = cube_coarse_density_impl(c, nullptr, false);
+int cube_coarse_forces_impl(cube_ctx* c, cube_stats* st, const float* pre, bool fresh) {
+  int r0 = cube_coarse_density_impl(c, nullptr, false, fresh);
   if (r0) return r0;
   return cube_coarse_spectral_impl(c, st, pre);
 }
@@ -973,7 +968,7 @@ int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
   return CUBE_OK;
 }
 
-int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool pre) {
+int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool pre, bool fresh) {
   KickArgs k{};
   int r;
   if (c->graph_mode) {  // sigma_vi is now sigma_vi_new for both
@@ -985,9 +980,10 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
     if (r) return r;
   }
   int cur = c->cur, alt = 1 - cur;
-  CUBE_CUDA(c, cudaMemsetAsync(c->dstats->vmax_bits, 0, 12, c->stream));
-  CUBE_CUDA(c, cudaMemsetAsync(c->dstats->vmax_lo_bits, 0, 12, c->stream));
-  CUBE_CUDA(c, cudaMemsetAsync(&c->dstats->nexact, 0, 8, c->stream));
+  if (!fresh) {
+    CUBE_CUDA(c, cudaMemsetAsync(c->dstats->vmax_bits, 0, 12, c->stream));
+    CUBE_CUDA(c, cudaMemsetAsync(c->dstats->vmax_lo_bits, 0, 12, c->stream));
+  }
   k.g = make_geo(c);
   k.np = c->np;
   k.xp = c->xp[cur];
@@ -1011,7 +1007,6 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
   k.dt = dt;
   k.vmax_bits = c->dstats->vmax_bits;
   k.vmax_lo = c->dstats->vmax_lo_bits;
-  k.nexact = &c->dstats->nexact;
   k.vmax_only = 0;
   k.exact_only = c->opt_exact_kicks;
   cube_phase_begin(c, PH_C_KICK);
@@ -1071,7 +1066,6 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
     const float tau = est ? 0.7f * bits_float(c->hstats->vmax_est_bits[d]) : k.tau[d];
     if (!(vm[d] >= tau)) rerun = true;
   }
-  unsigned long long nex = c->hstats->nexact;
   if (rerun) {
     CUBE_CUDA(c, cudaMemsetAsync(c->dstats->vmax_bits, 0, 12, c->stream));
     k.vmax_only = 1;
@@ -1088,7 +1082,6 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
   c->vp[cur] = c->vp[alt];
   c->vp[alt] = t;
   for (int d = 0; d < 3; d++) c->vmax_prev[d] = vm[d];
-  c->kick_exact_lanes = nex;
   if (st) {
     for (int d = 0; d < 3; d++) st->vmax[d] = vm[d];
     st->f2_max_coarse = bits_float(c->hstats->f2_coarse_bits);

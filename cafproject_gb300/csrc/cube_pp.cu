@@ -766,8 +766,14 @@ __device__ __forceinline__ void sub_cell(const void* xp, int64_t p, int izipx, i
 }
 
 // a cell's occupied sub-cells and those held twice or more: one thread per
-// coarse cell over its particles (no atomics; every cell's words written)
+// coarse cell over its particles (no atomics; every cell's words written); and
+// the activity words and counts zeroed for k_pp_nbmask
 __global__ void __launch_bounds__(256) k_pp_occ(PPFilter f) {
+  const int64_t nw = (f.np + 31) / 32;
+  for (int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < nw; w += (int64_t)gridDim.x * blockDim.x) {
+    f.act[w] = 0u;
+    f.wcnt[w] = 0;
+  }
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < f.ncells; c += (int64_t)gridDim.x * blockDim.x) {
     const int n = __ldg(f.rhoc + c);
     const int64_t p0 = __ldg(f.cstart + c);
@@ -848,7 +854,7 @@ __global__ void __launch_bounds__(256) k_pp_nbmask(PPFilter f) {
       e |= l;
     }
     // then the cell's own particles: active where their sub-cell's bit is
-    // set (act and wcnt zeroed before the launch)
+    // set (k_pp_occ zeroed act and wcnt)
     const unsigned long long a = e | __ldg(f.occ + f.ncells + c);
     const int n = __ldg(f.rhoc + c);
     const int64_t p0 = __ldg(f.cstart + c);
@@ -952,12 +958,11 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
   }
   a.heavy = c->opt_pp_heavy > 0 ? c->opt_pp_heavy : PP_HEAVY;
   a.max_parts = c->opt_pp_parts > 0 ? c->opt_pp_parts : 255;
-  a.nlist = c->pp_nlist;
+  a.nlist = c->dstats->pp_nlist;  // zeroed with the stats
   a.scr_cap = c->pp_scr_cap;
   a.scr_pts = c->pp_scr_pts;
   a.scr_kinfo = reinterpret_cast<unsigned*>(c->pp_scr_pts + c->pp_scr_cap);
   a.scr_order = a.scr_kinfo + c->pp_scr_cap;
-  CUBE_CUDA(c, cudaMemsetAsync(c->pp_nlist, 0, 11 * sizeof(int), c->stream));
   a.pidx = nullptr;
   a.act = nullptr;
   a.nact = nullptr;
@@ -987,8 +992,6 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
     f.st = c->dstats;
     const int64_t nw = (c->np + 31) / 32;
     k_pp_occ<<<cube_grid(c->ncells, 256), 256, 0, c->stream>>>(f);
-    CUBE_CUDA(c, cudaMemsetAsync(c->pp_act, 0, 4 * (size_t)nw, c->stream));
-    CUBE_CUDA(c, cudaMemsetAsync(c->pp_wcnt, 0, 4 * (size_t)nw, c->stream));
     k_pp_nbmask<<<cube_grid(c->ncells, 256), 256, 0, c->stream>>>(f);
     if (c->np > 0) {
       r = cube_scan_counts(c, c->pp_wcnt, c->pp_wstart, nw);
@@ -1008,11 +1011,11 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
   const int start = c->opt_pp_level;
   if (start == 1 || start == 2)
     k_pp_list_all<<<cube_grid(nbrick, 256), 256, 0, c->stream>>>(c->pp_list[start - 1], c->pp_lpart[start - 1],
-                                                                 (int)nbrick, c->pp_nlist + start - 1,
+                                                                 (int)nbrick, a.nlist + start - 1,
                                                                  start == 1 ? 3 : 1);
   else if (start >= 3)  // cells
     k_pp_list_all<<<cube_grid(c->ncells, 256), 256, 0, c->stream>>>(c->pp_list[start - 1], c->pp_lpart[start - 1],
-                                                                     (int)c->ncells, c->pp_nlist + start - 1,
+                                                                     (int)c->ncells, a.nlist + start - 1,
                                                                      start == 5 ? 1 : 3);
   if (start <= 0) {
     if (c->pp_act_valid && !c->graph_mode && c->pp_active_frac < PP_SPARSE_FRAC)
@@ -1041,7 +1044,6 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
     CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->pp, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, c->stream));
     return CUBE_OK;
   }
-  CUBE_CUDA(c, cudaMemcpyAsync(c->pp_nlist_host, c->pp_nlist, 5 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   return CUBE_OK;
 }
 
@@ -1078,7 +1080,7 @@ int cube_pp_finish(cube_ctx* c, cube_stats* st) {
     st->f2_max_pp = bits_float(c->hstats->f2_pp_bits);
     st->npairs = (int64_t)c->hstats->npairs;
     st->itest1 = (int64_t)c->hstats->itest1;
-    st->pp_dense_bricks = c->pp_nlist_host[0];
+    st->pp_dense_bricks = c->hstats->pp_nlist[0];
   }
   return CUBE_OK;
 }

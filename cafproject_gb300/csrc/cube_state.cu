@@ -67,30 +67,65 @@ __global__ void k_scan_sums(long long* __restrict__ bsum, int64_t nb) {
   }
 }
 
-__global__ void k_scan_final(const int32_t* __restrict__ cnt, int64_t n, const long long* __restrict__ bsum,
-                             int64_t* __restrict__ starts) {
-  __shared__ long long s[33];
-  __shared__ int32_t tile[SCAN_CHUNK];
-  int64_t base = (int64_t)blockIdx.x * SCAN_CHUNK;
-  for (int i = threadIdx.x; i < SCAN_CHUNK; i += SCAN_T) {
-    int64_t k = base + i;
-    tile[i] = k < n ? cnt[k] : 0;
+// The chunk at base of the counts, scanned into starts from off on: counts and
+// results pass through shared memory so that the global accesses are
+// consecutive; a word of padding per thread's stretch keeps the stretches of
+// neighbouring threads in different banks (256^3 counts: 89 -> 35 us).  (Within a chunk offsets are 32-bit:
+// an image holds fewer than 2^31 particles.)
+__device__ __forceinline__ int scan_at(int i) { return i + i / SCAN_I; }
+__device__ __forceinline__ void scan_chunk(const int32_t* __restrict__ cnt, int64_t n, int64_t base,
+                                           int64_t* __restrict__ starts, int32_t* tile, long long* s, long long off) {
+  for (int i = threadIdx.x; i < SCAN_CHUNK; i += SCAN_T) tile[scan_at(i)] = base + i < n ? cnt[base + i] : 0;
+  __syncthreads();
+  int32_t* mine = tile + scan_at(threadIdx.x * SCAN_I);
+  int v = 0;
+#pragma unroll
+  for (int i = 0; i < SCAN_I; i++) v += mine[i];
+  long long tot;
+  int run = (int)block_excl_scan(v, s, tot);
+#pragma unroll
+  for (int i = 0; i < SCAN_I; i++) {
+    const int x = mine[i];
+    mine[i] = run;
+    run += x;
   }
   __syncthreads();
-  long long v = 0;
-  for (int i = 0; i < SCAN_I; i++) v += tile[threadIdx.x * SCAN_I + i];
-  long long tot;
-  long long run = block_excl_scan(v, s, tot) + bsum[blockIdx.x];
-  for (int i = 0; i < SCAN_I; i++) {
-    int64_t k = base + (int64_t)threadIdx.x * SCAN_I + i;
-    if (k < n) starts[k] = run;
-    run += tile[threadIdx.x * SCAN_I + i];
-    if (k == n - 1) starts[n] = run;
-  }
+  for (int i = threadIdx.x; i < SCAN_CHUNK && base + i < n; i += SCAN_T) starts[base + i] = off + tile[scan_at(i)];
+  if (threadIdx.x == 0 && base + SCAN_CHUNK >= n) starts[n] = off + tot;
+}
+constexpr int SCAN_TILE = SCAN_CHUNK + SCAN_T;
+
+__global__ void __launch_bounds__(SCAN_T) k_scan_final(const int32_t* __restrict__ cnt, int64_t n,
+                                                       const long long* __restrict__ bsum,
+                                                       int64_t* __restrict__ starts) {
+  __shared__ long long s[33];
+  __shared__ int32_t tile[SCAN_TILE];
+  scan_chunk(cnt, n, (int64_t)blockIdx.x * SCAN_CHUNK, starts, tile, s, bsum[blockIdx.x]);
+}
+
+// Up to SCAN_SMALL counts in one launch: each block adds up everything before
+// its chunk itself (at most half a megabyte in all, from L2), so no block waits
+// for another: 12 us and two gaps in three launches for 32^3 cells, 6.7 us so.
+constexpr int64_t SCAN_SMALL = 1 << 17;
+__global__ void __launch_bounds__(SCAN_T) k_scan_small(const int32_t* __restrict__ cnt, int64_t n,
+                                                       int64_t* __restrict__ starts) {
+  __shared__ long long s[33];
+  __shared__ int32_t tile[SCAN_TILE];
+  const int64_t base = (int64_t)blockIdx.x * SCAN_CHUNK;
+  long long before = 0, off;
+#pragma unroll 8
+  for (int64_t k = threadIdx.x; k < base; k += SCAN_T) before += cnt[k];
+  block_excl_scan(before, s, off);  // its total: everything before the chunk
+  scan_chunk(cnt, n, base, starts, tile, s, off);
 }
 
 int cube_scan_counts(cube_ctx* c, const int32_t* counts, int64_t* starts, int64_t n) {
   int64_t nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
+  if (n > 0 && n <= SCAN_SMALL) {
+    k_scan_small<<<(unsigned)nb, SCAN_T, 0, c->stream>>>(counts, n, starts);
+    CUBE_CUDA(c, cudaGetLastError());
+    return CUBE_OK;
+  }
   if ((size_t)nb * 8 > c->scan_tmp_bytes) return cube_fail(c, CUBE_ERR_ARG, "scan scratch too small");
   long long* bsum = (long long*)c->scan_tmp;
   k_scan_blocksum<<<(unsigned)nb, SCAN_T, 0, c->stream>>>(counts, n, bsum);

@@ -58,6 +58,7 @@ struct UpdArgs {
   const StepDev* sd;  // graph mode: dt_mid and nlayer from the device
   int32_t* vdense;    // destination cells over VF_DENSE particles, for k_vfield_dense
   int64_t p_lo;       // k_dest: first particle of this launch (particles [p_lo, np))
+  int rank_init;      // k_dest: set every rank to the "no rank" sentinel (for the walker)
 };
 
 __device__ __forceinline__ float dtm(const UpdArgs& a) { return a.sd ? __ldg(&a.sd->h.dt_mid) : a.dt_mid; }
@@ -108,6 +109,7 @@ __global__ void k_dest(UpdArgs a) {
   int local_max = 0;
   for (int64_t p = a.p_lo + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.np; p += stride) {
     int64_t cell = a.pcell[p];
+    if (a.rank_init) a.rank[p] = 0xffffffffu;
     int gc[3];
     cell_coords(g, cell, gc[0], gc[1], gc[2]);
     // per dim: up to two frames (offset o of the local coordinate) that land;
@@ -851,14 +853,61 @@ __device__ __forceinline__ void ff_add(float& hi, float& lo, float x, float xlo)
 }
 
 // sigma_v sums of the new state (update_particle.f90:172-196): per-block FP64
-// partials in a fixed partition, summed in a fixed order by k_sigma_final.
-// Each block ends in FP64 shuffles on the narrow FP64 pipe, so small states
-// take fewer blocks (sigma_blocks): 2048 blocks for every size took 27 us for
-// 64^3 particles, 10 us with a block per 1024.
-__global__ void k_sigma(const void* __restrict__ vp, const int32_t* __restrict__ pcell, const float* __restrict__ vfield,
-                        int64_t np, int64_t ncells, const float2* __restrict__ dech, int nvbin, int izipv,
-                        double* __restrict__ part) {
-  __shared__ double s[3][32];
+// partials in a fixed partition, which the last block to finish adds in a fixed
+// order: thread t the partials t, t + 256, ..., then the warps' lanes, then the
+// warps.  (One thread adding all 3 x 2048 from global memory took 364 us, most
+// of a small box's step in a captured graph; a kernel of its own for the sums
+// 3.7 us and a launch.)  Each block ends in FP64 shuffles on the narrow FP64
+// pipe, so small states take fewer blocks (sigma_blocks): 2048 blocks for every
+// size took 27 us for 64^3 particles, 10 us with a block per 1024.
+struct SigmaArgs {
+  const void* vp;
+  const int32_t* pcell;
+  const float* vfield;
+  int64_t np, ncells;
+  const float2* dech;
+  int nvbin, izipv;
+  double* part;      // 3 per block
+  unsigned* count;   // blocks done; the last one leaves it at zero
+  DevStats* st;      // eager: receives the sums
+  // graph mode: also sigma_vi_new, with the host path's arithmetic (correctly
+  // rounded sqrt and division), and its vcoef for the encode estimate
+  double npg;
+  StepDev* sd;
+  StepOut* so;
+};
+constexpr int SG_THREADS = 256;
+__device__ void sigma_total(const SigmaArgs& a, double (*w)[SG_THREADS / 32]) {
+  double s[3] = {0.0, 0.0, 0.0};
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += SG_THREADS)
+    for (int t = 0; t < 3; t++) s[t] += *(volatile double*)(a.part + 3 * b + t);
+  for (int t = 0; t < 3; t++) {
+    for (int o = 16; o > 0; o >>= 1) s[t] += __shfl_xor_sync(0xffffffffu, s[t], o);
+    if ((threadIdx.x & 31) == 0) w[t][threadIdx.x >> 5] = s[t];
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int t = 0; t < 3; t++) {
+    s[t] = 0.0;
+    for (int i = 0; i < SG_THREADS / 32; i++) s[t] += w[t][i];
+    if (a.st) a.st->sums[t] = s[t];
+  }
+  if (!a.sd) return;
+  const double std_res = sqrt(s[1] / a.npg);
+  const float sn = (float)(std_res / (double)sqrtf(3.0f));  // update_particle.f90:224
+  a.sd->sigma_new = sn;
+  a.sd->cf_new = sn > 0.f ? (float)vcoef(sn) : 0.f;
+  if (a.so) {
+    for (int t = 0; t < 3; t++) a.so->sums[t] = s[t];
+    a.so->sigma_new = sn;
+  }
+}
+
+__global__ void __launch_bounds__(SG_THREADS) k_sigma(SigmaArgs a) {
+  __shared__ double s[3][SG_THREADS / 32];
+  __shared__ bool last;
+  const int64_t np = a.np, ncells = a.ncells;
+  const float* __restrict__ vfield = a.vfield;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   // per-thread float-float accumulators (exact products by FMA), one FP64
@@ -870,10 +919,10 @@ __global__ void k_sigma(const void* __restrict__ vp, const int32_t* __restrict__
     ff_add(ch, cl, q, 0.f);
   }
   for (int64_t p = t0; p < np; p += stride) {
-    int64_t c = pcell[p];
+    int64_t c = a.pcell[p];
     if (c < 0 || c >= ncells) continue;
     for (int d = 0; d < 3; d++) {
-      float2 v = __ldg(dech + load_code(vp, 3 * p + d, izipv) + nvbin / 2);
+      float2 v = __ldg(a.dech + load_code(a.vp, 3 * p + d, a.izipv) + a.nvbin / 2);
       float p2 = __fmul_rn(v.x, v.x);
       ff_add(rh, rl, p2, __fmaf_rn(v.x, v.x, -p2) + 2.f * v.x * v.y);
       float w, ew;
@@ -898,45 +947,15 @@ __global__ void k_sigma(const void* __restrict__ vp, const int32_t* __restrict__
   __syncthreads();
   if (threadIdx.x == 0) {
     double t[3] = {0, 0, 0};
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++)
+    for (int i = 0; i < SG_THREADS / 32; i++)
       for (int k = 0; k < 3; k++) t[k] += s[k][i];
-    for (int k = 0; k < 3; k++) part[3 * blockIdx.x + k] = t[k];
-  }
-}
-
-// The sums over the block partials: thread t adds partials t, t + 256, ...,
-// the warps' lanes and then the warps' sums are added in order.  One thread
-// adding all 3 x 2048 from global memory took 364 us, most of a small box's
-// step in a captured graph; 3.7 us this way.  In graph mode (sd set) also
-// sigma_vi_new with the host path's arithmetic (correctly rounded sqrt and
-// division) and its vcoef for the encode estimate.
-constexpr int SF_THREADS = 256;
-__global__ void __launch_bounds__(SF_THREADS) k_sigma_final(const double* __restrict__ part, int nb, DevStats* st,
-                                                            double npg, StepDev* sd, StepOut* so) {
-  __shared__ double w[3][SF_THREADS / 32];
-  double s[3] = {0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nb; b += SF_THREADS)
-    for (int t = 0; t < 3; t++) s[t] += part[3 * b + t];
-  for (int t = 0; t < 3; t++) {
-    for (int o = 16; o > 0; o >>= 1) s[t] += __shfl_xor_sync(0xffffffffu, s[t], o);
-    if ((threadIdx.x & 31) == 0) w[t][threadIdx.x >> 5] = s[t];
+    for (int k = 0; k < 3; k++) a.part[3 * blockIdx.x + k] = t[k];
+    __threadfence();
+    last = atomicInc(a.count, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
+    __threadfence();
   }
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  for (int t = 0; t < 3; t++) {
-    s[t] = 0.0;
-    for (int i = 0; i < SF_THREADS / 32; i++) s[t] += w[t][i];
-    if (st) st->sums[t] = s[t];
-  }
-  if (!sd) return;
-  const double std_res = sqrt(s[1] / npg);
-  const float sn = (float)(std_res / (double)sqrtf(3.0f));  // update_particle.f90:224
-  sd->sigma_new = sn;
-  sd->cf_new = sn > 0.f ? (float)vcoef(sn) : 0.f;
-  if (so) {
-    for (int t = 0; t < 3; t++) so->sums[t] = s[t];
-    so->sigma_new = sn;
-  }
+  if (last) sigma_total(a, s);
 }
 
 int sigma_blocks(const cube_ctx* c, int64_t np) {
@@ -994,7 +1013,7 @@ static int update_x_graph(cube_ctx* c) {
   a.vdense = c->vdense;
   const int B = 256;
   cudaStream_t s = c->stream;
-  CUBE_CUDA(c, cudaMemsetAsync(c->rank, 0xFF, 4 * (size_t)c->np, s));
+  a.rank_init = 1;
   k_dest<<<cube_grid(c->np, B), B, 0, s>>>(a);
   CUBE_CUDA(c, cudaMemsetAsync(c->offc, 0, sizeof(uint16_t) * NOFF * (size_t)c->ncells, s));
   k_rank_local<<<cube_grid(c->np, 256), 256, 0, s>>>(a);
@@ -1014,11 +1033,10 @@ static int update_x_graph(cube_ctx* c) {
   // fine kick is the first to need them (it waits for ev_codec)
   CUBE_CUDA(c, cudaEventRecord(c->ev_aux, s));
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_aux, c->ev_aux, 0));
-  const int nb = sigma_blocks(c, c->np);
-  k_sigma<<<nb, 256, 0, c->stream_aux>>>(c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, cv.dech, c->nvbin,
-                                         c->p.izipv, c->red_tmp);
   const double npg = (double)(c->npglobal > 0 ? c->npglobal : c->np);
-  k_sigma_final<<<1, SF_THREADS, 0, c->stream_aux>>>(c->red_tmp, nb, nullptr, npg, c->sd, c->sout);
+  const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, cv.dech, c->nvbin, c->p.izipv,
+                     c->red_tmp, c->red_count, nullptr, npg, c->sd, c->sout};
+  k_sigma<<<sigma_blocks(c, c->np), SG_THREADS, 0, c->stream_aux>>>(sg);
   CUBE_CUDA(c, cudaGetLastError());
   c->stream = c->stream_aux;
   r = cube_codec_build_dev(c, 1 - c->graph_slot, &c->sd->sigma_new);
@@ -1077,7 +1095,6 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   a.pcell_new = c->pcell[kn];
   a.vdense = c->vdense;
   const int B = 256;
-  CUBE_CUDA(c, cudaMemsetAsync(c->rank, 0xFF, 4 * (size_t)c->np, c->stream));  // "no rank" sentinel
   cube_phase_begin(c, PH_UPD_DEST);
   if (c->xv_pending && c->up_np == c->np) {
     // a pending cube_upload_begin: take xp and vp piece by piece as they land
@@ -1102,6 +1119,7 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   int64_t np_new = 0;
   auto walk = [&]() -> int {
     cube_phase_begin(c, PH_UPD_RANK);
+    CUBE_CUDA(c, cudaMemsetAsync(c->rank, 0xFF, 4 * (size_t)c->np, c->stream));  // "no rank" sentinel
     k_rank<<<cube_grid(c->ncells, 128, 32), 128, 0, c->stream>>>(a);
     cube_phase_end(c, PH_UPD_RANK);
     CUBE_CUDA(c, cudaGetLastError());
@@ -1189,11 +1207,10 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   cube_phase_end(c, PH_UPD_SCATTER);
   CUBE_CUDA(c, cudaGetLastError());
   // sigma statistics of the new state (decoded with sigma_vi)
-  const int nb = sigma_blocks(c, np_new);
   cube_phase_begin(c, PH_UPD_SIGMA);
-  k_sigma<<<nb, 256, 0, c->stream>>>(c->vp[kn], c->pcell[kn], c->vfield[kn], np_new, c->ncells, cv.dech,
-                                      c->nvbin, c->p.izipv, c->red_tmp);
-  k_sigma_final<<<1, SF_THREADS, 0, c->stream>>>(c->red_tmp, nb, c->dstats, 0.0, nullptr, nullptr);
+  const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], np_new, c->ncells, cv.dech, c->nvbin, c->p.izipv,
+                     c->red_tmp, c->red_count, c->dstats, 0.0, nullptr, nullptr};
+  k_sigma<<<sigma_blocks(c, np_new), SG_THREADS, 0, c->stream>>>(sg);
   cube_phase_end(c, PH_UPD_SIGMA);
   CUBE_CUDA(c, cudaGetLastError());
   r = cube_stats_fetch(c);
