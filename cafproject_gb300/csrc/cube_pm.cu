@@ -94,6 +94,7 @@ struct DepArgs {
   float* rho;                 // padded periodic mesh, row stride n+2
   unsigned long long* total;  // sum of all owned cells in fixed point (exact)
   int ng;                     // power-spectrum mesh (kPk only)
+  float rnc;                  // kPk: RN(1/nc)
   float qscale, qinv;         // fixed-point scale 2^s and 2^-s (dep_shift)
   int accumulate;             // add to the mesh (a second species) instead of writing it
 };
@@ -172,7 +173,10 @@ __global__ void __launch_bounds__(256) k_deposit_det(DepArgs a) {
         float frac = __fmul_rn(pos_off_f(code, g.izipx), g.izipx == 1 ? 1.0f / 256.0f : 1.0f / 65536.0f);
         // the particle's own global frame, as the reference rounds it
         float pos = __fadd_rn((float)v, frac);
-        tx = __fsub_rn(__fdiv_rn(__fmul_rn(pos, (float)a.ng), (float)nc), 0.5f);
+        // the quotient by nc, correctly rounded: Markstein's correction step as
+        // in div_const (nc is a whole number, its reciprocal rounded to nearest)
+        const float num = __fmul_rn(pos, (float)a.ng), q = __fmul_rn(num, a.rnc);
+        tx = __fsub_rn(__fmaf_rn(__fmaf_rn(-q, (float)nc, num), a.rnc, q), 0.5f);
       } else {
         tx = MPC == 1 ? coarse_tempx(v, code, g.izipx) : fine_tempx(MPC, v, code, g.izipx);
       }
@@ -798,7 +802,7 @@ int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate) {
   Geo g = make_geo(c);
   CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), s));
   const int sh = dep_shift(c->p.mass_p);
-  DepArgs a{g, c->xp[c->cur], c->rhoc[c->cur], c->cstart[c->cur], c->p.mass_p, c->rho_f, &c->dstats->rhof_fix, 0,
+  DepArgs a{g, c->xp[c->cur], c->rhoc[c->cur], c->cstart[c->cur], c->p.mass_p, c->rho_f, &c->dstats->rhof_fix, 0, 0.f,
             std::ldexp(1.0f, sh), std::ldexp(1.0f, -sh), accumulate ? 1 : 0};
   cube_phase_begin(c, PH_F_DEPOSIT);
   int r = launch_fine_deposit(c, a);
@@ -905,7 +909,7 @@ int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool pre, bool with_
 int cube_pk_deposit(cube_ctx* c, int ng, float* rho, unsigned long long* total) {
   const int sh = dep_shift(1.0f);
   DepArgs a{make_geo(c), c->xp[c->cur], c->rhoc[c->cur], c->cstart[c->cur], 1.0f, rho, total, ng,
-            std::ldexp(1.0f, sh), std::ldexp(1.0f, -sh), 0};
+            1.0f / (float)c->p.nc, std::ldexp(1.0f, sh), std::ldexp(1.0f, -sh), 0};
   int nc = c->p.nc;
   if (ng == nc) return launch_deposit<1, 8, 8, 8, 1, 1, true>(c, a);
   if (ng == 2 * nc) return launch_deposit<2, 8, 8, 4, 1, 1, true>(c, a);
@@ -921,7 +925,7 @@ int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate, bool 
     CUBE_CUDA(c, cudaMemsetAsync(&c->dstats->rhoc_fix, 0, 8, c->stream));
   }
   const int sh = dep_shift(c->p.mass_p);
-  DepArgs a{g, c->xp[c->cur], c->rhoc[c->cur], c->cstart[c->cur], c->p.mass_p, c->rho_c, &c->dstats->rhoc_fix, 0,
+  DepArgs a{g, c->xp[c->cur], c->rhoc[c->cur], c->cstart[c->cur], c->p.mass_p, c->rho_c, &c->dstats->rhoc_fix, 0, 0.f,
             std::ldexp(1.0f, sh), std::ldexp(1.0f, -sh), accumulate ? 1 : 0};
   cube_phase_begin(c, PH_C_DEPOSIT);
   int r = launch_coarse_deposit(c, a);
