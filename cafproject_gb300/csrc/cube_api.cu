@@ -450,12 +450,15 @@ extern "C" int cube_pm_coarse_kick(cube_ctx* c, float a_mid, float dt, cube_stat
 extern "C" int cube_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_stats* st) {
   int r = check_ready(c);
   if (r) return r;
+  // every stage is queued; the stats come back once, with the coarse kick's
   const float pre[2] = {a_mid, dt};
-  if ((r = cube_fine_forces_impl(c, st, pre))) return r;
+  if ((r = cube_fine_forces_impl(c, nullptr, pre))) return r;
   if ((r = cube_fine_kick_impl(c, a_mid, dt, true))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
-  if ((r = cube_coarse_forces_impl(c, st, pre, true))) return r;
-  return cube_coarse_kick_impl(c, a_mid, dt, st, true, true);
+  if ((r = cube_coarse_forces_impl(c, nullptr, pre, true))) return r;
+  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true, true))) return r;
+  if (st) cube_fine_stats(c, st);
+  return CUBE_OK;
 }
 
 // ext_pp_force followed by particle_mesh (main.f90:113-116) with PP on a
@@ -477,30 +480,29 @@ extern "C" int cube_pp_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_st
     c->dstats = c->dstats_pp;
     c->hstats = c->hstats_pp;
     r = cube_pp_launch(c, a_mid, dt, /*defer_kick=*/true);
+    // its stats travel behind it: the host waits once, for the coarse kick's
+    if (!r && cudaMemcpyAsync(c->hstats_pp, c->dstats_pp, sizeof(DevStats), cudaMemcpyDeviceToHost, c->stream_pp) !=
+                  cudaSuccess)
+      r = CUBE_ERR_CUDA;
     if (!r) r = cudaEventRecord(c->ev_pp, c->stream_pp) == cudaSuccess ? CUBE_OK : CUBE_ERR_CUDA;
     c->stream = s0;
     c->dstats = d0;
     c->hstats = h0;
     if (r) return r;
   }
-  if ((r = cube_fine_forces_impl(c, st_pm, pre))) return r;
-  if ((r = cube_coarse_forces_impl(c, st_pm, pre, true))) return r;
+  if ((r = cube_fine_forces_impl(c, nullptr, pre))) return r;
+  if ((r = cube_coarse_forces_impl(c, nullptr, pre, true))) return r;
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_pp, 0));
   // the fine kick applies PP's kick first (ext_pp_force.f90:116-121), then its own
   if ((r = cube_fine_kick_impl(c, a_mid, dt, true, /*with_pp=*/true))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
   if ((r = cube_coarse_kick_impl(c, a_mid, dt, st_pm, true, true))) return r;
-  {  // PP's stats (its stream is done: the kicks waited for it)
-    cudaStream_t s0 = c->stream;
-    DevStats *d0 = c->dstats, *h0 = c->hstats;
-    c->stream = c->stream_pp;
-    c->dstats = c->dstats_pp;
-    c->hstats = c->hstats_pp;
-    r = cube_pp_finish(c, st_pp);
-    c->stream = s0;
-    c->dstats = d0;
-    c->hstats = h0;
-  }
+  if (st_pm) cube_fine_stats(c, st_pm);
+  // PP's stats are in their host copy: the kicks waited for its stream
+  DevStats* h0 = c->hstats;
+  c->hstats = c->hstats_pp;
+  r = cube_pp_finish(c, st_pp, true);
+  c->hstats = h0;
   return r;
 }
 
@@ -517,15 +519,16 @@ extern "C" int cube_particle_mesh2(cube_ctx* c, cube_ctx* nu, float a_mid, float
   const float pre[2] = {a_mid, dt};
   if ((r = cube_fine_density_impl(c, nullptr, false))) return r;
   if ((r = cube_fine_density_impl(nu, nullptr, true))) return cube_fail(c, r, nu->err);
-  if ((r = cube_fine_spectral_impl(c, st, pre))) return r;
+  if ((r = cube_fine_spectral_impl(c, nullptr, pre))) return r;
   if ((r = cube_fine_kick_impl(c, a_mid, dt, true))) return r;
   if ((r = cube_fine_kick_impl(nu, a_mid, dt, true))) return cube_fail(c, r, nu->err);
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193-194
   nu->sigma_vi = nu->sigma_vi_new;
   if ((r = cube_coarse_density_impl(c, nullptr, false, true))) return r;
   if ((r = cube_coarse_density_impl(nu, nullptr, true, true))) return cube_fail(c, r, nu->err);
-  if ((r = cube_coarse_spectral_impl(c, st, pre))) return r;
+  if ((r = cube_coarse_spectral_impl(c, nullptr, pre))) return r;
   if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true, true))) return r;
+  if (st) cube_fine_stats(c, st);
   if ((r = cube_coarse_kick_impl(nu, a_mid, dt, st_nu, true, true))) return cube_fail(c, r, nu->err);
   // testrhof / testrhoc sum both species' mass (pm.f90:108, 258); the coarse
   // kick left the second species' deposited masses in its host stats

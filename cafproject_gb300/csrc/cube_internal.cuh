@@ -46,6 +46,7 @@ struct DevStats {
   unsigned int vmax_lo_bits[3];           // coarse kick: max of certified lower bounds of |v + vfield|
   unsigned long long pp_active;           // PP prefilter: particles with a neighbour besides themselves
   double sums[3];                         // update_x: the sigma_v sums (update_particle.f90:172-196)
+  long long np_new;                       // update_x: particles of the new state
   int pp_nlist[11];  // PP: lengths of the levels' lists (5), then each level's next-item counter (6)
 };
 
@@ -714,7 +715,7 @@ int cube_pp_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st);
 // defer_kick: leave the kick to the fine kick (cube_fine_kick_impl with_pp)
 int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick = false);
 int cube_pp_init(cube_ctx* c);  // once per context: the staging kernels' shared-memory sizes
-int cube_pp_finish(cube_ctx* c, cube_stats* st);
+int cube_pp_finish(cube_ctx* c, cube_stats* st, bool fetched = false);  // fetched: hstats holds the stats already
 // density deposits; accumulate: add to the mesh (the linked species) instead of writing it
 int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false);
 // fresh (the coarse stages): the stats were zeroed by this step's fine density
@@ -749,6 +750,8 @@ int cube_copy_join(cube_ctx* c);
 int cube_sort_pairs(cube_ctx* c, int64_t n, int begin_bit, int end_bit, uint64_t** keys, int32_t** vals);
 // orders the context stream after a deferred pid upload
 int cube_pid_join(cube_ctx* c);
+// stats of the last force pass from hstats: the fine level's
+void cube_fine_stats(const cube_ctx* c, cube_stats* st);
 // ... after every piece of a pending cube_upload_begin (xp, vp and pid)
 int cube_upload_join(cube_ctx* c);
 int cube_copy_stream(cube_ctx* c);

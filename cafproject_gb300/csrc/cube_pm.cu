@@ -816,6 +816,11 @@ int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate) {
   return CUBE_OK;
 }
 
+void cube_fine_stats(const cube_ctx* c, cube_stats* st) {
+  st->f2_max_fine = bits_float(c->hstats->f2_fine_bits);
+  st->testrhof = std::ldexp((double)c->hstats->rhof_fix, -dep_shift(c->p.mass_p));
+}
+
 int cube_fine_forces_impl(cube_ctx* c, cube_stats* st, const float* pre) {
   int r0 = cube_fine_density_impl(c, nullptr, false);
   if (r0) return r0;
@@ -848,8 +853,7 @@ int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
   if (st) {
     int r = cube_stats_fetch(c);
     if (r) return r;
-    st->f2_max_fine = bits_float(c->hstats->f2_fine_bits);
-    st->testrhof = std::ldexp((double)c->hstats->rhof_fix, -dep_shift(c->p.mass_p));
+    cube_fine_stats(c, st);
   }
   return CUBE_OK;
 }

@@ -1063,9 +1063,11 @@ int cube_pp_init(cube_ctx* c) {
 
 // the stats of the launches above, once they are done (itest1 check of
 // ext_pp_force.f90:141)
-int cube_pp_finish(cube_ctx* c, cube_stats* st) {
-  int r = cube_stats_fetch(c);
-  if (r) return r;
+int cube_pp_finish(cube_ctx* c, cube_stats* st, bool fetched) {
+  if (!fetched) {
+    int r = cube_stats_fetch(c);
+    if (r) return r;
+  }
   if (c->hstats->pp_overflow)
     return cube_fail(c, CUBE_ERR_PP_OVERFLOW, "PP: " + std::to_string(c->hstats->pp_overflow) +
                                                    " cell(s) with their fine-cell ring hold more particles than the " +

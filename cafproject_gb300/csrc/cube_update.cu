@@ -58,6 +58,7 @@ struct UpdArgs {
   const StepDev* sd;  // graph mode: dt_mid and nlayer from the device
   int32_t* vdense;    // destination cells over VF_DENSE particles, for k_vfield_dense
   int64_t p_lo;       // k_dest: first particle of this launch (particles [p_lo, np))
+  int spec;           // counting path queued ahead of the check that it applies
   int rank_init;      // k_dest: set every rank to the "no rank" sentinel (for the walker)
 };
 
@@ -67,6 +68,9 @@ __device__ __forceinline__ int nlay(const UpdArgs& a) { return a.sd ? __ldg(&a.s
 // the walker unless the counting path flagged itself inapplicable, the
 // counting path's placement when it did
 __device__ __forceinline__ bool counting_failed(const UpdArgs& a) { return (*(volatile int*)&a.st->flags & 12) != 0; }
+// kernels of the counting path queued before the host knows that it applies
+// (a captured step; an eager one, up to the sums) do nothing when it does not
+__device__ __forceinline__ bool queued_in_vain(const UpdArgs& a) { return a.spec && counting_failed(a); }
 
 
 // global coarse coordinate of tile-local cell l (1-based) of tile coordinate t
@@ -423,7 +427,7 @@ __global__ void k_rank_base(UpdArgs a) {
 }
 
 __global__ void k_rank_place(UpdArgs a) {
-  if (a.sd && counting_failed(a)) return;
+  if (queued_in_vain(a)) return;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.np; p += (int64_t)gridDim.x * blockDim.x) {
     int32_t D = a.dest[p];
     if (D < 0) continue;
@@ -441,7 +445,7 @@ __global__ void k_rank_place(UpdArgs a) {
 constexpr uint32_t VF_DENSE = 256;
 constexpr uint32_t VF_BATCH = 4;
 __global__ void k_vfield_new(UpdArgs a) {
-  if (a.sd && counting_failed(a)) return;
+  if (queued_in_vain(a)) return;
   for (int64_t D = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; D < a.ncells;
        D += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t cnt = (uint32_t)a.cnt_new[D];
@@ -490,7 +494,7 @@ __global__ void k_vfield_new(UpdArgs a) {
 // sequential real(4) sum over them in rank order, the same arithmetic as
 // k_vfield_new's thread
 __global__ void __launch_bounds__(128) k_vfield_dense(UpdArgs a) {
-  if (a.sd && counting_failed(a)) return;
+  if (queued_in_vain(a)) return;
   __shared__ float2 sdd[4][32][3];
   __shared__ float svf[4][32][3];
   __shared__ int scode[4][32][3];
@@ -808,6 +812,7 @@ __global__ void __launch_bounds__(256) k_sort_gather(UpdArgs a, const uint64_t* 
 
 // U3: scatter every primary copy to its place in the new disjoint order.
 __global__ void __launch_bounds__(256) k_scatter(UpdArgs a) {
+  if (!a.sd && queued_in_vain(a)) return;  // (a captured step's walker has set the ranks instead)
   __shared__ unsigned long long s_q[8][SC_Q];
   RecodeQueue rq{s_q[threadIdx.x >> 5], 0};
   const int lane = threadIdx.x & 31;
@@ -865,6 +870,7 @@ struct SigmaArgs {
   const int32_t* pcell;
   const float* vfield;
   int64_t np, ncells;
+  const int64_t* npp;  // when set, the particle count on the device (at most np)
   const float2* dech;
   int nvbin, izipv;
   double* part;      // 3 per block
@@ -892,6 +898,7 @@ __device__ void sigma_total(const SigmaArgs& a, double (*w)[SG_THREADS / 32]) {
     for (int i = 0; i < SG_THREADS / 32; i++) s[t] += w[t][i];
     if (a.st) a.st->sums[t] = s[t];
   }
+  if (a.st && a.npp) a.st->np_new = *a.npp;
   if (!a.sd) return;
   const double std_res = sqrt(s[1] / a.npg);
   const float sn = (float)(std_res / (double)sqrtf(3.0f));  // update_particle.f90:224
@@ -906,7 +913,7 @@ __device__ void sigma_total(const SigmaArgs& a, double (*w)[SG_THREADS / 32]) {
 __global__ void __launch_bounds__(SG_THREADS) k_sigma(SigmaArgs a) {
   __shared__ double s[3][SG_THREADS / 32];
   __shared__ bool last;
-  const int64_t np = a.np, ncells = a.ncells;
+  const int64_t np = a.npp ? min(a.np, *a.npp) : a.np, ncells = a.ncells;
   const float* __restrict__ vfield = a.vfield;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1014,6 +1021,7 @@ static int update_x_graph(cube_ctx* c) {
   const int B = 256;
   cudaStream_t s = c->stream;
   a.rank_init = 1;
+  a.spec = 1;
   k_dest<<<cube_grid(c->np, B), B, 0, s>>>(a);
   CUBE_CUDA(c, cudaMemsetAsync(c->offc, 0, sizeof(uint16_t) * NOFF * (size_t)c->ncells, s));
   k_rank_local<<<cube_grid(c->np, 256), 256, 0, s>>>(a);
@@ -1034,8 +1042,8 @@ static int update_x_graph(cube_ctx* c) {
   CUBE_CUDA(c, cudaEventRecord(c->ev_aux, s));
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_aux, c->ev_aux, 0));
   const double npg = (double)(c->npglobal > 0 ? c->npglobal : c->np);
-  const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, cv.dech, c->nvbin, c->p.izipv,
-                     c->red_tmp, c->red_count, nullptr, npg, c->sd, c->sout};
+  const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, nullptr, cv.dech, c->nvbin,
+                     c->p.izipv, c->red_tmp, c->red_count, nullptr, npg, c->sd, c->sout};
   k_sigma<<<sigma_blocks(c, c->np), SG_THREADS, 0, c->stream_aux>>>(sg);
   CUBE_CUDA(c, cudaGetLastError());
   c->stream = c->stream_aux;
@@ -1125,15 +1133,39 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
     CUBE_CUDA(c, cudaGetLastError());
     return CUBE_OK;
   };
-  auto scan = [&]() -> int {
+  auto scan_only = [&]() -> int {
     cube_phase_begin(c, PH_UPD_SCAN);
     int rr = cube_scan_counts(c, c->rhoc[kn], c->cstart[kn], c->ncells);
     cube_phase_end(c, PH_UPD_SCAN);
+    return rr;
+  };
+  auto scan = [&]() -> int {
+    int rr = scan_only();
     if (rr) return rr;
     CUBE_CUDA(c, cudaMemcpyAsync(&np_new, c->cstart[kn] + c->ncells, 8, cudaMemcpyDeviceToHost, c->stream));
     return cube_stats_fetch(c);
   };
+  auto means = [&]() -> int {
+    k_vfield_new<<<cube_grid(c->ncells, 128, 32), 128, 0, c->stream>>>(a);
+    k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 16), 128, 0, c->stream>>>(a);
+    CUBE_CUDA(c, cudaGetLastError());
+    return CUBE_OK;
+  };
+  // sigma statistics of the new state (decoded with sigma_vi), then the stats
+  auto sigma = [&](int64_t np_most) -> int {
+    cube_phase_begin(c, PH_UPD_SIGMA);
+    const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], np_most, c->ncells, c->cstart[kn] + c->ncells, cv.dech,
+                       c->nvbin, c->p.izipv, c->red_tmp, c->red_count, c->dstats, 0.0, nullptr, nullptr};
+    k_sigma<<<sigma_blocks(c, np_most), SG_THREADS, 0, c->stream>>>(sg);
+    cube_phase_end(c, PH_UPD_SIGMA);
+    CUBE_CUDA(c, cudaGetLastError());
+    return cube_stats_fetch(c);
+  };
   if (path == COUNT) {
+    // the whole path is queued before the host looks: its kernels check on the
+    // device that it applies, and do nothing else when it does not (then no
+    // particle is lost to a second frame and the new count is at most the old)
+    a.spec = 1;
     cube_phase_begin(c, PH_UPD_RANK);
     CUBE_CUDA(c, cudaMemsetAsync(c->offc, 0, sizeof(uint16_t) * NOFF * (size_t)c->ncells, c->stream));
     k_rank_local<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(a);
@@ -1141,8 +1173,20 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
     k_rank_base<<<cube_grid(c->ncells, 256), 256, 0, c->stream>>>(a);
     cube_phase_end(c, PH_UPD_RANK);
     CUBE_CUDA(c, cudaGetLastError());
-    if ((r = scan())) return r;
+    if ((r = scan_only())) return r;
+    cube_phase_begin(c, PH_UPD_PLACE);
+    k_rank_place<<<cube_grid(c->np, B), B, 0, c->stream>>>(a);
+    if ((r = means())) return r;
+    cube_phase_end(c, PH_UPD_PLACE);
+    if ((r = cube_pid_join(c))) return r;  // a deferred pid upload lands before the scatter reads it
+    cube_phase_begin(c, PH_UPD_SCATTER);
+    k_scatter<<<cube_grid(c->np, B), B, 0, c->stream>>>(a);
+    cube_phase_end(c, PH_UPD_SCATTER);
+    CUBE_CUDA(c, cudaGetLastError());
+    if ((r = sigma(c->np))) return r;
+    np_new = c->hstats->np_new;
     if (c->hstats->flags & 12) path = SORT;  // counting path not applicable
+    a.spec = 0;
   } else if (path == WALK) {
     if ((r = walk()) || (r = scan())) return r;
   } else {
@@ -1187,34 +1231,24 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   DevStats hs = *c->hstats;
   if (np_new > c->p.np_max)
     return cube_fail(c, CUBE_ERR_IMAGE_OVERFLOW, "new particle count exceeds np_max");
-  if (path != WALK) {
-    cube_phase_begin(c, PH_UPD_PLACE);
-    if (path == COUNT) k_rank_place<<<cube_grid(c->np, B), B, 0, c->stream>>>(a);
-    k_vfield_new<<<cube_grid(c->ncells, 128, 32), 128, 0, c->stream>>>(a);
-    k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 16), 128, 0, c->stream>>>(a);
-    cube_phase_end(c, PH_UPD_PLACE);
+  if (path != COUNT) {
+    if (path == SORT) {
+      cube_phase_begin(c, PH_UPD_PLACE);
+      if ((r = means())) return r;
+      cube_phase_end(c, PH_UPD_PLACE);
+    }
+    if ((r = cube_pid_join(c))) return r;
+    cube_phase_begin(c, PH_UPD_SCATTER);
+    if (skeys) {
+      k_sort_gather<<<cube_grid(np_new, B), B, 0, c->stream>>>(a, skeys, np_new, 64 - db);
+    } else {
+      k_scatter<<<cube_grid(c->np, B), B, 0, c->stream>>>(a);
+      if (hs.ndup_list) k_scatter_xtra<<<cube_grid((int64_t)hs.ndup_list, B), B, 0, c->stream>>>(a);
+    }
+    cube_phase_end(c, PH_UPD_SCATTER);
     CUBE_CUDA(c, cudaGetLastError());
+    if ((r = sigma(np_new))) return r;
   }
-  r = cube_pid_join(c);  // a deferred pid upload lands before the scatter reads it
-  if (r) return r;
-  cube_phase_begin(c, PH_UPD_SCATTER);
-  if (skeys) {
-    k_sort_gather<<<cube_grid(np_new, B), B, 0, c->stream>>>(a, skeys, np_new, 64 - db);
-  } else {
-    k_scatter<<<cube_grid(c->np, B), B, 0, c->stream>>>(a);
-    if (hs.ndup_list) k_scatter_xtra<<<cube_grid((int64_t)hs.ndup_list, B), B, 0, c->stream>>>(a);
-  }
-  cube_phase_end(c, PH_UPD_SCATTER);
-  CUBE_CUDA(c, cudaGetLastError());
-  // sigma statistics of the new state (decoded with sigma_vi)
-  cube_phase_begin(c, PH_UPD_SIGMA);
-  const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], np_new, c->ncells, cv.dech, c->nvbin, c->p.izipv,
-                     c->red_tmp, c->red_count, c->dstats, 0.0, nullptr, nullptr};
-  k_sigma<<<sigma_blocks(c, np_new), SG_THREADS, 0, c->stream>>>(sg);
-  cube_phase_end(c, PH_UPD_SIGMA);
-  CUBE_CUDA(c, cudaGetLastError());
-  r = cube_stats_fetch(c);
-  if (r) return r;
   if (c->hstats->flags & 2)
     return cube_fail(c, CUBE_ERR_COUNT_MISMATCH, "a re-sorted particle had no rank in its destination cell");
   const double* sums = c->hstats->sums;
