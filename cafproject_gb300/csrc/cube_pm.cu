@@ -11,6 +11,7 @@
 // Coarse level: nc^3 periodic mesh, deposit with the -0.5 shift
 // (pm.f90:221), R2C, i*K_c, C2R, kick (pm.f90:322-387) with vmax.
 // The 1/n^3 normalisation is folded into the stored kernels.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -330,48 +331,70 @@ __global__ void k_green3(const float2* __restrict__ rk, const float* __restrict_
   }
 }
 
-// maxval(sum(force**2,1)) over the mesh (pm.f90:126, 315): float2 loads along x
-// (rows start 8-byte aligned: stride n+2), blockDim.y rows (y, z) at a time, as
-// many as fill a block of 256 threads (a row a block left three quarters of the
-// threads of a 128^3 mesh idle: 12.6 -> 8.1 us)
+// maxval(sum(force**2,1)) over the mesh (pm.f90:126, 315), and for kPre each
+// force value rewritten as its kick factor force*a_mid*dt/6/pi.  Bound by
+// memory (24 bytes a cell for kPre): the three padded meshes are walked as flat
+// arrays of 16 bytes, F2_LOADS of each in flight a thread, and the two values
+// of padding behind each row (n even) are left out of the maximum.  Row by row
+// in 8 bytes it took 4.48 ms at 1024^3 and 12.6 us at 128^3 (three quarters of
+// the threads idle there), 4.10 ms and 7.7 us flat; 3.82 ms at the copy rate.
+// (Repeating a row's first value in its padding, to spare the kicks the wrap in
+// x, took 6.5 ms instead of 4.6 row by row: the padding shares its sector with
+// the next row's start, whose load another block has pending.)
 __device__ __forceinline__ float f2sum(float a, float b, float c) {
   return __fadd_rn(__fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b)), __fmul_rn(c, c));
 }
-// kPre: then rewrite each force value as its kick factor force*a_mid*dt/6/pi
-// (repeating a row's first value in its padding, to spare the kicks the wrap in
-// x, took 6.5 ms instead of 4.6 at 1024^3: the padding shares its sector with
-// the next row's start, whose load another block has pending)
+constexpr int F2_LOADS = 2;
 template <bool kPre>
-__global__ void k_f2max(float* __restrict__ f0, float* __restrict__ f1, float* __restrict__ f2, int n,
-                        unsigned int* __restrict__ out, float a_mid, float dt, const StepDev* sd) {
+__global__ void __launch_bounds__(256) k_f2max(float4* __restrict__ f0, float4* __restrict__ f1,
+                                               float4* __restrict__ f2, int64_t quads, FastDiv drow,
+                                               uint32_t wrap, unsigned int* __restrict__ out, float a_mid, float dt,
+                                               const StepDev* sd) {
   if (sd) {  // graph mode
     a_mid = sd->h.a_mid;
     dt = sd->h.dt;
   }
-  const int64_t rows = (int64_t)n * n;
-  const int h = n >> 1;
+  // value pairs: drow.d of them a row, the last one padding; wrap = 2^32 mod
+  // drow.d brings the pair index of a mesh beyond 2^32 pairs (n > 2046) back
+  auto in_row = [&](uint64_t k) {
+    uint32_t r = (uint32_t)k;
+    r -= fdiv(r, drow) * drow.d;
+    if (k >> 32) {
+      r += (uint32_t)(k >> 32) * wrap;
+      r -= fdiv(r, drow) * drow.d;
+    }
+    return r;
+  };
   float m = 0.f;
-  for (int64_t r = blockIdx.x * (int64_t)blockDim.y + threadIdx.y; r < rows; r += (int64_t)gridDim.x * blockDim.y) {
-    const int64_t o = r * (n + 2);
-    float2* a = reinterpret_cast<float2*>(f0 + o);
-    float2* b = reinterpret_cast<float2*>(f1 + o);
-    float2* c = reinterpret_cast<float2*>(f2 + o);
-    for (int x = threadIdx.x; x < h; x += blockDim.x) {
-      float2 u = a[x], v = b[x], w = c[x];
-      m = fmaxf(m, fmaxf(f2sum(u.x, v.x, w.x), f2sum(u.y, v.y, w.y)));
-      if (kPre) {
-        a[x] = make_float2(kick_pre(u.x, a_mid, dt), kick_pre(u.y, a_mid, dt));
-        b[x] = make_float2(kick_pre(v.x, a_mid, dt), kick_pre(v.y, a_mid, dt));
-        c[x] = make_float2(kick_pre(w.x, a_mid, dt), kick_pre(w.y, a_mid, dt));
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  auto pre4 = [&](float4 v) {
+    return make_float4(kick_pre(v.x, a_mid, dt), kick_pre(v.y, a_mid, dt), kick_pre(v.z, a_mid, dt),
+                       kick_pre(v.w, a_mid, dt));
+  };
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < quads; i0 += F2_LOADS * step) {
+    float4 u[F2_LOADS], v[F2_LOADS], w[F2_LOADS];
+#pragma unroll
+    for (int j = 0; j < F2_LOADS; j++) {
+      const int64_t i = i0 + j * step;
+      if (i < quads) {
+        u[j] = f0[i];
+        v[j] = f1[i];
+        w[j] = f2[i];
       }
     }
-    if ((n & 1) && threadIdx.x == 0) {
-      const int64_t e = o + n - 1;
-      m = fmaxf(m, f2sum(f0[e], f1[e], f2[e]));
+#pragma unroll
+    for (int j = 0; j < F2_LOADS; j++) {
+      const int64_t i = i0 + j * step;
+      if (i >= quads) break;
+      const uint32_t r = in_row(2 * (uint64_t)i);  // the second pair follows it, or starts the next row
+      const float a = fmaxf(f2sum(u[j].x, v[j].x, w[j].x), f2sum(u[j].y, v[j].y, w[j].y));
+      const float b = fmaxf(f2sum(u[j].z, v[j].z, w[j].z), f2sum(u[j].w, v[j].w, w[j].w));
+      if (r != drow.d - 1) m = fmaxf(m, a);
+      if (r != drow.d - 2) m = fmaxf(m, b);
       if (kPre) {
-        f0[e] = kick_pre(f0[e], a_mid, dt);
-        f1[e] = kick_pre(f1[e], a_mid, dt);
-        f2[e] = kick_pre(f2[e], a_mid, dt);
+        f0[i] = pre4(u[j]);
+        f1[i] = pre4(v[j]);
+        f2[i] = pre4(w[j]);
       }
     }
   }
@@ -382,11 +405,11 @@ __global__ void k_f2max(float* __restrict__ f0, float* __restrict__ f1, float* _
 // the maxima pass over n^3 cells of three padded meshes
 template <bool kPre>
 void launch_f2max(cube_ctx* c, float* const f[3], int n, unsigned int* out, const float* pre) {
-  int bx = 32;
-  while (bx < 256 && bx < n / 2) bx *= 2;
-  const dim3 block(bx, 256 / bx);
-  k_f2max<kPre><<<cube_grid((int64_t)n * n, (int)block.y, 8), block, 0, c->stream>>>(
-      f[0], f[1], f[2], n, out, kPre ? pre[0] : 0.f, kPre ? pre[1] : 0.f, kPre && c->graph_mode ? c->sd : nullptr);
+  const int64_t quads = (int64_t)(n + 2) * n * n / 4;
+  k_f2max<kPre><<<cube_grid(quads, 256 * F2_LOADS, 8), 256, 0, c->stream>>>(
+      (float4*)f[0], (float4*)f[1], (float4*)f[2], quads, make_fastdiv((uint32_t)(n / 2 + 1)),
+      (uint32_t)((1ull << 32) % (uint64_t)(n / 2 + 1)), out,
+      kPre ? pre[0] : 0.f, kPre ? pre[1] : 0.f, kPre && c->graph_mode ? c->sd : nullptr);
 }
 
 // ------------------------------------------------------------------- kicks
@@ -1019,11 +1042,13 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
   k.exact_only = c->opt_exact_kicks;
   cube_phase_begin(c, PH_C_KICK);
   if (c->vp_host && !c->graph_mode) {
-    // a download is waiting for vp: kick in eight pieces of particles, each
-    // piece's codes going to the host while the next is kicked
+    // a download is waiting for vp: kick in pieces of particles, each piece's
+    // codes going to the host while the next is kicked; eight, or fewer of at
+    // least 2^18 (below that a piece's launch and copy cost more than they hide)
     const size_t bx = 3 * (size_t)c->p.izipx, bv = 3 * (size_t)c->p.izipv;
-    for (int i = 0; i < 8; i++) {
-      const int64_t p0 = c->np * i / 8, p1 = c->np * (i + 1) / 8;
+    const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(8, c->np >> 18));
+    for (int i = 0; i < pieces; i++) {
+      const int64_t p0 = c->np * i / pieces, p1 = c->np * (i + 1) / pieces;
       if (p1 <= p0) continue;
       KickArgs kp = k;
       kp.np = p1 - p0;
