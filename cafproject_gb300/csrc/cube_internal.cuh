@@ -221,6 +221,7 @@ struct cube_ctx {
   void* vp_host = nullptr;  // vp destination of a pending download
   bool pid_pending = false, xv_pending = false;
   int64_t up_np = 0;        // particle count of the pending upload's pieces
+  int up_pieces = UP_PIECES;  // how many it has (fewer for a small state)
   // per-phase timers (null when disabled)
   struct CubeTimers* timers = nullptr;
   // stats

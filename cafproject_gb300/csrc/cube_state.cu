@@ -1,6 +1,7 @@
 // cube_state.cu -- state upload/download, the per-particle cell index, the
 // velocity-code tables, the deterministic exclusive scan (the spine of
 // variables.f90:96-211) and the statistics read-back.
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -170,8 +171,9 @@ int cube_state_in(cube_ctx* c, int64_t np, const void* xp, const void* vp, const
     CUBE_CUDA(c, cudaStreamWaitEvent(s, c->ev_copy_start, 0));
     CUBE_CUDA(c, cudaMemcpyAsync(c->vfield[k], vfield, (size_t)12 * c->ncells, cudaMemcpyHostToDevice, s));
     const size_t bx = 3 * (size_t)p.izipx, bv = 3 * (size_t)p.izipv;
-    for (int i = 0; i < cube_ctx::UP_PIECES; i++) {
-      const int64_t p0 = np * i / cube_ctx::UP_PIECES, p1 = np * (i + 1) / cube_ctx::UP_PIECES;
+    c->up_pieces = (int)std::max<int64_t>(1, std::min<int64_t>(cube_ctx::UP_PIECES, np >> 18));
+    for (int i = 0; i < c->up_pieces; i++) {
+      const int64_t p0 = np * i / c->up_pieces, p1 = np * (i + 1) / c->up_pieces;
       CUBE_CUDA(c, cudaMemcpyAsync((char*)c->xp[k] + bx * p0, (const char*)xp + bx * p0, bx * (p1 - p0),
                                    cudaMemcpyHostToDevice, s));
       CUBE_CUDA(c, cudaMemcpyAsync((char*)c->vp[k] + bv * p0, (const char*)vp + bv * p0, bv * (p1 - p0),
