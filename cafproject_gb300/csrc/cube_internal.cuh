@@ -37,7 +37,7 @@ struct DevStats {
   unsigned int vmax_bits[3];
   unsigned long long npairs, itest1;
   unsigned long long ndup_list;  // entries in the extra-copy list
-  unsigned int ndense;           // destination cells left to the warp-per-cell vfield pass
+  unsigned int ndense, ndense_block;  // destination cells left to a warp, or a block, each in the vfield pass
   unsigned int vmax_est_bits[3]; // fine kick: max |v + vfield| in FP32, when the last vmax is unknown
   double testrhof, testrhoc;
   unsigned long long rhof_fix, rhoc_fix;  // deposited mass in 2^-32 fixed point

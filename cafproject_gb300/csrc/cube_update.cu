@@ -56,7 +56,8 @@ struct UpdArgs {
   int32_t* pid_new;
   int32_t* pcell_new;
   const StepDev* sd;  // graph mode: dt_mid and nlayer from the device
-  int32_t* vdense;    // destination cells over VF_DENSE particles, for k_vfield_dense
+  int32_t* vdense;    // destination cells over vf_dense particles, for k_vfield_dense
+  uint32_t vf_dense;
   int64_t p_lo;       // k_dest: first particle of this launch (particles [p_lo, np))
   int spec;           // counting path queued ahead of the check that it applies
   int rank_init;      // k_dest: set every rank to the "no rank" sentinel (for the walker)
@@ -496,19 +497,26 @@ __global__ void k_rank_place(UpdArgs a) {
   }
 }
 
-// a cell over VF_DENSE particles goes to k_vfield_dense: one thread summing
-// hundreds of particles in rank order would set the kernel's tail.  The
-// thread path loads VF_BATCH particles' codes, decoded values and source
+// A cell over vf_dense particles goes to k_vfield_dense: a warp of the thread
+// path runs as long as its fullest cell.  At 256 particles for every state, a
+// clustered one (256^3 particles at z = 0, eight a cell on average) kept 5 of 32
+// lanes busy; three times the mean count (24 there) leaves a uniform state to
+// the thread path, which then fills its warps: 0.88 -> 0.28 ms there.
+// The thread path loads VF_BATCH particles' codes, decoded values and source
 // means ahead of their (sequential) sums, so the loads of a batch overlap.
-constexpr uint32_t VF_DENSE = 256;
+constexpr uint32_t VF_BLOCK = 256;  // over this a block takes the cell, up to it a warp
+uint32_t vf_dense(const cube_ctx* c, int64_t np) {
+  return (uint32_t)std::min<int64_t>(VF_BLOCK, std::max<int64_t>(24, 3 * np / std::max<int64_t>(1, c->ncells)));
+}
 constexpr uint32_t VF_BATCH = 4;
 __global__ void k_vfield_new(UpdArgs a) {
   if (queued_in_vain(a)) return;
   for (int64_t D = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; D < a.ncells;
        D += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t cnt = (uint32_t)a.cnt_new[D];
-    if (cnt > VF_DENSE) {
-      a.vdense[atomicAdd(&a.st->ndense, 1u)] = (int32_t)D;
+    if (cnt > a.vf_dense) {  // listed: a warp's from the front, a block's from the back
+      if (cnt > VF_BLOCK) a.vdense[a.ncells - 1 - atomicAdd(&a.st->ndense_block, 1u)] = (int32_t)D;
+      else a.vdense[atomicAdd(&a.st->ndense, 1u)] = (int32_t)D;
       continue;
     }
     float acc[3];
@@ -546,44 +554,114 @@ __global__ void k_vfield_new(UpdArgs a) {
   }
 }
 
-// vfield_new of the listed dense cells, one warp per cell: the lanes load 32
-// particles' codes, decoded values and source-cell means at a time (all
-// independent), then lanes 0-2 -- one per component -- run the reference's
-// sequential real(4) sum over them in rank order, the same arithmetic as
-// k_vfield_new's thread
-__global__ void __launch_bounds__(128) k_vfield_dense(UpdArgs a) {
-  if (queued_in_vain(a)) return;
-  __shared__ float2 sdd[4][32][3];
-  __shared__ float svf[4][32][3];
-  __shared__ int scode[4][32][3];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const uint32_t n = *(volatile unsigned int*)&a.st->ndense;
-  for (int64_t it = blockIdx.x * (int64_t)(blockDim.x >> 5) + w; it < (int64_t)n; it += nw) {
-    const int64_t D = a.vdense[it];
-    const uint32_t cnt = (uint32_t)a.cnt_new[D];
-    const int64_t i0 = a.cstart_new[D];
-    float acc = lane < 3 ? __fmul_rn(a.vfield[3 * D + lane], 0.1f) : 0.f;  // vfield*weight_v
-    for (uint32_t j0 = 0; j0 < cnt; j0 += 32) {
-      const uint32_t m = min(32u, cnt - j0);
-      if ((uint32_t)lane < m) {
-        const int64_t p = a.perm[i0 + j0 + lane];
-        const int64_t S = a.pcell[p];
+// vfield_new of a listed cell by G threads (a warp or a block), G particles in
+// rank order at a time.  The sum is sequential, each step rounded to real(4),
+// so the steps are first run without their certificates and then checked: the
+// threads load their particles' values side by side and form each term as
+// float-float; three of them (one a component) run the chain, a TwoSum and two
+// additions a step; then every thread works out its own step in full from the
+// chain's sum before it.  Where the two differ the chain resumes from the exact
+// value (almost never; a chain of plain FP32 additions differed in every tenth
+// step or so).  The result is the sequential sum's to the bit.  Three lanes
+// running the full steps one after another set the kernel's tail by the
+// fullest cell: 0.62 ms for the cells over 256 of 256^3 particles at z = 0, 0.53
+// now for those over 24.
+template <int G>
+struct DenseMean {
+  float h[3][G], l[3][G], pre[3][G + 1], acc[3], fix[3];
+  int st[3], bad[3];
+};
+template <int G>
+__device__ __forceinline__ void dense_sync() {
+  if (G == 32) __syncwarp();
+  else __syncthreads();
+}
+template <int G>
+__device__ void dense_mean(const UpdArgs& a, int64_t D, DenseMean<G>& s, int tid) {
+  const int cnt = a.cnt_new[D];
+  const int64_t i0 = a.cstart_new[D];
+  if (tid < 3) s.acc[tid] = __fmul_rn(a.vfield[3 * D + tid], 0.1f);  // vfield*weight_v
+  for (int j0 = 0; j0 < cnt; j0 += G) {
+    const int m = min(G, cnt - j0);
+    int code[3] = {0, 0, 0};
+    float vfs[3] = {0.f, 0.f, 0.f};
+    float2 dd[3] = {};
+    if (tid < m) {
+      const int64_t p = a.perm[i0 + j0 + tid];
+      const int64_t S = a.pcell[p];
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-          const int vcode = load_code(a.vp, 3 * p + d, a.g.izipv);
-          scode[w][lane][d] = vcode;
-          sdd[w][lane][d] = codec_decode_ff(a.cv, vcode);
-          svf[w][lane][d] = a.vfield[3 * S + d];
-        }
+      for (int d = 0; d < 3; d++) {
+        code[d] = load_code(a.vp, 3 * p + d, a.g.izipv);
+        vfs[d] = a.vfield[3 * S + d];
       }
-      __syncwarp();
-      if (lane < 3)
-        for (uint32_t j = 0; j < m; j++) acc = accumulate_vals(a, acc, scode[w][j][lane], sdd[w][j][lane], svf[w][j][lane]);
-      __syncwarp();
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        dd[d] = codec_decode_ff(a.cv, code[d]);
+        float hi, lo;
+        two_sum(dd[d].x, vfs[d], hi, lo);
+        s.h[d][tid] = hi;
+        s.l[d][tid] = __fadd_rn(lo, dd[d].y);
+      }
     }
-    if (lane < 3) a.vfield_new[3 * D + lane] = vfield_quotient(acc, cnt, a.exact_only);
+    if (tid < 3) s.st[tid] = 0;
+    for (;;) {
+      dense_sync<G>();
+      if (tid < 3) {
+        float x = s.acc[tid];
+#pragma unroll 8
+        for (int j = s.st[tid]; j < m; j++) {
+          s.pre[tid][j] = x;
+          float t, e;
+          two_sum(x, s.h[tid][j], t, e);
+          x = __fadd_rn(t, __fadd_rn(e, s.l[tid][j]));
+        }
+        s.pre[tid][m] = x;
+        s.bad[tid] = m;
+      }
+      dense_sync<G>();
+      float r[3] = {0.f, 0.f, 0.f};
+      if (tid < m) {
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+          if (tid >= s.st[d]) {
+            r[d] = accumulate_vals(a, s.pre[d][tid], code[d], dd[d], vfs[d]);
+            if (__float_as_uint(r[d]) != __float_as_uint(s.pre[d][tid + 1])) atomicMin(&s.bad[d], tid);
+          }
+      }
+      dense_sync<G>();
+      const bool done = s.bad[0] == m && s.bad[1] == m && s.bad[2] == m;
+      if (tid < m) {
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+          if (s.bad[d] == tid) s.fix[d] = r[d];
+      }
+      dense_sync<G>();
+      if (tid < 3) {
+        s.acc[tid] = s.bad[tid] < m ? s.fix[tid] : s.pre[tid][m];
+        s.st[tid] = min(s.bad[tid] + 1, m);
+      }
+      if (done) break;  // the same for every thread
+    }
   }
+  dense_sync<G>();
+  if (tid < 3) a.vfield_new[3 * D + tid] = vfield_quotient(s.acc[tid], (uint32_t)cnt, a.exact_only);
+  dense_sync<G>();
+}
+
+__global__ void __launch_bounds__(VF_BLOCK) k_vfield_dense(UpdArgs a) {
+  if (queued_in_vain(a)) return;
+  constexpr int NW = VF_BLOCK / 32;
+  __shared__ union {
+    DenseMean<(int)VF_BLOCK> block;
+    DenseMean<32> warp[NW];
+  } s;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t nblock = *(volatile unsigned int*)&a.st->ndense_block, nwarp = *(volatile unsigned int*)&a.st->ndense;
+  for (uint32_t it = blockIdx.x; it < nblock; it += gridDim.x)
+    dense_mean<(int)VF_BLOCK>(a, a.vdense[a.ncells - 1 - it], s.block, threadIdx.x);
+  __syncthreads();
+  for (uint32_t it = blockIdx.x * NW + w; it < nwarp; it += gridDim.x * NW)
+    dense_mean<32>(a, a.vdense[it], s.warp[w], lane);
 }
 
 // U2: one thread per destination cell walks the sources in visit order.
@@ -1076,6 +1154,7 @@ static int update_x_graph(cube_ctx* c) {
   a.pid_new = c->pid[kn];
   a.pcell_new = c->pcell[kn];
   a.vdense = c->vdense;
+  a.vf_dense = vf_dense(c, c->np);
   const int B = 256;
   cudaStream_t s = c->stream;
   a.rank_init = 1;
@@ -1091,7 +1170,7 @@ static int update_x_graph(cube_ctx* c) {
   if (r) return r;
   k_rank_place<<<cube_grid(c->np, B), B, 0, s>>>(a);
   k_vfield_new<<<cube_grid(c->ncells, 128, 32), 128, 0, s>>>(a);
-  k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 16), 128, 0, s>>>(a);
+  k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 6), VF_BLOCK, 0, s>>>(a);
   k_scatter<<<cube_grid(c->np, B), B, 0, s>>>(a);
   k_scatter_xtra<<<cube_grid(c->xtra_cap, B, 2), B, 0, s>>>(a);
   CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->upd, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, s));
@@ -1160,6 +1239,7 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   a.pid_new = c->pid[kn];
   a.pcell_new = c->pcell[kn];
   a.vdense = c->vdense;
+  a.vf_dense = vf_dense(c, c->np);
   const int B = 256;
   cube_phase_begin(c, PH_UPD_DEST);
   if (c->xv_pending && c->up_np == c->np) {
@@ -1205,7 +1285,7 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   };
   auto means = [&]() -> int {
     k_vfield_new<<<cube_grid(c->ncells, 128, 32), 128, 0, c->stream>>>(a);
-    k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 16), 128, 0, c->stream>>>(a);
+    k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 6), VF_BLOCK, 0, c->stream>>>(a);
     CUBE_CUDA(c, cudaGetLastError());
     return CUBE_OK;
   };
