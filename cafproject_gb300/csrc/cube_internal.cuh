@@ -574,6 +574,22 @@ __device__ __forceinline__ float div_const(float x, float c, float rc) {
   return __fmaf_rn(r, rc, q);
 }
 
+// 1/sqrt(x) rounded to nearest, for 2^-40 <= x < 2^13 (squared distances in
+// fine cells: a code step squared at least, 27 at most; NaN for x = 0): the
+// approximate instruction, its residual e = 1 - x y^2 with the product's
+// rounding error carried along by two FMAs, and the series y (1 + e/2 + 3/8 e^2)
+// of Newton's iteration for the square root's reciprocal.  Compared with
+// __frsqrt_rn for every float of the range (cube_arith_check); eight
+// instructions and no branch, where the library's form also serves subnormals.
+__device__ __forceinline__ float rsqrt_rn(float x) {
+  float y;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  const float s = __fmul_rn(x, y);
+  float e = __fmaf_rn(-__fmaf_rn(x, y, -s), y, __fmaf_rn(-s, y, 1.0f));
+  e = __fmaf_rn(__fmul_rn(0.75f, e), e, e);
+  return __fmaf_rn(__fmul_rn(0.5f, y), e, y);
+}
+
 // one CIC kick term force*a_mid*dt/6/pi*wa*wb*wc in real(4), left to right
 // (pm.f90:146), split at the weights: kick_pre depends on the mesh point only,
 // kick_w applies the particle's three CIC weights to it

@@ -66,6 +66,7 @@ constexpr size_t PP_SMEM1B = pp_smem(PP_CAP1, PNF_MAX);
 constexpr int PP_CAP_S = 384;
 constexpr int PP_THREADS_S = 128;
 constexpr size_t PP_SMEM_S = pp_smem(PP_CAP_S, PNF_MAX);
+constexpr int PP_BIN_ORDER = 1000;  // staged particles from which a block walks in bin order
 constexpr float PP_SPARSE_FRAC = 0.25f;  // active share below which level 0 takes the small blocks
 static_assert(PP_CAP1 < 65536 && PP_CAP1 < (1 << 19), "slots are 16-bit, ranks fit 19 bits");
 static_assert(PNF_MAX < (1 << 13) && PNF1 < (1 << 8), "bins fit 13 bits (bricks) and 8 bits (cells)");
@@ -157,14 +158,17 @@ __device__ __forceinline__ void pp_fold(long long* Q, float* s, float* c) {
 }
 
 // one pair: add the force of a particle at offset r (FP32).  1/|r| is the
-// correctly rounded reciprocal square root, |r| = r^2 * (1/|r|), and 1/|r|^3
+// correctly rounded reciprocal square root (rsqrt_rn: 79 -> 66 cycles a pair and
+// warp against __frsqrt_rn; with x and y, or two pairs, in packed instructions
+// 62 and 59: the pair is bound by the FP32 pipe, which a packed one holds
+// twice as long), |r| = r^2 * (1/|r|), and 1/|r|^3
 // three more roundings: within about two ulps like the square root plus
 // division it replaces, at fewer instructions (the approximate hardware
 // reciprocal square root alone moved the codes of the strongest kicks by two)
 __device__ __forceinline__ void pair_force(const PPArgs& a, float rx, float ry, float rz, float* sum, float* comp) {
   // explicit roundings: every kernel evaluates the same bits for a pair
   float r2 = __fmaf_rn(rx, rx, __fmaf_rn(ry, ry, __fmul_rn(rz, rz)));
-  float ri = __frsqrt_rn(r2);    // +inf for the self pair
+  float ri = rsqrt_rn(r2);       // NaN for the self pair
   float rm = __fmul_rn(r2, ri);  // NaN for the self pair
   if (!(rm > a.rsoft)) return;   // merge(force,0,rmag>rsoft); self pairs excluded
   float rc = __fmul_rn(rm, a.inv_cut);
@@ -410,9 +414,13 @@ __device__ bool pp_block(const PPArgs& a, const int C0[3], const int B[3], PPSme
   // rows of fine cells (4B[0] consecutive bins each) one after another.  A
   // sparse block walks its particles in slot order.  Part `part` of `nparts`
   // walks the block's particles [i0, i1) in bin order (slots differ from one
-  // staging to the next; bin order does not).
+  // staging to the next; bin order does not).  From PP_BIN_ORDER staged
+  // particles a sparse block too takes them in bin order: neighbours' lists are
+  // about as long, so fewer lanes wait (256^3 particles at z = 0: PP 9.76 ->
+  // 9.45 ms; at 500 the bin search cost blocks of a state at z = 5 more than
+  // that, 1.05 -> 1.11 ms).
   const bool crowded = 4 * nst >= NF;
-  const bool by_bin = crowded || nparts > 1;
+  const bool by_bin = crowded || nparts > 1 || nst >= PP_BIN_ORDER;
   const int RX = 4 * B[1], nrc = RX * 4 * B[2];
   if (by_bin)
     for (int r = threadIdx.x; r < nrc; r += blockDim.x) {

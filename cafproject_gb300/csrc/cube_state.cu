@@ -544,7 +544,8 @@ extern "C" int cube_codec_check(cube_ctx* c, float sigma, const double* v, int64
 // ------------------------------------------------------ arithmetic self check
 // Every float bit pattern x (NaN excluded): div_const(x, c, RN(1/c)) against
 // the IEEE division __fdiv_rn(x, c) for c = 6 and c = pi_f, the two divisors of
-// the kick terms.  Counts differing results (bitwise) per divisor.
+// the kick terms.  Counts differing results (bitwise) per divisor; the first
+// count also takes rsqrt_rn against __frsqrt_rn over the range it is for.
 __global__ void k_arith_check(unsigned long long* mism) {
   unsigned long long m6 = 0, mpi = 0;
   const float r6 = __frcp_rn(6.0f), rpi = __frcp_rn(CUBE_PI_F);
@@ -553,6 +554,7 @@ __global__ void k_arith_check(unsigned long long* mism) {
     float x = __uint_as_float((unsigned int)i);
     if (x != x) continue;
     m6 += __float_as_uint(div_const(x, 6.0f, r6)) != __float_as_uint(__fdiv_rn(x, 6.0f));
+    if (x >= 9.094947e-13f && x < 8192.0f) m6 += __float_as_uint(rsqrt_rn(x)) != __float_as_uint(__frsqrt_rn(x));
     mpi += __float_as_uint(div_const(x, CUBE_PI_F, rpi)) != __float_as_uint(__fdiv_rn(x, CUBE_PI_F));
   }
   for (int o = 16; o > 0; o >>= 1) {

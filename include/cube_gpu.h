@@ -371,7 +371,9 @@ int cube_codec_check(cube_ctx* ctx, float sigma, const double* v, int64_t n, int
 /* Arithmetic self check: the kick terms divide by 6 and by pi_f with an
    FMA-corrected reciprocal product instead of the IEEE division; this runs
    both over every float bit pattern (NaN excluded) and writes the number of
-   differing results for each divisor into mismatches[0..1] (expected 0). */
+   differing results for each divisor into mismatches[0..1] (expected 0).  The
+   pair force's reciprocal square root against the library's, over the squared
+   distances it is for, is counted in mismatches[0] too. */
 int cube_arith_check(cube_ctx* ctx, int64_t* mismatches);
 
 /* cube_codec_check without any device allocation (no counterpart in the
