@@ -73,7 +73,7 @@ static void release(cube_ctx* c) {
   void* bufs[] = {c->xp[0], c->xp[1], c->vp[0], c->vp[1], c->pid[0], c->pid[1], c->pcell[0], c->pcell[1],
                   c->rhoc[0], c->rhoc[1],
                   c->vfield[0], c->vfield[1], c->cstart[0], c->cstart[1], c->dest, c->dframe, c->doff, c->lrank, c->offc, c->perm, c->vdense, c->rank, c->xtra,
-                  c->scan_tmp, c->red_tmp, c->tan_tab, c->codec[0].dec, c->codec[1].dec, c->codec[0].bnd, c->codec[1].bnd, c->codec[0].dech, c->codec[1].dech, c->codec[0].decf, c->codec[1].decf, c->codec[0].rt, c->codec[1].rt, c->rho_f, c->force_f[0],
+                  c->scan_tmp, c->red_tmp, c->tan_tab, c->enc_edge, c->codec[0].dec, c->codec[1].dec, c->codec[0].bnd, c->codec[1].bnd, c->codec[0].dech, c->codec[1].dech, c->codec[0].decf, c->codec[1].decf, c->codec[0].rt, c->codec[1].rt, c->rho_f, c->force_f[0],
                   c->force_f[1], c->force_f[2], c->kern_f, c->kern_f_raw, c->rho_c, c->force_c[0],
                   c->force_c[1], c->force_c[2], c->kern_c, c->fpp, c->pp_list[0], c->pp_list[1], c->pp_list[2], c->pp_list[3], c->pp_list[4], c->pp_scr_pts,
                   c->pp_lpart[0], c->pp_lpart[1], c->pp_lpart[2], c->pp_lpart[3], c->pp_lpart[4], c->red_count, c->dstats,
@@ -225,12 +225,13 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
   ALLOC(c->red_count, sizeof(unsigned));
   CUBE_CUDA(c, cudaMemsetAsync(c->red_count, 0, sizeof(unsigned), c->stream));
   ALLOC(c->tan_tab, 4 * c->nvbin);
+  ALLOC(c->enc_edge, 8 * (c->nvbin / 2));
   for (int k = 0; k < 2; k++) {
     ALLOC(c->codec[k].dec, 8 * c->nvbin);
     ALLOC(c->codec[k].dech, 8 * c->nvbin);
     ALLOC(c->codec[k].bnd, 8 * (c->nvbin / 2 + 1));
     ALLOC(c->codec[k].decf, 4 * (c->nvbin / 2 + 1));
-    ALLOC(c->codec[k].rt, 4 * (c->nvbin + 1));
+    ALLOC(c->codec[k].rt, 4 * (c->nvbin + 3));
   }
   if (owner) {
     c->rho_f = owner->rho_f;

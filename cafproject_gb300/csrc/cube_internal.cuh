@@ -133,6 +133,7 @@ struct cube_ctx {
   int red_blocks = 0;
   // velocity code tables
   float* tan_tab = nullptr;     // float(tan(pi*v/(nvbin-1))) for v in [-nvbin/2, nvbin/2)
+  double* enc_edge = nullptr;   // enc_edge[n] = smallest vcoef*|v| that encodes to n (n=1..nvbin/2-1)
   struct Codec {
     float sigma = -1.f;
     double* dec = nullptr;     // dec[v+nvbin/2] = tan code / vcoef(sigma), real(8)
@@ -140,7 +141,8 @@ struct cube_ctx {
     float* decf = nullptr;     // decf[|v|] = the float hi of |dec| (odd in v; decf[nvbin/2] from v = -nvbin/2)
     long long* bnd = nullptr;  // bnd[n] = bits of the smallest |v| that encodes to n (n=1..nvbin/2-1)
     // rt[v+nvbin/2] = the code of dec[v+nvbin/2] (a kick by zero); then one
-    // more entry, the number of codes above -nvbin/2 that it changes
+    // more entry, the number of codes above -nvbin/2 that it changes, and two
+    // of k_codec_tables' own
     int32_t* rt = nullptr;
   } codec[2];
   int codec_next = 0;
@@ -410,8 +412,8 @@ __device__ __forceinline__ long long v_encode(double v, double c, int nvbin) {
 }
 // The same encode without FP64 transcendentals.  u(v) above is a monotone
 // function of v and odd in v, so nint(u(v)) = sign(v) * #{n >= 1 : bnd[n] <= |v|},
-// where bnd[n] is the smallest double whose u reaches n - 0.5 (found once per
-// sigma by bisection over the doubles, k_encode_bounds).  An FP32 estimate
+// where bnd[n] is the smallest double whose u reaches n - 0.5 (once per sigma,
+// k_codec_tables).  An FP32 estimate
 // picks the bin; at most a step or two of exact integer comparisons of the
 // doubles' bit patterns (valid for non-negative doubles) settles it.
 __device__ __forceinline__ float approx_float_pos(long long bits) {

@@ -305,6 +305,27 @@ int cube_state_out_finish(cube_ctx* c) {
 }
 
 // ------------------------------------------------------ velocity tables
+// edge[n] = the smallest double p >= 0 with real(nvbin-1)*atan(p)/pi >= n - 0.5
+// in FP64 (n = 1..nvbin/2-1): where the encode of vcoef*v = p reaches code n
+// (update_particle.f90:117), by bisection over the ordered non-negative doubles
+// from u(0) = 0 and u(+inf) = (nvbin-1)/2 * pi/pi_f > nvbin/2 - 1.5.  It depends
+// on the code width alone, so it is found once per context; a sigma's own edges
+// follow from it by multiplications (v_edge).
+__global__ void k_encode_edges(int nvbin, double* __restrict__ edge) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nvbin / 2) return;
+  const double thr = (double)n - 0.5;
+  long long lo = 0, hi = 0x7ff0000000000000LL;
+  while (n > 0 && hi - lo > 1) {
+    const long long mid = lo + (hi - lo) / 2;
+    if (__ddiv_rn(__dmul_rn((double)(nvbin - 1), atan(__longlong_as_double(mid))), (double)CUBE_PI_F) >= thr)
+      hi = mid;
+    else
+      lo = mid;
+  }
+  edge[n] = n > 0 ? __longlong_as_double(hi) : 0.0;
+}
+
 // tan_tab[v + nvbin/2] = real(4) tan(pi*real(v)/real(nvbin-1)), the decode of
 // update_particle.f90:67, taken as the correctly rounded float(tan(double)).
 int cube_build_tables(cube_ctx* c) {
@@ -318,103 +339,104 @@ int cube_build_tables(cube_ctx* c) {
     t[i] = (float)std::tan((double)arg);
   }
   CUBE_CUDA(c, cudaMemcpyAsync(c->tan_tab, t.data(), 4 * (size_t)nv, cudaMemcpyHostToDevice, c->stream));
+  k_encode_edges<<<(nv / 2 + 127) / 128, 128, 0, c->stream>>>(nv, c->enc_edge);
+  CUBE_CUDA(c, cudaGetLastError());
+  for (int k = 0; k < 2; k++) CUBE_CUDA(c, cudaMemsetAsync(c->codec[k].rt + nv, 0, 4 * 3, c->stream));
   CUBE_CUDA(c, cudaStreamSynchronize(c->stream));
   return CUBE_OK;
 }
 
-// sigp, when set, supplies sigma from the device (graph mode)
-// decf and rt may be null; the count behind rt starts at zero here
-__global__ void k_decode_table(const float* __restrict__ tan_tab, int nv, float sigma, const float* sigp,
-                               double* __restrict__ dec, float2* __restrict__ dech, float* __restrict__ decf,
-                               int32_t* __restrict__ rt) {
-  if (sigp) sigma = *sigp;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0 && rt) rt[nv] = 0;
-  if (i < nv) {
-    double d = __ddiv_rn((double)tan_tab[i], vcoef(sigma));
-    dec[i] = d;
-    float hi = __double2float_rn(d);
-    dech[i] = make_float2(hi, __double2float_rn(__dsub_rn(d, (double)hi)));
-    if (decf && i <= nv / 2) decf[nv / 2 - i] = -hi;  // tan is odd, to the bit
-  }
-}
-
-// bnd[n] = bit pattern of the smallest double a >= 0 with
-// u(a) = real(nvbin-1)*atan(vcoef*a)/pi >= n - 0.5, i.e. where nint(u) reaches n
-// (update_particle.f90:117).  Bisection over the ordered non-negative doubles,
-// keeping u(lo) < n - 0.5 <= u(hi): u(0) = 0 < 0.5 and u(+inf) =
-// (nvbin-1)/2 * pi/pi_f > nvbin/2 - 1.5.  The bracket starts from the
-// closed-form inverse tan(thr*pi/(nvbin-1))/vcoef (a few ulps off) and widens
-// geometrically until it holds, so a boundary costs a handful of FP64 atan
-// evaluations instead of 64; the result is the same smallest double.  Bound by
-// the FP64 pipe (42 us for 2-byte codes), so a step's tables are built beside
-// its densities and transforms, on the auxiliary stream: 48^3 particles 2.62 ->
-// 2.44 ms a leg of four steps, 64^3 2.60 -> 2.41.
-__device__ __forceinline__ double enc_u(long long bits, double c, int nvbin) {
-  return __ddiv_rn(__dmul_rn((double)(nvbin - 1), atan(__dmul_rn(c, __longlong_as_double(bits)))), (double)CUBE_PI_F);
-}
-__global__ void k_encode_bounds(float sigma, const float* sigp, int nvbin, long long* __restrict__ bnd) {
-  if (sigp) sigma = *sigp;
-  int n = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  int nmax = nvbin / 2 - 1;
-  if (n == 1) bnd[0] = 0;
-  if (n > nmax) return;
-  double c = vcoef(sigma);
-  double thr = (double)n - 0.5;
-  const long long kInf = 0x7ff0000000000000LL;
-  long long lo = 0, hi = kInf;
-  const double a = tan(thr * (double)CUBE_PI_F / (double)(nvbin - 1)) / c;
-  if (a > 0.0 && a < 1.0e300) {
-    const long long g = __double_as_longlong(a);
-    long long step = 2;
-    if (enc_u(g, c, nvbin) >= thr) {
-      hi = g;
-      for (int it = 0; it < 40; it++) {
-        const long long t = g - step;
-        if (t <= 0) break;
-        if (enc_u(t, c, nvbin) < thr) {
-          lo = t;
-          break;
-        }
-        hi = t;
-        step *= 4;
-      }
-    } else {
-      lo = g;
-      for (int it = 0; it < 40; it++) {
-        const long long t = g + step;
-        if (t >= kInf) break;
-        if (enc_u(t, c, nvbin) >= thr) {
-          hi = t;
-          break;
-        }
-        lo = t;
-        step *= 4;
-      }
+// bits of the smallest double a >= 0 with fl(c*a) >= e (+inf when none has).
+// The quotient is within an ulp or two of it, so a product or three settle it;
+// a quotient that is zero, infinite or NaN takes the bisection over all doubles.
+__device__ __forceinline__ long long v_edge(double e, double c) {
+  const double q = __ddiv_rn(e, c);
+  if (q > 1.0e-300 && q < 1.0e300) {
+    long long g = __double_as_longlong(q);
+    for (int it = 0; it < 8; it++) {
+      if (!(__dmul_rn(c, __longlong_as_double(g)) >= e))
+        g++;
+      else if (__dmul_rn(c, __longlong_as_double(g - 1)) >= e)
+        g--;
+      else
+        return g;
     }
   }
+  long long lo = 0, hi = 0x7ff0000000000000LL;
   while (hi - lo > 1) {
-    long long mid = lo + (hi - lo) / 2;
-    if (enc_u(mid, c, nvbin) >= thr)
+    const long long mid = lo + (hi - lo) / 2;
+    if (__dmul_rn(c, __longlong_as_double(mid)) >= e)
       hi = mid;
     else
       lo = mid;
   }
-  bnd[n] = hi;
+  return hi;
 }
 
-// rt[v+half] = the code a zero kick gives code v: decode, then encode with the
-// same sigma (the reference's FP64 expressions, update_particle.f90:67,117);
-// a particle whose PP force is zero takes its code from here
-__global__ void k_reencode(CodecView k, const float* sigp, float sigma, int nvbin, int32_t* __restrict__ rt) {
+// A sigma's tables, thread m those of the codes m and -m (tan is odd, to the
+// bit): the decode and its float splits; bnd[m]; and rt, the code a zero kick
+// gives each code (decode, then encode with the same sigma; a particle whose PP
+// force is zero takes its code from there), found from the edges of vcoef*v.
+// decf and rt may be null; behind rt[nvbin], the count of codes it changes, lie
+// the running count and the blocks done, zero between launches.  sigp, when
+// set, supplies sigma from the device (graph mode).  Bound by the FP64 pipe: two
+// divisions and a few products a thread.  Bisecting each sigma's edges with FP64
+// arctangents, with the decode and the re-encode in kernels of their own, took
+// 42 + 9 + 8 us for 2-byte codes and 114 + 30 + 28 with 12 boxes side by side;
+// this kernel takes 6 and 23.  A leg of four steps at 64^3 particles went from
+// 1.74 to 1.66 ms, the 12 boxes' two steps from 3.29 to 2.96.
+constexpr int CT_THREADS = 128;
+__global__ void __launch_bounds__(CT_THREADS) k_codec_tables(const float* __restrict__ tan_tab,
+                                                             const double* __restrict__ edge, int nv, float sigma,
+                                                             const float* sigp, double* __restrict__ dec,
+                                                             float2* __restrict__ dech, float* __restrict__ decf,
+                                                             long long* __restrict__ bnd, int32_t* __restrict__ rt) {
   if (sigp) sigma = *sigp;
-  k.cf = (float)vcoef(sigma);
-  k.cfp = nullptr;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nvbin) return;
-  const int32_t n = (int32_t)codec_encode(k, codec_decode(k, i - k.half));
-  rt[i] = n;
-  if (i > 0 && n != i - k.half) atomicAdd(rt + nvbin, 1);
+  const int half = nv / 2, nmax = half - 1;
+  const int m = blockIdx.x * CT_THREADS + threadIdx.x;
+  int changed = 0;
+  if (m <= half) {
+    const double c = vcoef(sigma);
+    const double d = __ddiv_rn((double)tan_tab[half - m], c);  // code -m
+    const float hi = __double2float_rn(d);
+    const float lo = __double2float_rn(__dsub_rn(d, (double)hi));
+    const bool two = m > 0 && m < half;
+    dec[half - m] = d;
+    dech[half - m] = make_float2(hi, lo);
+    if (two) {
+      dec[half + m] = -d;
+      dech[half + m] = make_float2(-hi, __fsub_rn(0.f, lo));  // +0 stays +0
+    }
+    if (decf) decf[m] = -hi;
+    if (m < half) bnd[m] = m > 0 ? v_edge(edge[m], c) : 0;
+    if (rt) {
+      // the last n with edge[n] <= p; n = m but for codes past the last edge
+      const double p = __dmul_rn(c, fabs(d));
+      int n = min(m, nmax);
+      if (!(p >= edge[n]) || (n < nmax && p >= edge[n + 1])) {
+        int a = 0, b = nmax + 1;
+        while (b - a > 1) {
+          const int k = (a + b) / 2;
+          if (p >= edge[k])
+            a = k;
+          else
+            b = k;
+        }
+        n = a;
+      }
+      const int32_t sn = d < 0.0 ? -n : n;
+      rt[half - m] = sn;
+      if (two) rt[half + m] = -sn;
+      changed = m < half && sn != -m ? (two ? 2 : 1) : 0;
+    }
+  }
+  if (!rt) return;
+  changed = __syncthreads_count(changed) + __syncthreads_count(changed == 2);
+  if (threadIdx.x != 0) return;
+  unsigned* tail = (unsigned*)rt + nv + 1;
+  if (changed) atomicAdd(tail, (unsigned)changed);
+  __threadfence();
+  if (atomicInc(tail + 1, gridDim.x - 1) == gridDim.x - 1) rt[nv] = (int32_t)atomicExch(tail, 0u);
 }
 
 static void view_of(const cube_ctx* c, const cube_ctx::Codec& k, CodecView* v) {
@@ -430,17 +452,14 @@ static void view_of(const cube_ctx* c, const cube_ctx::Codec& k, CodecView* v) {
   v->rt = k.rt;
 }
 
+static void launch_codec_tables(cube_ctx* c, const cube_ctx::Codec& k, float sigma, const float* sigp) {
+  k_codec_tables<<<(c->nvbin / 2 + CT_THREADS) / CT_THREADS, CT_THREADS, 0, c->stream>>>(
+      c->tan_tab, c->enc_edge, c->nvbin, sigma, sigp, k.dec, k.dech, k.decf, k.bnd, k.rt);
+}
+
 static int build_codec(cube_ctx* c, int slot, float sigma, const float* sigp = nullptr) {
   cube_ctx::Codec& k = c->codec[slot];
-  k_decode_table<<<(c->nvbin + 255) / 256, 256, 0, c->stream>>>(c->tan_tab, c->nvbin, sigma, sigp, k.dec, k.dech,
-                                                                  k.decf, k.rt);
-  int nmax = c->nvbin / 2 - 1;
-  k_encode_bounds<<<(nmax + 127) / 128, 128, 0, c->stream>>>(sigma, sigp, c->nvbin, k.bnd);
-  if (k.rt) {
-    CodecView v;
-    view_of(c, k, &v);
-    k_reencode<<<(c->nvbin + 255) / 256, 256, 0, c->stream>>>(v, sigp, sigma, c->nvbin, k.rt);
-  }
+  launch_codec_tables(c, k, sigma, sigp);
   CUBE_CUDA(c, cudaGetLastError());
   k.sigma = sigma;
   return CUBE_OK;
@@ -653,14 +672,8 @@ extern "C" int cube_codec_check_static(cube_ctx* c, float sigma, const double* v
   view_of(c, tab, &k);
   // every early return below first drains the stream, so the lock is never
   // released with work on the shared array still in flight
-  const int nmax = c->nvbin / 2 - 1;
-  k_decode_table<<<(c->nvbin + 255) / 256, 256, 0, c->stream>>>(c->tan_tab, c->nvbin, sigma, nullptr, tab.dec,
-                                                                  tab.dech, nullptr, nullptr);
+  launch_codec_tables(c, tab, sigma, nullptr);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) {
-    k_encode_bounds<<<(nmax + 127) / 128, 128, 0, c->stream>>>(sigma, nullptr, c->nvbin, tab.bnd);
-    e = cudaGetLastError();
-  }
   if (e == cudaSuccess) e = cudaMemcpyAsync(dv, v, 8 * (size_t)n, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
     k_codec_check<<<cube_grid(n, 256), 256, 0, c->stream>>>(dv, n, vcoef_host(sigma), c->nvbin, k, dd, dt);

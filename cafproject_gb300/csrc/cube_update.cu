@@ -1000,7 +1000,10 @@ __device__ __forceinline__ void ff_add(float& hi, float& lo, float x, float xlo)
 // of a small box's step in a captured graph; a kernel of its own for the sums
 // 3.7 us and a launch.)  Each block ends in FP64 shuffles on the narrow FP64
 // pipe, so small states take fewer blocks (sigma_blocks): 2048 blocks for every
-// size took 27 us for 64^3 particles, 10 us with a block per 1024.
+// size took 27 us for 64^3 particles, 10 us with a block per 1024.  Queued
+// behind a counting path that turns out not to apply it returns at once
+// (128^3 particles in 2-byte codes beside 256^3 in 1-byte ones, two of six
+// launches: 135 us each).
 struct SigmaArgs {
   const void* vp;
   const int32_t* pcell;
@@ -1012,6 +1015,7 @@ struct SigmaArgs {
   double* part;      // 3 per block
   unsigned* count;   // blocks done; the last one leaves it at zero
   DevStats* st;      // eager: receives the sums
+  bool spec;         // queued ahead of the check that the counting path applies (st): not summed when it does not
   // graph mode: also sigma_vi_new, with the host path's arithmetic (correctly
   // rounded sqrt and division), and its vcoef for the encode estimate
   double npg;
@@ -1049,6 +1053,7 @@ __device__ void sigma_total(const SigmaArgs& a, double (*w)[SG_THREADS / 32]) {
 __global__ void __launch_bounds__(SG_THREADS) k_sigma(SigmaArgs a) {
   __shared__ double s[3][SG_THREADS / 32];
   __shared__ bool last;
+  if (a.spec && (*(volatile int*)&a.st->flags & 12)) return;  // every block, so the count stays zero
   const int64_t np = a.npp ? min(a.np, *a.npp) : a.np, ncells = a.ncells;
   const float* __restrict__ vfield = a.vfield;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1180,7 +1185,7 @@ static int update_x_graph(cube_ctx* c) {
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_aux, c->ev_aux, 0));
   const double npg = (double)(c->npglobal > 0 ? c->npglobal : c->np);
   const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, nullptr, cv.dech, c->nvbin,
-                     c->p.izipv, c->red_tmp, c->red_count, nullptr, npg, c->sd, c->sout};
+                     c->p.izipv, c->red_tmp, c->red_count, nullptr, false, npg, c->sd, c->sout};
   k_sigma<<<sigma_blocks(c, c->np), SG_THREADS, 0, c->stream_aux>>>(sg);
   CUBE_CUDA(c, cudaGetLastError());
   c->stream = c->stream_aux;
@@ -1293,7 +1298,8 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   auto sigma = [&](int64_t np_most) -> int {
     cube_phase_begin(c, PH_UPD_SIGMA);
     const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], np_most, c->ncells, c->cstart[kn] + c->ncells, cv.dech,
-                       c->nvbin, c->p.izipv, c->red_tmp, c->red_count, c->dstats, 0.0, nullptr, nullptr};
+                       c->nvbin, c->p.izipv, c->red_tmp, c->red_count, c->dstats, a.spec != 0, 0.0, nullptr,
+                       nullptr};
     k_sigma<<<sigma_blocks(c, np_most), SG_THREADS, 0, c->stream>>>(sg);
     cube_phase_end(c, PH_UPD_SIGMA);
     CUBE_CUDA(c, cudaGetLastError());
