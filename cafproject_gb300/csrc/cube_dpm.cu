@@ -70,7 +70,7 @@ struct cube_dpm {
   float* mesh = nullptr;   // padded ng^3: rho / phi
   float* adj = nullptr;    // padded ng^3: phibar / rhobar
   long long* fix = nullptr;  // ng^3 fixed-point sums of the scatters (zero between uses)
-  unsigned int* gmax = nullptr;  // device: max |gv| (float bits) for the stencil scatter's scale
+  unsigned int* gmax = nullptr;  // per step: max |gv| (float bits) for its stencil scatter's scale
   int dep_shift = 0;       // the deposit's fixed point: value = integer * 2^-dep_shift
   float* lat = nullptr;    // padded npd^3: noise / IC potential / their adjoints
   float *x = nullptr, *v = nullptr, *gx = nullptr, *gv = nullptr;
@@ -238,13 +238,18 @@ __device__ __forceinline__ int adj_shift(float kick, int64_t np, const unsigned 
 // 2^sh as a float (sh within the float exponent range)
 __device__ __forceinline__ float pow2f(int sh) { return ldexpf(1.0f, max(-126, min(127, sh))); }
 
-// max |gv| over the particles (float bits, non-negative: integer max orders them)
+// a warp's maximum of the non-negative m to *out (float bits: integer max orders
+// them); the look before the atomic keeps most warps from it
+__device__ __forceinline__ void put_max(float m, unsigned int* out) {
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0 && __float_as_uint(m) > *(volatile unsigned int*)out) atomicMax(out, __float_as_uint(m));
+}
+// max |v| of a final state's velocity cotangents
 __global__ void k_dpm_absmax(const float* __restrict__ v, int64_t n, unsigned int* __restrict__ out) {
   float m = 0.f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     m = fmaxf(m, fabsf(v[i]));
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+  put_max(m, out);
 }
 
 // fixed-point sums -> the padded FP32 mesh, zeroing the sums for their next use;
@@ -291,12 +296,41 @@ __device__ __forceinline__ float& minus_ref(Stencil& s, int d, int ax, int ay, i
 }
 
 // ------------------------------------------------------------------ kernels
-// d' = d + drift*v (when v is given), stored to dout / pos when given, then
-// the CIC deposit of mass at d'
-// (dout may be din: each thread reads its particle before writing it)
-__global__ void __launch_bounds__(256) k_dpm_deposit(const float* xin, const float* __restrict__ vin, float drift,
-                                                     int64_t np, Lattice L, float mass, float* xout,
-                                                     float* __restrict__ pos, long long* __restrict__ fix,
+// v' = v + kick * F(x), F the CIC-interpolated central-difference force of phi
+__device__ __forceinline__ void kick_at(const float* __restrict__ phi, int ng, const Cic& c, float kick, float* v) {
+  Stencil s;
+  stencil_load(phi, ng, c, s);
+  float f[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+  for (int az = 0; az < 2; az++)
+#pragma unroll
+    for (int ay = 0; ay < 2; ay++)
+#pragma unroll
+      for (int ax = 0; ax < 2; ax++) {
+        const float w = c.w[0][ax] * c.w[1][ay] * c.w[2][az];
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+          f[d] += w * (0.5f * (minus_ref(s, d, ax, ay, az) - plus_ref(s, d, ax, ay, az)));
+      }
+#pragma unroll
+  for (int d = 0; d < 3; d++) v[d] += kick * f[d];
+}
+
+// One step up to its density: with kKick the kick of the step before (potential
+// phi), the state then to save when given (a segment's start), the drift
+// d' = d + drift*v (when vin is given), stored to xout when given, and the CIC
+// deposit of mass at d'.  (The outputs may be the inputs: each thread reads its
+// particle before writing it.)  The kick beside the deposit, and the segments'
+// states from it instead of copies, save passes over the state and nodes of the
+// graph, which at 40^3 particles cost more than the work in them: there a
+// gradient went from 1.01 to 0.93 ms; at 128^3 particles on 256^3 cells kick and
+// deposit from 64 + 77 to 129 us (135 with 80 registers instead of 64), and the
+// copies of 10 us each are gone.
+template <bool kKick>
+__global__ void __launch_bounds__(256, 4) k_dpm_deposit(const float* xin, const float* vin,
+                                                     const float* __restrict__ phi, float kick, float drift,
+                                                     int64_t np, Lattice L, float mass, float* xout, float* vout,
+                                                     float* __restrict__ save, long long* __restrict__ fix,
                                                      float scale) {
   const int ng = L.ng;
   // whole warps stay in the loop for the exchanges of a lane pair
@@ -304,18 +338,27 @@ __global__ void __launch_bounds__(256) k_dpm_deposit(const float* xin, const flo
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t p = pair_particle(i);
     const bool on = p < np;
-    float x[3] = {0.f, 0.f, 0.f};
+    float x[3] = {0.f, 0.f, 0.f}, v[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int e = 0; e < 3; e++) {
       if (on) x[e] = xin[3 * p + e];
-      if (on && vin) x[e] = x[e] + drift * vin[3 * p + e];
+      if (on && vin) v[e] = vin[3 * p + e];
+    }
+    Cic c;
+    if (kKick) {
+      cic_setup(on ? p : 0, x, L, c);
+      kick_at(phi, ng, c, kick, v);
     }
 #pragma unroll
     for (int e = 0; e < 3; e++) {
+      if (kKick && on) vout[3 * p + e] = v[e];
+      if (on && save) {
+        save[3 * p + e] = x[e];
+        save[3 * (np + p) + e] = v[e];
+      }
+      if (vin) x[e] = x[e] + drift * v[e];
       if (on && xout) xout[3 * p + e] = x[e];
-      if (on && pos) pos[3 * p + e] = x[e];
     }
-    Cic c;
     cic_setup(on ? p : 0, x, L, c);
     PairRows r;
     pair_setup(c, i, np, r);
@@ -351,30 +394,17 @@ __global__ void k_dpm_green(float* __restrict__ g, int ng) {
   }
 }
 
-// v += kick * F(x), F the CIC-interpolated central-difference force of phi
-__global__ void __launch_bounds__(256) k_dpm_kick(const float* __restrict__ x, float* __restrict__ v, int64_t np,
+// the last step's kick
+__global__ void __launch_bounds__(256, 4) k_dpm_kick(const float* __restrict__ x, float* __restrict__ v, int64_t np,
                                                   Lattice L, const float* __restrict__ phi, float kick) {
-  const int ng = L.ng;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
     const float xp[3] = {x[3 * p], x[3 * p + 1], x[3 * p + 2]};
+    float vp[3] = {v[3 * p], v[3 * p + 1], v[3 * p + 2]};
     Cic c;
     cic_setup(p, xp, L, c);
-    Stencil s;
-    stencil_load(phi, ng, c, s);
-    float f[3] = {0.f, 0.f, 0.f};
+    kick_at(phi, L.ng, c, kick, vp);
 #pragma unroll
-    for (int az = 0; az < 2; az++)
-#pragma unroll
-      for (int ay = 0; ay < 2; ay++)
-#pragma unroll
-        for (int ax = 0; ax < 2; ax++) {
-          const float w = c.w[0][ax] * c.w[1][ay] * c.w[2][az];
-#pragma unroll
-          for (int d = 0; d < 3; d++)
-            f[d] += w * (0.5f * (minus_ref(s, d, ax, ay, az) - plus_ref(s, d, ax, ay, az)));
-        }
-#pragma unroll
-    for (int d = 0; d < 3; d++) v[3 * p + d] += kick * f[d];
+    for (int d = 0; d < 3; d++) v[3 * p + d] = vp[d];
   }
 }
 
@@ -382,7 +412,7 @@ __global__ void __launch_bounds__(256) k_dpm_kick(const float* __restrict__ x, f
 // the kick): gx += kick * sum_d gv_d * grad(w) . F_d (the weights move with x),
 // and phibar += the interpolation-scatter of kick * gv through the central
 // differences
-__global__ void __launch_bounds__(256) k_dpm_kick_adj(const float* __restrict__ x, const float* __restrict__ gv,
+__global__ void __launch_bounds__(256, 3) k_dpm_kick_adj(const float* __restrict__ x, const float* __restrict__ gv,
                                                       int64_t np, Lattice L, const float* __restrict__ phi, float kick,
                                                       float* __restrict__ gx, long long* __restrict__ phibar,
                                                       const unsigned int* __restrict__ gmax) {
@@ -440,12 +470,14 @@ __global__ void __launch_bounds__(256) k_dpm_kick_adj(const float* __restrict__ 
 }
 
 // adjoint of the deposit at positions x: gx += mass * grad(w) . rhobar; then
-// the drift's transpose gv += drift * gx (gv may be null)
+// the drift's transpose gv += drift * gx (gv may be null), and the largest |gv|
+// to gmax (when set) for the stencil scatter of the step before
 __global__ void __launch_bounds__(256) k_dpm_deposit_adj(const float* __restrict__ x, int64_t np, Lattice L,
                                                          const float* __restrict__ rhobar, float mass, float drift,
                                                          float* __restrict__ gx, float* __restrict__ gv,
-                                                         int accumulate) {
+                                                         int accumulate, unsigned int* __restrict__ gmax) {
   const int ng = L.ng;
+  float m = 0.f;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
     const float xp[3] = {x[3 * p], x[3 * p + 1], x[3 * p + 2]};
     Cic c;
@@ -467,9 +499,14 @@ __global__ void __launch_bounds__(256) k_dpm_deposit_adj(const float* __restrict
     for (int e = 0; e < 3; e++) {
       const float t = (accumulate ? gx[3 * p + e] : 0.f) + mass * gxp[e];
       gx[3 * p + e] = t;
-      if (gv) gv[3 * p + e] += drift * t;
+      if (gv) {
+        const float w = gv[3 * p + e] + drift * t;
+        gv[3 * p + e] = w;
+        m = fmaxf(m, fabsf(w));
+      }
     }
   }
+  if (gmax) put_max(m, gmax);
 }
 
 // Zel'dovich state from the lattice potential phi (padded npd^3, normalised):
@@ -549,12 +586,13 @@ int fix_out(cube_dpm* d, float* mesh, int sh, float kick = 0.f, const unsigned i
   return CUBE_OK;
 }
 
-int deposit(cube_dpm* d, const float* xin, const float* vin, float drift, float* xout, float* pos,
-            float* mesh = nullptr) {
+// the density at d' into mesh; with phi the kick from it first (k_dpm_deposit)
+int deposit(cube_dpm* d, float* mesh, const float* xin, const float* vin, float drift, float* xout,
+            float* save = nullptr, const float* phi = nullptr, float kick = 0.f, float* vout = nullptr) {
   cube_ctx* c = &d->base;
-  if (!mesh) mesh = d->mesh;
-  k_dpm_deposit<<<cube_grid(d->np, 256), 256, 0, c->stream>>>(xin, vin, drift, d->np, d->lat_, d->mass, xout, pos,
-                                                               d->fix, std::ldexp(1.0f, d->dep_shift));
+  const auto f = phi ? k_dpm_deposit<true> : k_dpm_deposit<false>;
+  f<<<cube_grid(d->np, 256), 256, 0, c->stream>>>(xin, vin, phi, kick, drift, d->np, d->lat_, d->mass, xout, vout, save,
+                                                  d->fix, std::ldexp(1.0f, d->dep_shift));
   CUBE_CUDA(c, cudaGetLastError());
   return fix_out(d, mesh, d->dep_shift);
 }
@@ -566,22 +604,19 @@ int nseg(const cube_dpm* d) { return (d->nsteps + d->p.ckpt_every - 1) / d->p.ck
 int record_forward(cube_dpm* d) {
   cube_ctx* c = &d->base;
   cudaStream_t s = c->stream;
-  const size_t sb = sizeof(float) * 3 * (size_t)d->np;
   int r = spectral(d, d->lat, d->filt, d->npd, d->ic_r2c, d->ic_c2r);
   if (r) return r;
   k_dpm_ic<<<cube_grid(d->np, 256), 256, 0, s>>>(d->lat, d->npd, d->step, d->vf, d->x, d->v);
   CUBE_CUDA(c, cudaGetLastError());
   for (int i = 0; i < d->nsteps; i++) {
-    if (i % d->p.ckpt_every == 0) {
-      float* slot = d->seg + (size_t)(i / d->p.ckpt_every) * 6 * d->np;
-      CUBE_CUDA(c, cudaMemcpyAsync(slot, d->x, sb, cudaMemcpyDeviceToDevice, s));
-      CUBE_CUDA(c, cudaMemcpyAsync(slot + 3 * d->np, d->v, sb, cudaMemcpyDeviceToDevice, s));
-    }
-    if ((r = deposit(d, d->x, d->v, d->drift[i], d->x, nullptr))) return r;
+    float* slot = i % d->p.ckpt_every == 0 ? d->seg + (size_t)(i / d->p.ckpt_every) * 6 * d->np : nullptr;
+    if ((r = deposit(d, d->mesh, d->x, d->v, d->drift[i], d->x, slot, i ? d->mesh : nullptr, i ? d->kick[i - 1] : 0.f,
+                     d->v)))
+      return r;
     if ((r = spectral(d, d->mesh, d->green, d->ng, d->pm_r2c, d->pm_c2r))) return r;
-    k_dpm_kick<<<cube_grid(d->np, 256), 256, 0, s>>>(d->x, d->v, d->np, d->lat_, d->mesh, d->kick[i]);
-    CUBE_CUDA(c, cudaGetLastError());
   }
+  k_dpm_kick<<<cube_grid(d->np, 256), 256, 0, s>>>(d->x, d->v, d->np, d->lat_, d->mesh, d->kick[d->nsteps - 1]);
+  CUBE_CUDA(c, cudaGetLastError());
   return CUBE_OK;
 }
 
@@ -590,39 +625,40 @@ int record_forward(cube_dpm* d) {
 int record_backward(cube_dpm* d) {
   cube_ctx* c = &d->base;
   cudaStream_t s = c->stream;
-  const size_t sb = sizeof(float) * 3 * (size_t)d->np;
   const int64_t np = d->np;
+  const size_t mesh = pad_bytes(d->ng) / sizeof(float);
   int r;
+  // gmax[i]: the largest |gv| that step i's kick is transposed with
+  CUBE_CUDA(c, cudaMemsetAsync(d->gmax, 0, sizeof(unsigned int) * d->nsteps, s));
+  k_dpm_absmax<<<cube_grid(3 * np, 256, 4), 256, 0, s>>>(d->gv, 3 * np, d->gmax + d->nsteps - 1);
+  CUBE_CUDA(c, cudaGetLastError());
   for (int j = nseg(d) - 1; j >= 0; j--) {
     const int i0 = j * d->p.ckpt_every;
     const int i1 = std::min(i0 + d->p.ckpt_every, d->nsteps);
     const float* slot = d->seg + (size_t)j * 6 * np;
-    CUBE_CUDA(c, cudaMemcpyAsync(d->x, slot, sb, cudaMemcpyDeviceToDevice, s));
-    CUBE_CUDA(c, cudaMemcpyAsync(d->v, slot + 3 * np, sb, cudaMemcpyDeviceToDevice, s));
     // re-run the segment, keeping the post-drift positions and potentials
     for (int i = i0; i < i1; i++) {
       float* pos = d->pos + (size_t)(i - i0) * 3 * np;
-      float* phi = d->phis + (size_t)(i - i0) * (pad_bytes(d->ng) / sizeof(float));
-      if ((r = deposit(d, d->x, d->v, d->drift[i], d->x, pos, phi))) return r;
+      float* phi = d->phis + (size_t)(i - i0) * mesh;
+      if (i == i0)
+        r = deposit(d, phi, slot, slot + 3 * np, d->drift[i], pos);
+      else
+        r = deposit(d, phi, pos - 3 * np, i == i0 + 1 ? slot + 3 * np : d->v, d->drift[i], pos, nullptr, phi - mesh,
+                    d->kick[i - 1], d->v);
+      if (r) return r;
       if ((r = spectral(d, phi, d->green, d->ng, d->pm_r2c, d->pm_c2r))) return r;
-      if (i + 1 < i1) {
-        k_dpm_kick<<<cube_grid(np, 256), 256, 0, s>>>(d->x, d->v, np, d->lat_, phi, d->kick[i]);
-        CUBE_CUDA(c, cudaGetLastError());
-      }
     }
     // walk it in reverse
     for (int i = i1 - 1; i >= i0; i--) {
       const float* pos = d->pos + (size_t)(i - i0) * 3 * np;
-      const float* phi = d->phis + (size_t)(i - i0) * (pad_bytes(d->ng) / sizeof(float));
-      CUBE_CUDA(c, cudaMemsetAsync(d->gmax, 0, sizeof(unsigned int), s));
-      k_dpm_absmax<<<cube_grid(3 * np, 256, 4), 256, 0, s>>>(d->gv, 3 * np, d->gmax);
+      const float* phi = d->phis + (size_t)(i - i0) * mesh;
       k_dpm_kick_adj<<<cube_grid(np, 256), 256, 0, s>>>(pos, d->gv, np, d->lat_, phi, d->kick[i], d->gx, d->fix,
-                                                         d->gmax);
+                                                         d->gmax + i);
       CUBE_CUDA(c, cudaGetLastError());
-      if ((r = fix_out(d, d->adj, 0, d->kick[i], d->gmax))) return r;
+      if ((r = fix_out(d, d->adj, 0, d->kick[i], d->gmax + i))) return r;
       if ((r = spectral(d, d->adj, d->green, d->ng, d->pm_r2c, d->pm_c2r))) return r;
       k_dpm_deposit_adj<<<cube_grid(np, 256), 256, 0, s>>>(pos, np, d->lat_, d->adj, d->mass, d->drift[i], d->gx, d->gv,
-                                                            1);
+                                                            1, i ? d->gmax + i - 1 : nullptr);
       CUBE_CUDA(c, cudaGetLastError());
     }
   }
@@ -732,7 +768,7 @@ extern "C" int cube_dpm_create(const cube_dpm_params* p, const cube_cosmology* c
       (r = dalloc(d, &d->gx, sb)) || (r = dalloc(d, &d->gv, sb)) || (r = dalloc(d, &d->seg, 2 * sb * ns)) ||
       (r = dalloc(d, &d->pos, sb * p->ckpt_every)) || (r = dalloc(d, &d->phis, pad_bytes(d->ng) * p->ckpt_every)) ||
       (r = dalloc(d, reinterpret_cast<float**>(&d->fix), sizeof(long long) * (size_t)d->ng * d->ng * d->ng)) ||
-      (r = dalloc(d, reinterpret_cast<float**>(&d->gmax), sizeof(unsigned int))))
+      (r = dalloc(d, reinterpret_cast<float**>(&d->gmax), sizeof(unsigned int) * p->max_steps)))
     return r;
   CUBE_CUDA(c, cudaMemsetAsync(d->fix, 0, sizeof(long long) * (size_t)d->ng * d->ng * d->ng, c->stream));
   // deposit sums stay below 2^61: mass * np < 2^(ilogb + 1)
@@ -832,7 +868,7 @@ extern "C" int cube_dpm_density(cube_dpm* d, const float* x, float* rho) {
   int r = ready(d);
   if (r) return r;
   if (!x || !rho) return CUBE_ERR_ARG;
-  if ((r = deposit(d, x, nullptr, 0.f, nullptr, nullptr))) return r;
+  if ((r = deposit(d, d->mesh, x, nullptr, 0.f, nullptr))) return r;
   if ((r = from_padded(d, rho, d->mesh, d->ng))) return r;
   CUBE_CUDA(&d->base, cudaStreamSynchronize(d->base.stream));
   return CUBE_OK;
@@ -845,7 +881,7 @@ extern "C" int cube_dpm_density_adjoint(cube_dpm* d, const float* x, const float
   cube_ctx* c = &d->base;
   if ((r = to_padded(d, d->adj, grho, d->ng))) return r;
   k_dpm_deposit_adj<<<cube_grid(d->np, 256), 256, 0, c->stream>>>(x, d->np, d->lat_, d->adj, d->mass, 0.f, gx, nullptr,
-                                                                   0);
+                                                                   0, nullptr);
   CUBE_CUDA(c, cudaGetLastError());
   CUBE_CUDA(c, cudaStreamSynchronize(c->stream));
   return CUBE_OK;

@@ -1,5 +1,5 @@
 """The paired stencil scatter at particle counts that leave a part of the last
-warp's pairs empty (n^3 = 8, 16 and 24 beyond a multiple of 32) and lattices
+warp's pairs empty (n^3 = 8 or 24 beyond a multiple of 32) and lattices
 of one to three cells a particle: the gradient against FP64 autograd."""
 import pytest
 
