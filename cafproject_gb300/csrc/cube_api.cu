@@ -64,6 +64,7 @@ static void release(cube_ctx* c) {
     if (c->owner->linked == c) c->owner->linked = nullptr;
     c->rho_f = c->kern_f = c->kern_f_raw = c->rho_c = c->kern_c = nullptr;
     for (int d = 0; d < 3; d++) c->force_f[d] = c->force_c[d] = nullptr;
+    c->f2_kick = nullptr;
     c->cufft_work = nullptr;
     c->plan_f_r2c = c->plan_f_c2r = c->plan_c_r2c = c->plan_c_c2r = 0;
     c->stream = nullptr;
@@ -73,7 +74,7 @@ static void release(cube_ctx* c) {
   void* bufs[] = {c->xp[0], c->xp[1], c->vp[0], c->vp[1], c->pid[0], c->pid[1], c->pcell[0], c->pcell[1],
                   c->rhoc[0], c->rhoc[1],
                   c->vfield[0], c->vfield[1], c->cstart[0], c->cstart[1], c->dest, c->dframe, c->doff, c->lrank, c->offc, c->perm, c->vdense, c->rank, c->xtra,
-                  c->scan_tmp, c->red_tmp, c->tan_tab, c->enc_edge, c->codec[0].dec, c->codec[1].dec, c->codec[0].bnd, c->codec[1].bnd, c->codec[0].dech, c->codec[1].dech, c->codec[0].decf, c->codec[1].decf, c->codec[0].rt, c->codec[1].rt, c->rho_f, c->force_f[0],
+                  c->scan_tmp, c->red_tmp, c->tan_tab, c->enc_edge, c->f2_kick, c->codec[0].dec, c->codec[1].dec, c->codec[0].bnd, c->codec[1].bnd, c->codec[0].dech, c->codec[1].dech, c->codec[0].decf, c->codec[1].decf, c->codec[0].rt, c->codec[1].rt, c->rho_f, c->force_f[0],
                   c->force_f[1], c->force_f[2], c->kern_f, c->kern_f_raw, c->rho_c, c->force_c[0],
                   c->force_c[1], c->force_c[2], c->kern_c, c->fpp, c->pp_list[0], c->pp_list[1], c->pp_list[2], c->pp_list[3], c->pp_list[4], c->pp_scr_pts,
                   c->pp_lpart[0], c->pp_lpart[1], c->pp_lpart[2], c->pp_lpart[3], c->pp_lpart[4], c->red_count, c->dstats,
@@ -234,6 +235,7 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
     ALLOC(c->codec[k].rt, 4 * (c->nvbin + 3));
   }
   if (owner) {
+    c->f2_kick = owner->f2_kick;
     c->rho_f = owner->rho_f;
     c->kern_f = owner->kern_f;
     c->rho_c = owner->rho_c;
@@ -245,6 +247,8 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
   } else {
     int64_t nfh = (int64_t)(c->nf / 2 + 1);
     int64_t fpad = 2 * nfh * c->nf * (int64_t)c->nf;  // floats of a padded fine mesh
+    ALLOC(c->f2_kick, 8);
+    CUBE_CUDA(c, cudaMemsetAsync(c->f2_kick, 0xff, 8, c->stream));
     ALLOC(c->rho_f, 4 * fpad);
     ALLOC(c->force_f[0], 3 * 4 * fpad);  // one after another, for the batched transform
     for (int d = 1; d < 3; d++) c->force_f[d] = c->force_f[0] + d * fpad;
@@ -435,6 +439,7 @@ extern "C" int cube_pm_fine_forces(cube_ctx* c, cube_stats* st) {
 extern "C" int cube_pm_fine_kick(cube_ctx* c, float a_mid, float dt) {
   int r = check_ready(c);
   if (r) return r;
+  if ((r = cube_force_settle(c, 0))) return r;
   return cube_fine_kick_impl(c, a_mid, dt);
 }
 extern "C" int cube_pm_coarse_forces(cube_ctx* c, cube_stats* st) {
@@ -445,6 +450,7 @@ extern "C" int cube_pm_coarse_forces(cube_ctx* c, cube_stats* st) {
 extern "C" int cube_pm_coarse_kick(cube_ctx* c, float a_mid, float dt, cube_stats* st) {
   int r = check_ready(c);
   if (r) return r;
+  if ((r = cube_force_settle(c, 1))) return r;
   return cube_coarse_kick_impl(c, a_mid, dt, st);
 }
 
@@ -452,12 +458,13 @@ extern "C" int cube_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_stats
   int r = check_ready(c);
   if (r) return r;
   // every stage is queued; the stats come back once, with the coarse kick's
-  const float pre[2] = {a_mid, dt};
-  if ((r = cube_fine_forces_impl(c, nullptr, pre))) return r;
-  if ((r = cube_fine_kick_impl(c, a_mid, dt, true))) return r;
+  if ((r = cube_fine_forces_impl(c, nullptr))) return r;
+  cube_force_fused(c, 0, a_mid, dt);
+  if ((r = cube_fine_kick_impl(c, a_mid, dt))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
-  if ((r = cube_coarse_forces_impl(c, nullptr, pre, true))) return r;
-  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true, true))) return r;
+  if ((r = cube_coarse_forces_impl(c, nullptr, true))) return r;
+  cube_force_fused(c, 1, a_mid, dt);
+  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true))) return r;
   if (st) cube_fine_stats(c, st);
   return CUBE_OK;
 }
@@ -471,7 +478,6 @@ extern "C" int cube_pp_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_st
   int r = check_ready(c);
   if (r) return r;
   if (!c->stream_pp) return cube_fail(c, CUBE_ERR_ARG, "PP is off for this context (pp_on = 0)");
-  const float pre[2] = {a_mid, dt};
   CUBE_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_pp, c->ev_fork, 0));
   {  // PP's launches go to its stream with its own stats
@@ -491,13 +497,15 @@ extern "C" int cube_pp_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_st
     c->hstats = h0;
     if (r) return r;
   }
-  if ((r = cube_fine_forces_impl(c, nullptr, pre))) return r;
-  if ((r = cube_coarse_forces_impl(c, nullptr, pre, true))) return r;
+  if ((r = cube_fine_forces_impl(c, nullptr))) return r;
+  cube_force_fused(c, 0, a_mid, dt);
+  if ((r = cube_coarse_forces_impl(c, nullptr, true))) return r;
+  cube_force_fused(c, 1, a_mid, dt);
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_pp, 0));
   // the fine kick applies PP's kick first (ext_pp_force.f90:116-121), then its own
-  if ((r = cube_fine_kick_impl(c, a_mid, dt, true, /*with_pp=*/true))) return r;
+  if ((r = cube_fine_kick_impl(c, a_mid, dt, /*with_pp=*/true))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
-  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st_pm, true, true))) return r;
+  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st_pm, true))) return r;
   if (st_pm) cube_fine_stats(c, st_pm);
   // PP's stats are in their host copy: the kicks waited for its stream
   DevStats* h0 = c->hstats;
@@ -517,20 +525,21 @@ extern "C" int cube_particle_mesh2(cube_ctx* c, cube_ctx* nu, float a_mid, float
   if (!nu || nu->owner != c) return cube_fail(c, CUBE_ERR_ARG, "the second species must be linked to this context");
   if (!nu->have_state) return cube_fail(c, CUBE_ERR_STATE, "no state uploaded for the linked species");
   if ((r = cube_upload_join(nu))) return cube_fail(c, r, nu->err);
-  const float pre[2] = {a_mid, dt};
   if ((r = cube_fine_density_impl(c, nullptr, false))) return r;
   if ((r = cube_fine_density_impl(nu, nullptr, true))) return cube_fail(c, r, nu->err);
-  if ((r = cube_fine_spectral_impl(c, nullptr, pre))) return r;
-  if ((r = cube_fine_kick_impl(c, a_mid, dt, true))) return r;
-  if ((r = cube_fine_kick_impl(nu, a_mid, dt, true))) return cube_fail(c, r, nu->err);
+  if ((r = cube_fine_spectral_impl(c, nullptr))) return r;
+  cube_force_fused(c, 0, a_mid, dt);
+  if ((r = cube_fine_kick_impl(c, a_mid, dt))) return r;
+  if ((r = cube_fine_kick_impl(nu, a_mid, dt))) return cube_fail(c, r, nu->err);
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193-194
   nu->sigma_vi = nu->sigma_vi_new;
   if ((r = cube_coarse_density_impl(c, nullptr, false, true))) return r;
   if ((r = cube_coarse_density_impl(nu, nullptr, true, true))) return cube_fail(c, r, nu->err);
-  if ((r = cube_coarse_spectral_impl(c, nullptr, pre))) return r;
-  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true, true))) return r;
+  if ((r = cube_coarse_spectral_impl(c, nullptr))) return r;
+  cube_force_fused(c, 1, a_mid, dt);
+  if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true))) return r;
   if (st) cube_fine_stats(c, st);
-  if ((r = cube_coarse_kick_impl(nu, a_mid, dt, st_nu, true, true))) return cube_fail(c, r, nu->err);
+  if ((r = cube_coarse_kick_impl(nu, a_mid, dt, st_nu, true))) return cube_fail(c, r, nu->err);
   // testrhof / testrhoc sum both species' mass (pm.f90:108, 258); the coarse
   // kick left the second species' deposited masses in its host stats
   if (st) {
@@ -635,6 +644,7 @@ static int field_io(cube_ctx* c, int field, void* host, bool to_host) {
     case CUBE_FIELD_RHO_F:
       return mesh_copy(c, c->rho_f, nf, host, to_host);
     case CUBE_FIELD_FORCE_F:
+      if (int r = to_host ? cube_force_settle(c, 0) : cube_force_foreign(c, 0)) return r;
       for (int d = 0; d < 3; d++) {
         int r = mesh_copy(c, c->force_f[d], nf, (char*)host + (size_t)d * 4 * c->nfine, to_host);
         if (r) return r;
@@ -643,6 +653,7 @@ static int field_io(cube_ctx* c, int field, void* host, bool to_host) {
     case CUBE_FIELD_RHO_C:
       return mesh_copy(c, c->rho_c, nc, host, to_host);
     case CUBE_FIELD_FORCE_C:
+      if (int r = to_host ? cube_force_settle(c, 1) : cube_force_foreign(c, 1)) return r;
       for (int d = 0; d < 3; d++) {
         int r = mesh_copy(c, c->force_c[d], nc, (char*)host + (size_t)d * 4 * c->ncells, to_host);
         if (r) return r;

@@ -117,11 +117,10 @@ int box_step(cube_ctx* c, int ncell, const float2* sched, int nsteps) {
   int r = cube_update_x_impl(c, 0.f, 0.f, 0.f, nullptr);
   if (r) return r;
   if (c->p.pp_on && (r = cube_pp_impl(c, 0.f, 0.f, nullptr))) return r;
-  const float pre[2] = {0.f, 0.f};
-  if ((r = cube_fine_forces_impl(c, nullptr, pre))) return r;
-  if ((r = cube_fine_kick_impl(c, 0.f, 0.f, true))) return r;
-  if ((r = cube_coarse_forces_impl(c, nullptr, pre, true))) return r;
-  return cube_coarse_kick_impl(c, 0.f, 0.f, nullptr, true, true);
+  if ((r = cube_fine_forces_impl(c, nullptr))) return r;
+  if ((r = cube_fine_kick_impl(c, 0.f, 0.f))) return r;
+  if ((r = cube_coarse_forces_impl(c, nullptr, true))) return r;
+  return cube_coarse_kick_impl(c, 0.f, 0.f, nullptr, true);
 }
 
 int capture(cube_batch* b, int parity) {
@@ -335,6 +334,8 @@ int graph_steps(cube_batch* b, int n) {
     restore(c, b->snap[last][i]);
     c->sigma_vi = c->sigma_vi_new = hs[i].sigma_vi;
     for (int d = 0; d < 3; d++) c->vmax_prev[d] = hs[i].vmax_prev[d];
+    const float2 s = b->hsched[(size_t)i * b->nsteps + b->steps_done - 1];
+    for (int k = 0; k < 2; k++) cube_force_fused(c, k, s.y, s.x);
     // the step's own sigma_vi tables are the other slot's
     const int slot = (int)(b->steps_done & 1);
     c->codec[slot].sigma = hs[i].sigma_vi;

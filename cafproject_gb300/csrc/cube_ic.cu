@@ -504,6 +504,7 @@ static int ic_impl(cube_ctx* c, const cube_cosmology* cs, float z_init, uint32_t
   CUBE_FFT(c, cufftExecR2C(c->plan_f_r2c, c->rho_f, (cufftComplex*)c->rho_f));
   // 2. corrected potential kernel in force plane 0, tables in force plane 1
   float* kp = c->force_f[0];
+  if (int rf = cube_force_foreign(c, 0)) return rf;
   float* dtab = reinterpret_cast<float*>(c->force_f[1]);
   ScaleArgs sa;
   int r = ic_kernel_spectrum(c, nf, c->plan_f_r2c, c->plan_f_c2r, kp, dtab, *cs, a, sa);

@@ -132,6 +132,15 @@ struct cube_ctx {
   unsigned* red_count = nullptr;  // blocks of k_sigma done (zero between launches)
   int red_blocks = 0;
   // velocity code tables
+  // The kicks' look at the force meshes, beside them on their owner: the bits of
+  // the maxima of force^2 (fine, coarse), NaN when the meshes' content is not
+  // the last transforms'.  force_pre: a fused step left the meshes as forces
+  // where its caller finds force*a_mid*dt/6/pi (get_field)
+  unsigned* f2_kick = nullptr;
+  struct ForcePre {
+    bool on = false;
+    float a_mid = 0.f, dt = 0.f;
+  } force_pre[2];
   float* tan_tab = nullptr;     // float(tan(pi*v/(nvbin-1))) for v in [-nvbin/2, nvbin/2)
   double* enc_edge = nullptr;   // enc_edge[n] = smallest vcoef*|v| that encodes to n (n=1..nvbin/2-1)
   struct Codec {
@@ -622,6 +631,11 @@ inline float bits_float(unsigned int u) {
 __device__ __forceinline__ void atomic_max_pos(unsigned int* addr, float v) {
   atomicMax(addr, __float_as_uint(v));
 }
+// the same of a non-negative value per thread, once per warp
+__device__ __forceinline__ void warp_max_pos(unsigned int* addr, float v) {
+  const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
+  if ((threadIdx.x & 31) == 0) atomicMax(addr, m);
+}
 
 // ------------------------------------------------------- block helpers
 // In-place exclusive scan of n ints by the whole block (blockDim.x a multiple
@@ -739,17 +753,21 @@ int cube_pp_finish(cube_ctx* c, cube_stats* st, bool fetched = false);  // fetch
 int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false);
 // fresh (the coarse stages): the stats were zeroed by this step's fine density
 int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false, bool fresh = false);
-// pre (a_mid, dt) non-null: after the maxima, the force meshes are rewritten
-// as the mesh part of the kick term, force*a_mid*dt/6/pi, and the kick that
-// follows is given pre=true (fused step only; the stage calls keep forces)
-int cube_fine_forces_impl(cube_ctx* c, cube_stats* st, const float* pre = nullptr);
+int cube_fine_forces_impl(cube_ctx* c, cube_stats* st);
+// the force meshes' content as the fused step's caller finds it (ForcePre); and
+// that of other origin than the transforms'
+int cube_force_settle(cube_ctx* c, int coarse);
+int cube_force_foreign(cube_ctx* c, int coarse);
+inline void cube_force_fused(cube_ctx* c, int coarse, float a_mid, float dt) {
+  (c->owner ? c->owner : c)->force_pre[coarse] = {true, a_mid, dt};
+}
 // with_pp: first apply the PP kick that cube_pp_launch(.., defer_kick) left
 // to the fine kick (eager mode)
-int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool pre = false, bool with_pp = false);
-int cube_coarse_forces_impl(cube_ctx* c, cube_stats* st, const float* pre = nullptr, bool fresh = false);
-int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool pre = false, bool fresh = false);
-int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre);
-int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre);
+int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool with_pp = false);
+int cube_coarse_forces_impl(cube_ctx* c, cube_stats* st, bool fresh = false);
+int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool fresh = false);
+int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st);
+int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st);
 int cube_pk_deposit(cube_ctx* c, int ng, float* rho, unsigned long long* total);
 int dep_shift(float mass);  // deposits' fixed point: total = integer * 2^-dep_shift(mass)
 // initial-condition pieces shared with the differentiable form (cube_ic.cu):

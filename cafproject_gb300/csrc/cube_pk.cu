@@ -176,6 +176,7 @@ extern "C" int cube_power_spectrum(cube_ctx* c, int ng, float box, const float* 
   CUBE_CUDA(c, cudaSetDevice(c->device));
   if (int r = cube_upload_join(c)) return r;
   cudaStream_t s = c->stream;
+  if (int rf = cube_force_foreign(c, 0)) return rf;
   float* m1 = c->force_f[0];
   float* m2 = c->force_f[1];
   double* part = reinterpret_cast<double*>(c->force_f[2]);

@@ -320,8 +320,11 @@ int launch_coarse_deposit(cube_ctx* c, const DepArgs& a) {
 
 // ------------------------------------------------------- spectral multiply
 // out_d = i*K_d*rho_k for the three components in one pass (pm.f90:119-120)
+// (and *f2 cleared for the forces' maximum)
 __global__ void k_green3(const float2* __restrict__ rk, const float* __restrict__ kern, int64_t n,
-                         float2* __restrict__ o0, float2* __restrict__ o1, float2* __restrict__ o2) {
+                         float2* __restrict__ o0, float2* __restrict__ o1, float2* __restrict__ o2,
+                         unsigned* __restrict__ f2) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *f2 = 0u;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float2 r = rk[i];
     float k0 = kern[i], k1 = kern[n + i], k2 = kern[2 * n + i];
@@ -331,29 +334,20 @@ __global__ void k_green3(const float2* __restrict__ rk, const float* __restrict_
   }
 }
 
-// maxval(sum(force**2,1)) over the mesh (pm.f90:126, 315), and for kPre each
-// force value rewritten as its kick factor force*a_mid*dt/6/pi.  Bound by
-// memory (24 bytes a cell for kPre): the three padded meshes are walked as flat
-// arrays of 16 bytes, F2_LOADS of each in flight a thread, and the two values
-// of padding behind each row (n even) are left out of the maximum.  Row by row
-// in 8 bytes it took 4.48 ms at 1024^3 and 12.6 us at 128^3 (three quarters of
-// the threads idle there), 4.10 ms and 7.7 us flat; 3.82 ms at the copy rate.
-// (Repeating a row's first value in its padding, to spare the kicks the wrap in
-// x, took 6.5 ms instead of 4.6 row by row: the padding shares its sector with
-// the next row's start, whose load another block has pending.)
+// maxval(sum(force**2,1)) over the mesh (pm.f90:126, 315).  Bound by memory (12
+// bytes a cell): the three padded meshes are walked as flat arrays of 16 bytes,
+// F2_LOADS of each in flight a thread, and the two values of padding behind each
+// row (n even) are left out of the maximum.  While it also rewrote each force as
+// its kick factor (24 bytes a cell) it took 4.10 ms at 1024^3; 1.77 now, 1.90 at
+// the copy rate.
 __device__ __forceinline__ float f2sum(float a, float b, float c) {
   return __fadd_rn(__fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b)), __fmul_rn(c, c));
 }
 constexpr int F2_LOADS = 2;
-template <bool kPre>
-__global__ void __launch_bounds__(256) k_f2max(float4* __restrict__ f0, float4* __restrict__ f1,
-                                               float4* __restrict__ f2, int64_t quads, FastDiv drow,
-                                               uint32_t wrap, unsigned int* __restrict__ out, float a_mid, float dt,
-                                               const StepDev* sd) {
-  if (sd) {  // graph mode
-    a_mid = sd->h.a_mid;
-    dt = sd->h.dt;
-  }
+__global__ void __launch_bounds__(256) k_f2max(const float4* __restrict__ f0, const float4* __restrict__ f1,
+                                               const float4* __restrict__ f2, int64_t quads, FastDiv drow,
+                                               uint32_t wrap, unsigned int* __restrict__ out,
+                                               unsigned int* __restrict__ out2) {
   // value pairs: drow.d of them a row, the last one padding; wrap = 2^32 mod
   // drow.d brings the pair index of a mesh beyond 2^32 pairs (n > 2046) back
   auto in_row = [&](uint64_t k) {
@@ -365,12 +359,11 @@ __global__ void __launch_bounds__(256) k_f2max(float4* __restrict__ f0, float4* 
     }
     return r;
   };
+  __shared__ unsigned s_max;
+  if (threadIdx.x == 0) s_max = 0u;
+  __syncthreads();
   float m = 0.f;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  auto pre4 = [&](float4 v) {
-    return make_float4(kick_pre(v.x, a_mid, dt), kick_pre(v.y, a_mid, dt), kick_pre(v.z, a_mid, dt),
-                       kick_pre(v.w, a_mid, dt));
-  };
   for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < quads; i0 += F2_LOADS * step) {
     float4 u[F2_LOADS], v[F2_LOADS], w[F2_LOADS];
 #pragma unroll
@@ -391,25 +384,19 @@ __global__ void __launch_bounds__(256) k_f2max(float4* __restrict__ f0, float4* 
       const float b = fmaxf(f2sum(u[j].z, v[j].z, w[j].z), f2sum(u[j].w, v[j].w, w[j].w));
       if (r != drow.d - 1) m = fmaxf(m, a);
       if (r != drow.d - 2) m = fmaxf(m, b);
-      if (kPre) {
-        f0[i] = pre4(u[j]);
-        f1[i] = pre4(v[j]);
-        f2[i] = pre4(w[j]);
-      }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.f) atomic_max_pos(out, m);
+  warp_max_pos(&s_max, m);
+  __syncthreads();
+  if (threadIdx.x < 2) atomicMax(threadIdx.x ? out2 : out, s_max);
 }
 
 // the maxima pass over n^3 cells of three padded meshes
-template <bool kPre>
-void launch_f2max(cube_ctx* c, float* const f[3], int n, unsigned int* out, const float* pre) {
+void launch_f2max(cube_ctx* c, float* const f[3], int n, unsigned int* out, unsigned int* out2) {
   const int64_t quads = (int64_t)(n + 2) * n * n / 4;
-  k_f2max<kPre><<<cube_grid(quads, 256 * F2_LOADS, 8), 256, 0, c->stream>>>(
-      (float4*)f[0], (float4*)f[1], (float4*)f[2], quads, make_fastdiv((uint32_t)(n / 2 + 1)),
-      (uint32_t)((1ull << 32) % (uint64_t)(n / 2 + 1)), out,
-      kPre ? pre[0] : 0.f, kPre ? pre[1] : 0.f, kPre && c->graph_mode ? c->sd : nullptr);
+  k_f2max<<<cube_grid(quads, 256 * F2_LOADS, 8), 256, 0, c->stream>>>(
+      (const float4*)f[0], (const float4*)f[1], (const float4*)f[2], quads, make_fastdiv((uint32_t)(n / 2 + 1)),
+      (uint32_t)((1ull << 32) % (uint64_t)(n / 2 + 1)), out, out2);
 }
 
 // ------------------------------------------------------------------- kicks
@@ -424,6 +411,7 @@ struct KickArgs {
   const int64_t* cstart;
   const float* vfield;
   const float* f[3];
+  const unsigned* f2;      // bits of the maximum of force^2 over these meshes, or NaN
   CodecView cin, cout;     // decode with sigma_in, encode with sigma_out
   float a_mid, dt;
   unsigned int* vmax_bits; // coarse kick only: exact vmax per component
@@ -448,14 +436,21 @@ __device__ __forceinline__ float kick_tau(const KickArgs& a, int d) {
 
 // The kick velocity of the reference is the FP64 chain
 //   v = decode; v = v + t1; ...; v = v + t8       (pm.f90:145-153)
-// with t_i the real(4) CIC terms.  The fast path forms V_f = fl32(hi(decode) + S)
-// with S the FP32 sum of the terms; its distance from the reference value is
-// bounded by
-//   gamma_7 sum|t_i| + 2^-24 (|decode| + |V_f|) + 9*2^-53 (|decode| + sum|t_i| + |V_f|)
-// (recursive-summation bound, gamma_7 = 7u/(1-7u), u = 2^-24; the decode table's
-// float hi is within half an ulp).  certify_code keeps the code only when every
-// double inside that bound encodes to it; otherwise the lane runs the exact
-// chain, so the stored code is always the reference's.
+// with t_i the real(4) CIC terms force*a_mid*dt/6/pi*w*w*w (seven roundings
+// each).  The fast path forms the eight weights w*K*w*w once a particle, K =
+// kick_pre(1) (three roundings, and three more), S = sum force*weight by FMAs
+// (eight) and V_f = fl32(hi(decode) + S); its distance from the reference value
+// is bounded by
+//   gamma_21 sum|force*weight| + 2^-24 (|decode| + |V_f|) + 9*2^-53 (|decode| + sum + |V_f|)
+// (gamma_21 = 21u/(1-21u), 21u = 1.2517e-6, u = 2^-24; the decode table's float
+// hi is within half an ulp), and 1e-24 for products in the denormal range (a
+// term's lose 2^-150 each, of which the first is multiplied by dt < 1e20).
+// Forces or factors so large that the reference's own products may overflow (by
+// the mesh's maximum) are left to the exact chain, as is a factor below the
+// normal floats' range (kick_factor).
+// certify_code keeps the code only when every double inside that bound encodes
+// to it; otherwise the lane runs the exact chain, so the stored code is always
+// the reference's.
 //
 // The exact chain (and, in the coarse kick, the exact |v + vfield| of lanes
 // that may set vmax) is needed by a few components in a hundred, but a warp
@@ -472,7 +467,10 @@ __device__ __forceinline__ float kick_tau(const KickArgs& a, int d) {
 // component instead of five), one row address per pair of x corners, and every
 // component unrolled (indexing the codes in a loop had put them in local
 // memory): 6.74 -> 4.38 ms fine and 6.43 -> 3.70 ms coarse at 512^3 particles,
-// 63 % of the L1's wavefront rate now.
+// 63 % of the L1's wavefront rate.  The forces as the transforms leave them,
+// their factor in the particle's weights, cost the kicks 0.1 ms (4.29 and 3.75)
+// and spare the maxima pass 2.3 ms of writing; more than 64 registers, or spills
+// to hold the factor in one (it lies in shared memory), cost more than that.
 constexpr int KICK_Q = 64;  // queue entries per warp: at most 31 pending + 32 from one component
 __device__ __forceinline__ unsigned long long kick_qkey(int64_t p, int d, int code) {
   return ((unsigned long long)p << 18) | ((unsigned long long)(code & 0xffff) << 2) | (unsigned long long)d;
@@ -521,13 +519,23 @@ __device__ __forceinline__ void kick_corners(const KickArgs& a, int64_t p, KickC
   k.row[1][1] = (uint32_t)i2[1] + (uint32_t)n * (uint32_t)i2[2];
 }
 
-// the eight real(4) CIC terms of the component whose mesh is F, in the
-// reference's order: corners c111, c211, c121, c112, c122, c212, c221, c222
-template <bool kFine, bool kPre>
-__device__ __forceinline__ void kick_terms(const KickArgs& a, const KickCorners& k, const float* F, float t[8]) {
+// K, or NaN (which no certificate passes) where the fast path does not apply: it
+// takes K = 0 or a normal float with room for a weight below it, and no product
+// of a force near overflow.  f2 is the maximum of force^2 over the mesh, NaN when
+// that is not known
+__device__ __forceinline__ float kick_factor(float a_mid, float dt, float f2) {
+  const float K = kick_pre(1.0f, a_mid, dt);
+  const float big = fmaxf(fabsf(a_mid), fmaxf(fabsf(dt), fabsf(__fmul_rn(a_mid, dt))));
+  const bool ok = (a_mid == 0.f || dt == 0.f || fabsf(K) >= 1.0e-30f) && big < 1.0e20f && f2 < 1.0e30f;
+  return ok ? K : __int_as_float(0x7fffffff);
+}
+
+// the force of the component whose mesh is F at the eight corners, [z][y][x]
+template <bool kFine>
+__device__ __forceinline__ void kick_gather(const KickArgs& a, const KickCorners& k, const float* F,
+                                            float v[2][2][2]) {
   const uint32_t stride = (uint32_t)((kFine ? a.g.nf : a.g.nc) + 2) * 4u;  // bytes of a padded row
   const char* base = reinterpret_cast<const char*>(F + k.x);
-  float v[2][2][2];  // [z][y][x]
 #pragma unroll
   for (int z = 0; z < 2; z++)
 #pragma unroll
@@ -536,33 +544,29 @@ __device__ __forceinline__ void kick_terms(const KickArgs& a, const KickCorners&
       v[z][y][0] = __ldg(r);
       v[z][y][1] = __ldg(r + k.dx);
     }
-  auto term = [&](int x, int y, int z) {
-    const float wx = x ? k.d2[0] : k.d1[0], wy = y ? k.d2[1] : k.d1[1], wz = z ? k.d2[2] : k.d1[2];
-    return kPre ? kick_w(v[z][y][x], wx, wy, wz) : kick_term(v[z][y][x], kick_amid(a), kick_dt(a), wx, wy, wz);
-  };
-  t[0] = term(0, 0, 0);
-  t[1] = term(1, 0, 0);
-  t[2] = term(0, 1, 0);
-  t[3] = term(0, 0, 1);
-  t[4] = term(0, 1, 1);
-  t[5] = term(1, 0, 1);
-  t[6] = term(1, 1, 0);
-  t[7] = term(1, 1, 1);
 }
 
 // one queued component on the reference's FP64 chain: its code, and in the
 // coarse kick vmax=max(vmax,abs(vreal+vfield)) (pm.f90:349) as real(4)
-template <bool kFine, bool kPre>
+template <bool kFine>
 __device__ __noinline__ void kick_exact_entry(const KickArgs& a, unsigned long long key, float vm[3]) {
   const int64_t p = (int64_t)(key >> 18);
   const int d = (int)(key & 3ull);
   const int code = (int)(int16_t)(uint16_t)((key >> 2) & 0xffffull);
   KickCorners k;
   kick_corners<kFine>(a, p, k);
-  float t[8];
-  kick_terms<kFine, kPre>(a, k, d == 0 ? a.f[0] : (d == 1 ? a.f[1] : a.f[2]), t);
+  float f[2][2][2];
+  kick_gather<kFine>(a, k, d == 0 ? a.f[0] : (d == 1 ? a.f[1] : a.f[2]), f);
   double v = codec_decode(a.cin, code);
-  for (int i = 0; i < 8; i++) v = __dadd_rn(v, (double)t[i]);
+  // the real(4) CIC terms in the reference's order: corners c111, c211, c121,
+  // c112, c122, c212, c221, c222
+  constexpr int kX = 0xe2, kY = 0xd4, kZ = 0xb8;  // bit i: the upper corner of term i
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int x = (kX >> i) & 1, y = (kY >> i) & 1, z = (kZ >> i) & 1;
+    v = __dadd_rn(v, (double)kick_term(f[z][y][x], kick_amid(a), kick_dt(a), x ? k.d2[0] : k.d1[0],
+                                       y ? k.d2[1] : k.d1[1], z ? k.d2[2] : k.d1[2]));
+  }
   if (!kFine) {
     const double w = fabs(__dadd_rn(v, (double)a.vfield[3 * (int64_t)k.cell + d]));
     const float wf = __double2float_rn(w);
@@ -573,8 +577,7 @@ __device__ __noinline__ void kick_exact_entry(const KickArgs& a, unsigned long l
   if (!a.vmax_only) store_code(a.vp_out, 3 * p + d, a.g.izipv, codec_encode(a.cout, v));
 }
 
-// kPre: the meshes hold force*a_mid*dt/6/pi already (k_f2max<true>)
-template <bool kFine, bool kPre>
+template <bool kFine>
 __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
   if (a.vmax_only && a.sd) {  // graph mode: the exact vmax rerun runs only when some component needs it
     bool need = false;
@@ -590,6 +593,13 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
   float vlo[3] = {0.f, 0.f, 0.f};  // coarse: lower bounds of |v + vfield|
   // the zero-kick codes are the codes themselves, but for -nvbin/2, when the
   // table's count says so
+  __shared__ float s_K;
+  __shared__ unsigned s_max[6];  // float bits: vm, vlo
+  if (threadIdx.x < 6) s_max[threadIdx.x] = 0u;
+  if (threadIdx.x == 0)
+    s_K = a.exact_only ? __int_as_float(0x7fffffff)
+                       : kick_factor(kick_amid(a), kick_dt(a), __uint_as_float(__ldg(a.f2)));
+  __syncthreads();
   const bool rt_same = kFine && a.pp_act && __ldg(a.cin.rt + 2 * a.cin.half) == 0;
   // whole warps iterate together (the queue's ballots); lanes past the end
   // compute on the last particle and store nothing
@@ -599,6 +609,9 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
     const int64_t p = valid ? p0 : a.np - 1;
     KickCorners k;
     kick_corners<kFine>(a, p, k);
+    const float w0 = __fmul_rn(k.d1[0], s_K), w1 = __fmul_rn(k.d2[0], s_K);
+    const float w[2][2] = {{__fmul_rn(k.d1[1], k.d1[2]), __fmul_rn(k.d2[1], k.d1[2])},
+                           {__fmul_rn(k.d1[1], k.d2[2]), __fmul_rn(k.d2[1], k.d2[2])}};  // [z][y]
     int codes[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) codes[d] = load_code(a.vp_in, 3 * p + d, g.izipv);
@@ -618,19 +631,22 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
     }
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      float t[8];
-      kick_terms<kFine, kPre>(a, k, a.f[d], t);
+      float f[2][2][2];
+      kick_gather<kFine>(a, k, a.f[d], f);
       const float dh = codec_decode_f(a.cin, codes[d]);
-      float S = t[0], T = fabsf(t[0]);
+      float S = 0.f, T = 0.f;
 #pragma unroll
-      for (int i = 1; i < 8; i++) {
-        S = __fadd_rn(S, t[i]);
-        T = __fadd_rn(T, fabsf(t[i]));
-      }
+      for (int z = 0; z < 2; z++)
+#pragma unroll
+        for (int y = 0; y < 2; y++) {
+          const float f0 = f[z][y][0], f1 = f[z][y][1];
+          S = __fmaf_rn(__fmaf_rn(f1, w1, __fmul_rn(f0, w0)), w[z][y], S);
+          T = __fmaf_rn(__fmaf_rn(fabsf(f1), fabsf(w1), fabsf(__fmul_rn(f0, w0))), w[z][y], T);
+        }
       const float vf = __fadd_rn(dh, S);
-      const float E = 1.25f * (T * 4.76837158e-7f + (fabsf(dh) + fabsf(vf)) * 6.0e-8f + T * 1.0e-15f);
+      const float E = __fmaf_rn(T * 1.3e-6f + (fabsf(dh) + fabsf(vf)) * 6.0e-8f, 1.25f, 1.0e-24f);
       int n;
-      bool fast = certify_code(fabsf(vf), E, a.cout, &n) && !a.exact_only;
+      bool fast = certify_code(fabsf(vf), E, a.cout, &n);
       if (!kFine) {
         const float vfd = a.vfield[3 * (int64_t)k.cell + d];
         // |v + vfield| of the reference's FP64 v lies in [lo, ub]
@@ -652,7 +668,7 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
         // the chain for 32 queued entries at a time, one per lane
         if (qn >= 32) {
           __syncwarp();
-          kick_exact_entry<kFine, kPre>(a, s_q[wq][qn - 32 + lane], vm);
+          kick_exact_entry<kFine>(a, s_q[wq][qn - 32 + lane], vm);
           qn -= 32;
           __syncwarp();
         }
@@ -661,22 +677,30 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
   }
   __syncwarp();
   if (lane < qn) {
-    kick_exact_entry<kFine, kPre>(a, s_q[wq][lane], vm);
+    kick_exact_entry<kFine>(a, s_q[wq][lane], vm);
   }
-  if (!kFine || a.vmax_est) {
-    for (int d = 0; d < 3; d++) {
-      float m = vm[d];
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if ((threadIdx.x & 31) == 0) atomic_max_pos(kFine ? &a.vmax_est[d] : &a.vmax_bits[d], m);
-    }
+  // the block's maxima first: an atomic per warp and maximum, all on one
+  // sector, took a third of a millisecond of 256^3 particles' coarse kick
+  const bool mv = !kFine || a.vmax_est, ml = !kFine && !a.vmax_only;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    if (mv) warp_max_pos(&s_max[d], vm[d]);
+    if (ml) warp_max_pos(&s_max[3 + d], vlo[d]);
   }
-  if (!kFine && !a.vmax_only) {
-    for (int d = 0; d < 3; d++) {
-      float m = vlo[d];
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      if ((threadIdx.x & 31) == 0 && m > 0.f) atomic_max_pos(&a.vmax_lo[d], m);
-    }
-  }
+  __syncthreads();
+  const int t = threadIdx.x;
+  if (t < 3 && mv) atomicMax(kFine ? &a.vmax_est[t] : &a.vmax_bits[t], s_max[t]);
+  if (t >= 3 && t < 6 && ml) atomicMax(&a.vmax_lo[t - 3], s_max[t]);
+}
+
+// The blocks that an SM holds, once: every block ends in its warps' part-filled
+// queues, which cost as much as full ones, so fewer blocks are better (256^3
+// particles, coarse: 0.96 ms with 4 a SM, 1.13 with 16, 2.05 with a particle a
+// thread; 108^3: 0.18, 0.26, 0.31).  Above 2^26 particles the queues' share is
+// small and the balance of more blocks gives more (512^3, fine: 13.3 against 12.9).
+template <bool kFine>
+void launch_kick(cube_ctx* c, const KickArgs& k) {
+  k_kick<kFine><<<cube_grid(k.np, 256, k.np > (int64_t)1 << 26 ? 16 : 4), 256, 0, c->stream>>>(k);
 }
 
 }  // namespace
@@ -819,6 +843,31 @@ int cube_kernels_init(cube_ctx* c, const float* fine_table, const float* coarse_
   return CUBE_OK;
 }
 
+namespace {
+__global__ void k_force_pre(float* __restrict__ f, int64_t n, float a_mid, float dt) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    f[i] = kick_pre(f[i], a_mid, dt);
+}
+}  // namespace
+
+int cube_force_foreign(cube_ctx* c, int coarse) {
+  (c->owner ? c->owner : c)->force_pre[coarse].on = false;
+  CUBE_CUDA(c, cudaMemsetAsync(c->f2_kick + coarse, 0xff, 4, c->stream));
+  return CUBE_OK;
+}
+
+int cube_force_settle(cube_ctx* c, int coarse) {
+  const cube_ctx::ForcePre pre = (c->owner ? c->owner : c)->force_pre[coarse];
+  if (!pre.on) return CUBE_OK;
+  const int n = coarse ? c->p.nc : c->nf;
+  const int64_t cells = (int64_t)(n + 2) * n * n;
+  for (int d = 0; d < 3; d++)
+    k_force_pre<<<cube_grid(cells, 256), 256, 0, c->stream>>>(coarse ? c->force_c[d] : c->force_f[d], cells, pre.a_mid,
+                                                               pre.dt);
+  CUBE_CUDA(c, cudaGetLastError());
+  return cube_force_foreign(c, coarse);
+}
+
 // ----------------------------------------------------------------- fine
 int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate) {
   cudaStream_t s = c->stream;
@@ -844,14 +893,14 @@ void cube_fine_stats(const cube_ctx* c, cube_stats* st) {
   st->testrhof = std::ldexp((double)c->hstats->rhof_fix, -dep_shift(c->p.mass_p));
 }
 
-int cube_fine_forces_impl(cube_ctx* c, cube_stats* st, const float* pre) {
+int cube_fine_forces_impl(cube_ctx* c, cube_stats* st) {
   int r0 = cube_fine_density_impl(c, nullptr, false);
   if (r0) return r0;
-  return cube_fine_spectral_impl(c, st, pre);
+  return cube_fine_spectral_impl(c, st);
 }
 
 // forces from the density on the fine mesh (pm.f90:112-126)
-int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
+int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st) {
   cudaStream_t s = c->stream;
   int64_t nfh = c->nf / 2 + 1;
   int64_t nspec = nfh * c->nf * (int64_t)c->nf;
@@ -860,17 +909,15 @@ int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
   cube_phase_end(c, PH_F_R2C);
   cube_phase_begin(c, PH_F_GREEN);
   k_green3<<<cube_grid(nspec, 256), 256, 0, s>>>((const float2*)c->rho_f, c->kern_f, nspec, (float2*)c->force_f[0],
-                                                  (float2*)c->force_f[1], (float2*)c->force_f[2]);
+                                                  (float2*)c->force_f[1], (float2*)c->force_f[2], c->f2_kick);
   cube_phase_end(c, PH_F_GREEN);
   cube_phase_begin(c, PH_F_C2R);
   for (int d = 0; d < 3; d += c->f_c2r_batch)
     CUBE_FFT(c, cufftExecC2R(c->plan_f_c2r, (cufftComplex*)c->force_f[d], c->force_f[d]));
   cube_phase_end(c, PH_F_C2R);
   cube_phase_begin(c, PH_F_F2MAX);
-  if (pre)
-    launch_f2max<true>(c, c->force_f, c->nf, &c->dstats->f2_fine_bits, pre);
-  else
-    launch_f2max<false>(c, c->force_f, c->nf, &c->dstats->f2_fine_bits, nullptr);
+  launch_f2max(c, c->force_f, c->nf, &c->dstats->f2_fine_bits, c->f2_kick);
+  (c->owner ? c->owner : c)->force_pre[0].on = false;
   cube_phase_end(c, PH_F_F2MAX);
   CUBE_CUDA(c, cudaGetLastError());
   if (st) {
@@ -881,7 +928,7 @@ int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
   return CUBE_OK;
 }
 
-int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool pre, bool with_pp) {
+int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool with_pp) {
   KickArgs k{};
   if (with_pp) {  // the PP kick of cube_pp_launch(.., defer_kick), applied here
     if (c->graph_mode || !c->fpp) return cube_fail(c, CUBE_ERR_ARG, "PP kick in the fine kick: eager mode with PP only");
@@ -911,6 +958,7 @@ int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool pre, bool with_
   k.cstart = c->cstart[c->cur];
   k.vfield = c->vfield[c->cur];
   for (int d = 0; d < 3; d++) k.f[d] = c->force_f[d];
+  k.f2 = c->f2_kick;
   k.a_mid = a_mid;
   k.dt = dt;
   k.vmax_bits = nullptr;
@@ -921,10 +969,7 @@ int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool pre, bool with_
   if (!c->graph_mode && c->vmax_prev[0] == 0.f && c->vmax_prev[1] == 0.f && c->vmax_prev[2] == 0.f)
     k.vmax_est = c->dstats->vmax_est_bits;
   cube_phase_begin(c, PH_F_KICK);
-  if (pre)
-    k_kick<true, true><<<cube_grid(c->np, 256), 256, 0, c->stream>>>(k);
-  else
-    k_kick<true, false><<<cube_grid(c->np, 256), 256, 0, c->stream>>>(k);
+  launch_kick<true>(c, k);
   cube_phase_end(c, PH_F_KICK);
   CUBE_CUDA(c, cudaGetLastError());
   return CUBE_OK;
@@ -966,14 +1011,14 @@ int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate, bool 
   return CUBE_OK;
 }
 
-int cube_coarse_forces_impl(cube_ctx* c, cube_stats* st, const float* pre, bool fresh) {
+int cube_coarse_forces_impl(cube_ctx* c, cube_stats* st, bool fresh) {
   int r0 = cube_coarse_density_impl(c, nullptr, false, fresh);
   if (r0) return r0;
-  return cube_coarse_spectral_impl(c, st, pre);
+  return cube_coarse_spectral_impl(c, st);
 }
 
 // forces from the density on the coarse mesh (pm.f90:275-315)
-int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
+int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st) {
   cudaStream_t s = c->stream;
   int nc = c->p.nc;
   int64_t nch = nc / 2 + 1;
@@ -981,13 +1026,11 @@ int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
   cube_phase_begin(c, PH_C_FFT);
   CUBE_FFT(c, cufftExecR2C(c->plan_c_r2c, c->rho_c, (cufftComplex*)c->rho_c));
   k_green3<<<cube_grid(cspec, 256), 256, 0, s>>>((const float2*)c->rho_c, c->kern_c, cspec, (float2*)c->force_c[0],
-                                                  (float2*)c->force_c[1], (float2*)c->force_c[2]);
+                                                  (float2*)c->force_c[1], (float2*)c->force_c[2], c->f2_kick + 1);
   for (int d = 0; d < 3; d += c->c_c2r_batch)
     CUBE_FFT(c, cufftExecC2R(c->plan_c_c2r, (cufftComplex*)c->force_c[d], c->force_c[d]));
-  if (pre)
-    launch_f2max<true>(c, c->force_c, nc, &c->dstats->f2_coarse_bits, pre);
-  else
-    launch_f2max<false>(c, c->force_c, nc, &c->dstats->f2_coarse_bits, nullptr);
+  launch_f2max(c, c->force_c, nc, &c->dstats->f2_coarse_bits, c->f2_kick + 1);
+  (c->owner ? c->owner : c)->force_pre[1].on = false;
   cube_phase_end(c, PH_C_FFT);
   CUBE_CUDA(c, cudaGetLastError());
   if (st) {
@@ -999,7 +1042,7 @@ int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st, const float* pre) {
   return CUBE_OK;
 }
 
-int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool pre, bool fresh) {
+int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bool fresh) {
   KickArgs k{};
   int r;
   if (c->graph_mode) {  // sigma_vi is now sigma_vi_new for both
@@ -1022,6 +1065,7 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
   k.vp_out = c->vp[alt];  // the input codes stay intact for an exact vmax rerun
   k.pcell = c->pcell[cur];
   k.vfield = c->vfield[cur];
+  k.f2 = c->f2_kick + 1;
   for (int d = 0; d < 3; d++) {
     k.f[d] = c->force_c[d];
     // velocities change little per step: every lane that could reach 0.95 of
@@ -1056,10 +1100,7 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
       kp.vp_in = (const char*)k.vp_in + bv * p0;
       kp.vp_out = (char*)k.vp_out + bv * p0;
       kp.pcell = k.pcell + p0;
-      if (pre)
-        k_kick<false, true><<<cube_grid(kp.np, 256), 256, 0, c->stream>>>(kp);
-      else
-        k_kick<false, false><<<cube_grid(kp.np, 256), 256, 0, c->stream>>>(kp);
+      launch_kick<false>(c, kp);
       CUBE_CUDA(c, cudaEventRecord(c->ev_copy_start, c->stream));
       CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_copy, c->ev_copy_start, 0));
       CUBE_CUDA(c, cudaMemcpyAsync((char*)c->vp_host + bv * p0, kp.vp_out, bv * (p1 - p0), cudaMemcpyDeviceToHost,
@@ -1068,20 +1109,14 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
     CUBE_CUDA(c, cudaEventRecord(c->ev_copy, c->stream_copy));
     c->copy_pending = true;
     c->vp_host = nullptr;
-  } else if (pre)
-    k_kick<false, true><<<cube_grid(c->np, 256), 256, 0, c->stream>>>(k);
-  else
-    k_kick<false, false><<<cube_grid(c->np, 256), 256, 0, c->stream>>>(k);
+  } else launch_kick<false>(c, k);
   cube_phase_end(c, PH_C_KICK);
   CUBE_CUDA(c, cudaGetLastError());
   if (c->graph_mode) {
     // the exact rerun decides on the device whether it runs; the stats of the
     // whole particle_mesh go to the host's copy
     k.vmax_only = 1;
-    if (pre)
-      k_kick<false, true><<<cube_grid(c->np, 256), 256, 0, c->stream>>>(k);
-    else
-      k_kick<false, false><<<cube_grid(c->np, 256), 256, 0, c->stream>>>(k);
+    launch_kick<false>(c, k);
     CUBE_CUDA(c, cudaGetLastError());
     CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->coarse, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, c->stream));
     void* t = c->vp[cur];
@@ -1102,10 +1137,7 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
   if (rerun) {
     CUBE_CUDA(c, cudaMemsetAsync(c->dstats->vmax_bits, 0, 12, c->stream));
     k.vmax_only = 1;
-    if (pre)
-      k_kick<false, true><<<cube_grid(c->np, 256), 256, 0, c->stream>>>(k);
-    else
-      k_kick<false, false><<<cube_grid(c->np, 256), 256, 0, c->stream>>>(k);
+    launch_kick<false>(c, k);
     CUBE_CUDA(c, cudaGetLastError());
     r = cube_stats_fetch(c);
     if (r) return r;
