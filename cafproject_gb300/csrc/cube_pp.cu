@@ -243,16 +243,13 @@ __global__ void __launch_bounds__(256) k_pp_kick_idle(PPArgs a) {
 
 __device__ __forceinline__ void pp_reduce(const PPArgs& a, unsigned long long npairs, unsigned long long nwork,
                                           float f2max) {
-  for (int o = 16; o > 0; o >>= 1) {
-    npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
-    nwork += __shfl_xor_sync(0xffffffffu, nwork, o);
-    f2max = fmaxf(f2max, __shfl_xor_sync(0xffffffffu, f2max, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&a.st->npairs, npairs);
-    atomicAdd(&a.st->itest1, nwork);
-    atomic_max_pos(&a.st->f2_pp_bits, f2max);
-  }
+  __shared__ unsigned s_f2;
+  if (threadIdx.x == 0) s_f2 = 0u;
+  block_count({&a.st->npairs, &a.st->itest1}, {npairs, nwork});  // a barrier, at least
+  if (!__syncthreads_or(f2max > 0.f)) return;
+  warp_max_pos(&s_f2, f2max);
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(&a.st->f2_pp_bits, s_f2);
 }
 
 struct PPSmem {
@@ -879,18 +876,8 @@ __global__ void __launch_bounds__(256) k_pp_nbmask(PPFilter f) {
       }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    nact += __shfl_xor_sync(0xffffffffu, nact, o);
-    nidle += __shfl_xor_sync(0xffffffffu, nidle, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    // a particle left out has the one entry of itself and a zero force (itest1 counts it)
-    if (nidle) {
-      atomicAdd(&f.st->npairs, nidle);
-      atomicAdd(&f.st->itest1, nidle);
-    }
-    if (nact) atomicAdd(&f.st->pp_active, nact);
-  }
+  // a particle left out has the one entry of itself and a zero force (itest1 counts it)
+  block_count({&f.st->npairs, &f.st->itest1, &f.st->pp_active}, {nidle, nidle, nact});
 }
 
 // active particles before storage position q

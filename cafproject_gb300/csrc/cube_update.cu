@@ -231,6 +231,9 @@ __global__ void __launch_bounds__(256, 4) k_dest(UpdArgs a) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const float xres = g.izipx == 1 ? 1.0f / 256.0f : 1.0f / 65536.0f;
   const float dt = dtm(a), adt = fabsf(dt) * 1.2e-7f;
+  __shared__ unsigned s_disp;
+  if (threadIdx.x == 0) s_disp = 0u;
+  __syncthreads();
   int local_max = 0;
   for (int64_t p = a.p_lo + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.np; p += stride) {
     const int32_t cell = a.pcell[p];
@@ -277,8 +280,9 @@ __global__ void __launch_bounds__(256, 4) k_dest(UpdArgs a) {
     }
   }
   // block max of the displacement
-  for (int o = 16; o > 0; o >>= 1) local_max = max(local_max, __shfl_xor_sync(0xffffffffu, local_max, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(&a.st->max_disp, local_max);
+  warp_max_pos(&s_disp, __uint_as_float((unsigned)local_max));  // the bits of an integer >= 0 order as it does
+  __syncthreads();
+  if (threadIdx.x == 0 && s_disp) atomicMax(&a.st->max_disp, (int)s_disp);
 }
 
 // vfield_new = vfield_new + vreal (update_particle.f90:72): the real(8) sum
