@@ -800,7 +800,12 @@ __device__ __forceinline__ unsigned write_particle_at(const UpdArgs& a, int64_t 
 // need it, so nearly every warp would run it, mostly idle, at each of them
 // (k_scatter of 512^3 particles: 4.05 -> 3.17 ms with the queue and the
 // table-free test together).  An entry holds the particle and its new index (31 bits
-// each: the permutation is int32) and the component.
+// each: the permutation is int32) and the component.  A warp ends with a
+// part-filled queue, so the kernels that keep one take the blocks that fit at
+// once (MOVE_BLOCKS an SM) and no more: with 16 an SM k_scatter took 411 us for
+// 256^3 late particles, 201 for 208^3, 38 for 108^3 and 3.21 ms for 512^3;
+// with 6, 387, 193, 33 and 3.03.
+constexpr int MOVE_BLOCKS = 6;
 constexpr int SC_Q = 128;  // entries per warp: at most 31 pending + 96 of one pass
 struct RecodeQueue {
   unsigned long long* q;
@@ -951,7 +956,7 @@ __global__ void __launch_bounds__(256) k_sort_gather(UpdArgs a, const uint64_t* 
 }
 
 // U3: scatter every primary copy to its place in the new disjoint order.
-__global__ void __launch_bounds__(256, 6) k_scatter(UpdArgs a) {
+__global__ void __launch_bounds__(256, MOVE_BLOCKS) k_scatter(UpdArgs a) {
   if (!a.sd && queued_in_vain(a)) return;  // (a captured step's walker has set the ranks instead)
   __shared__ unsigned long long s_q[8][SC_Q];
   RecodeQueue rq{s_q[threadIdx.x >> 5], 0};
@@ -1177,10 +1182,10 @@ static int update_x_graph(cube_ctx* c) {
   CUBE_CUDA(c, cudaGetLastError());
   int r = cube_scan_counts(c, c->rhoc[kn], c->cstart[kn], c->ncells);
   if (r) return r;
-  k_rank_place<<<cube_grid(c->np, B), B, 0, s>>>(a);
+  k_rank_place<<<cube_grid(c->np, B, 8), B, 0, s>>>(a);
   k_vfield_new<<<cube_grid(c->ncells, 128, 32), 128, 0, s>>>(a);
   k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 6), VF_BLOCK, 0, s>>>(a);
-  k_scatter<<<cube_grid(c->np, B), B, 0, s>>>(a);
+  k_scatter<<<cube_grid(c->np, B, MOVE_BLOCKS), B, 0, s>>>(a);
   k_scatter_xtra<<<cube_grid(c->xtra_cap, B, 2), B, 0, s>>>(a);
   CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->upd, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, s));
   // sigma_vi_new and its codec tables beside the densities and transforms: the
@@ -1323,12 +1328,12 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
     CUBE_CUDA(c, cudaGetLastError());
     if ((r = scan_only())) return r;
     cube_phase_begin(c, PH_UPD_PLACE);
-    k_rank_place<<<cube_grid(c->np, B), B, 0, c->stream>>>(a);
+    k_rank_place<<<cube_grid(c->np, B, 8), B, 0, c->stream>>>(a);
     if ((r = means())) return r;
     cube_phase_end(c, PH_UPD_PLACE);
     if ((r = cube_pid_join(c))) return r;  // a deferred pid upload lands before the scatter reads it
     cube_phase_begin(c, PH_UPD_SCATTER);
-    k_scatter<<<cube_grid(c->np, B), B, 0, c->stream>>>(a);
+    k_scatter<<<cube_grid(c->np, B, MOVE_BLOCKS), B, 0, c->stream>>>(a);
     cube_phase_end(c, PH_UPD_SCATTER);
     CUBE_CUDA(c, cudaGetLastError());
     if ((r = sigma(c->np))) return r;
@@ -1388,9 +1393,9 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
     if ((r = cube_pid_join(c))) return r;
     cube_phase_begin(c, PH_UPD_SCATTER);
     if (skeys) {
-      k_sort_gather<<<cube_grid(np_new, B), B, 0, c->stream>>>(a, skeys, np_new, 64 - db);
+      k_sort_gather<<<cube_grid(np_new, B, MOVE_BLOCKS), B, 0, c->stream>>>(a, skeys, np_new, 64 - db);
     } else {
-      k_scatter<<<cube_grid(c->np, B), B, 0, c->stream>>>(a);
+      k_scatter<<<cube_grid(c->np, B, MOVE_BLOCKS), B, 0, c->stream>>>(a);
       if (hs.ndup_list) k_scatter_xtra<<<cube_grid((int64_t)hs.ndup_list, B), B, 0, c->stream>>>(a);
     }
     cube_phase_end(c, PH_UPD_SCATTER);
