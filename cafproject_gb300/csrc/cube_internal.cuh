@@ -79,7 +79,7 @@ struct StepDev {
 };
 // what the host reads back after a graph step: the stats of each stage
 struct StepOut {
-  DevStats upd, pp, fine, coarse;
+  DevStats upd, pp, coarse;  // coarse: the fine and the coarse stages'
   double sums[3];  // sigma statistics (update_particle.f90:171-224)
   float sigma_new;
   int pad;

@@ -872,7 +872,7 @@ int cube_force_settle(cube_ctx* c, int coarse) {
 int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate) {
   cudaStream_t s = c->stream;
   Geo g = make_geo(c);
-  CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), s));
+  if (!c->graph_mode) CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), s));  // (zeroed at the step's head)
   const int sh = dep_shift(c->p.mass_p);
   DepArgs a{g, c->xp[c->cur], c->rhoc[c->cur], c->cstart[c->cur], c->p.mass_p, c->rho_f, &c->dstats->rhof_fix, 0, 0.f,
             std::ldexp(1.0f, sh), std::ldexp(1.0f, -sh), accumulate ? 1 : 0};
@@ -1113,12 +1113,10 @@ int cube_coarse_kick_impl(cube_ctx* c, float a_mid, float dt, cube_stats* st, bo
   cube_phase_end(c, PH_C_KICK);
   CUBE_CUDA(c, cudaGetLastError());
   if (c->graph_mode) {
-    // the exact rerun decides on the device whether it runs; the stats of the
-    // whole particle_mesh go to the host's copy
+    // the exact rerun decides on the device whether it runs
     k.vmax_only = 1;
     launch_kick<false>(c, k);
     CUBE_CUDA(c, cudaGetLastError());
-    CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->coarse, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, c->stream));
     void* t = c->vp[cur];
     c->vp[cur] = c->vp[alt];
     c->vp[alt] = t;

@@ -192,26 +192,31 @@ __device__ __forceinline__ float pp_store_force(const PPArgs& a, int64_t p, cons
 }
 
 // kick + exact velocity code of every particle, in storage order (coalesced
-// code and force accesses; the pair kernels visit particles in staging order)
+// code and force accesses; the pair kernels visit particles in staging order).
+// A particle the prefilter left out has a zero pair force (fpp not written):
+// each code becomes the code of its own decoded value, from the codec's table
 __global__ void __launch_bounds__(256) k_pp_kick(PPArgs a) {
   const Geo& g = a.g;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.np; p += (int64_t)gridDim.x * blockDim.x) {
     float F[3];
     int code[3];
-    // a particle the prefilter left out has a zero pair force (fpp not written)
-    const bool on = !a.act || ((__ldg(a.act + (p >> 5)) >> (p & 31)) & 1u);
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-      F[d] = on ? a.fpp[3 * p + d] : 0.f;
-      code[d] = load_code(a.vp, 3 * p + d, g.izipv);
+    for (int d = 0; d < 3; d++) code[d] = load_code(a.vp, 3 * p + d, g.izipv);
+    if (a.act && !((__ldg(a.act + (p >> 5)) >> (p & 31)) & 1u)) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) code[d] = __ldg(a.cv.rt + code[d] + a.cv.half);
+    } else {
+#pragma unroll
+      for (int d = 0; d < 3; d++) F[d] = a.fpp[3 * p + d];
+      pp_kick3(a.cv, code, F, pp_kick_f(a), pp_kick_d(a), a.exact_only);
     }
-    pp_kick3(a.cv, code, F, pp_kick_f(a), pp_kick_d(a), a.exact_only);
 #pragma unroll
     for (int d = 0; d < 3; d++) store_code(a.vp, 3 * p + d, g.izipv, code[d]);
   }
 }
 
-// With the prefilter: the kick of the active particles (the list pidx) ...
+// With the prefilter, the others left to the fine kick: the kick of the active
+// particles (the list pidx)
 __global__ void __launch_bounds__(256) k_pp_kick_active(PPArgs a) {
   const Geo& g = a.g;
   const int64_t n = __ldg(a.nact);
@@ -227,17 +232,6 @@ __global__ void __launch_bounds__(256) k_pp_kick_active(PPArgs a) {
     pp_kick3(a.cv, code, F, pp_kick_f(a), pp_kick_d(a), a.exact_only);
 #pragma unroll
     for (int d = 0; d < 3; d++) store_code(a.vp, 3 * p + d, g.izipv, code[d]);
-  }
-}
-// ... and of the others: a zero force, so each code becomes the code of its
-// own decoded value (the codec's zero-kick table)
-__global__ void __launch_bounds__(256) k_pp_kick_idle(PPArgs a) {
-  const Geo& g = a.g;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.np; p += (int64_t)gridDim.x * blockDim.x) {
-    if ((__ldg(a.act + (p >> 5)) >> (p & 31)) & 1u) continue;
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-      store_code(a.vp, 3 * p + d, g.izipv, __ldg(a.cv.rt + load_code(a.vp, 3 * p + d, g.izipv) + a.cv.half));
   }
 }
 
@@ -929,7 +923,7 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
     r = cube_codec_pair(c, c->sigma_vi, c->sigma_vi, &a.cv, nullptr);
     if (r) return r;
   }
-  CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), c->stream));
+  if (!c->graph_mode) CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), c->stream));
   a.g = make_geo(c);
   a.np = c->np;
   a.xp = c->xp[c->cur];
@@ -1025,20 +1019,12 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
   const int g4 = (int)std::max<int64_t>(1, std::min<int64_t>(one_per_sm, c->pp_scr_cap / (2 * PP_CAP1)));
   if (start <= 4) k_pp_global<4><<<g4, PP_THREADS1, 0, c->stream>>>(a);
   k_pp_global<5><<<1, PP_THREADS1, 0, c->stream>>>(a);
-  if (c->pp_act_valid) {
-    // the active particles' kick now (a deferred fine kick then gives the
-    // others their zero-kick codes); the others' here when not deferred
-    k_pp_kick_active<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(a);
-    if (!defer_kick) k_pp_kick_idle<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(a);
-  } else if (!defer_kick) {
+  if (!defer_kick)
     k_pp_kick<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(a);
-  }
+  else if (c->pp_act_valid)  // the fine kick gives the others their zero-kick codes
+    k_pp_kick_active<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(a);
   CUBE_CUDA(c, cudaGetLastError());
   cube_phase_end(c, PH_PP);
-  if (c->graph_mode) {
-    CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->pp, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, c->stream));
-    return CUBE_OK;
-  }
   return CUBE_OK;
 }
 

@@ -24,6 +24,7 @@ namespace {
 
 constexpr double kWeightV = (double)0.1f;  // real(8),parameter :: weight_v=0.1 (a real(4) literal)
 
+constexpr int NOFF = 27;  // the counting path: a cell's neighbours and itself
 struct UpdArgs {
   Geo g;
   int64_t np, ncells;
@@ -59,6 +60,8 @@ struct UpdArgs {
   int32_t* vdense;    // destination cells over vf_dense particles, for k_vfield_dense
   uint32_t vf_dense;
   int64_t p_lo;       // k_dest: first particle of this launch (particles [p_lo, np))
+  int zero_offc;      // k_dest: clear offc for the counting path
+  int xtra_too;       // k_scatter: the extra copies as well (captured step)
   int spec;           // counting path queued ahead of the check that it applies
   int rank_init;      // k_dest: set every rank to the "no rank" sentinel (for the walker)
 };
@@ -234,6 +237,11 @@ __global__ void __launch_bounds__(256, 4) k_dest(UpdArgs a) {
   __shared__ unsigned s_disp;
   if (threadIdx.x == 0) s_disp = 0u;
   __syncthreads();
+  if (a.zero_offc) {  // 54 bytes a cell; stores beside the particles' work instead of a launch
+    const int64_t n = NOFF * a.ncells, t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    for (int64_t i = t; i < n / 8; i += stride) reinterpret_cast<uint4*>(a.offc)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (t < n % 8) a.offc[n - 1 - t] = 0;
+  }
   int local_max = 0;
   for (int64_t p = a.p_lo + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.np; p += stride) {
     const int32_t cell = a.pcell[p];
@@ -329,7 +337,6 @@ __device__ __forceinline__ float vfield_quotient(float acc, uint32_t cnt, int ex
 // base ranks in place; after the scan, rank = base + local rank and the
 // inverse permutation; per destination, vfield_new summed in rank order, i.e.
 // the reference's visit order.
-constexpr int NOFF = 27;
 
 // one thread per particle: its rank among the earlier particles of its cell
 // bound for the same neighbour (storage order); the last of them also writes
@@ -955,6 +962,24 @@ __global__ void __launch_bounds__(256) k_sort_gather(UpdArgs a, const uint64_t* 
   recode_rest(a, rq);
 }
 
+// U3: the extra copies of the list to theirs
+__device__ __noinline__ void scatter_xtra(const UpdArgs& a) {
+  int64_t nx = (int64_t)(a.st->ndup_list < (unsigned long long)a.xtra_cap ? a.st->ndup_list : (unsigned long long)a.xtra_cap);
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nx; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t p = a.xtra[e].x;
+    const int32_t D = a.xtra[e].y;
+    const uint32_t r = (uint32_t)a.xtra[e].z;
+    if (!rank_ok(a, D, r)) continue;
+    const int64_t idx = a.cstart_new[D] + r;
+    const unsigned open = write_particle_at(a, p, D, idx);
+    for (int d = 0; d < 3; d++)
+      if ((open >> d) & 1u)
+        store_code_i(a.vp_new, 3 * idx + d, a.g.izipv,
+                     recode_exact(a, load_code(a.vp, 3 * p + d, a.g.izipv), a.vfield[3 * (int64_t)a.pcell[p] + d],
+                                  a.vfield_new[3 * (int64_t)D + d]));
+  }
+}
+
 // U3: scatter every primary copy to its place in the new disjoint order.
 __global__ void __launch_bounds__(256, MOVE_BLOCKS) k_scatter(UpdArgs a) {
   if (!a.sd && queued_in_vain(a)) return;  // (a captured step's walker has set the ranks instead)
@@ -976,24 +1001,10 @@ __global__ void __launch_bounds__(256, MOVE_BLOCKS) k_scatter(UpdArgs a) {
     recode_push(a, rq, open, p, idx);
   }
   recode_rest(a, rq);
+  if (a.xtra_too) scatter_xtra(a);
 }
 
-__global__ void k_scatter_xtra(UpdArgs a) {
-  int64_t nx = (int64_t)(a.st->ndup_list < (unsigned long long)a.xtra_cap ? a.st->ndup_list : (unsigned long long)a.xtra_cap);
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nx; e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t p = a.xtra[e].x;
-    const int32_t D = a.xtra[e].y;
-    const uint32_t r = (uint32_t)a.xtra[e].z;
-    if (!rank_ok(a, D, r)) continue;
-    const int64_t idx = a.cstart_new[D] + r;
-    const unsigned open = write_particle_at(a, p, D, idx);
-    for (int d = 0; d < 3; d++)
-      if ((open >> d) & 1u)
-        store_code_i(a.vp_new, 3 * idx + d, a.g.izipv,
-                     recode_exact(a, load_code(a.vp, 3 * p + d, a.g.izipv), a.vfield[3 * (int64_t)a.pcell[p] + d],
-                                  a.vfield_new[3 * (int64_t)D + d]));
-  }
-}
+__global__ void k_scatter_xtra(UpdArgs a) { scatter_xtra(a); }
 
 __device__ __forceinline__ void ff_add(float& hi, float& lo, float x, float xlo) {
   float s, e;
@@ -1134,7 +1145,6 @@ static int update_x_graph(cube_ctx* c) {
   int k = c->cur, kn = 1 - k;
   CodecView cv;
   cube_codec_view_dev(c, c->graph_slot, &c->sd->h.cf_vi, &cv);
-  CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), c->stream));
   UpdArgs a{};
   a.g = g;
   a.np = c->np;
@@ -1172,9 +1182,10 @@ static int update_x_graph(cube_ctx* c) {
   const int B = 256;
   cudaStream_t s = c->stream;
   a.rank_init = 1;
+  a.zero_offc = 1;
+  a.xtra_too = 1;
   a.spec = 1;
   k_dest<<<cube_grid(c->np, B), B, 0, s>>>(a);
-  CUBE_CUDA(c, cudaMemsetAsync(c->offc, 0, sizeof(uint16_t) * NOFF * (size_t)c->ncells, s));
   k_rank_local<<<cube_grid(c->np, 256), 256, 0, s>>>(a);
   k_rank_dense<<<cube_grid((int64_t)1 << 40, 1, 4), RD_THREADS, 0, s>>>(a);
   k_rank_base<<<cube_grid(c->ncells, 256), 256, 0, s>>>(a);
@@ -1186,8 +1197,6 @@ static int update_x_graph(cube_ctx* c) {
   k_vfield_new<<<cube_grid(c->ncells, 128, 32), 128, 0, s>>>(a);
   k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 6), VF_BLOCK, 0, s>>>(a);
   k_scatter<<<cube_grid(c->np, B, MOVE_BLOCKS), B, 0, s>>>(a);
-  k_scatter_xtra<<<cube_grid(c->xtra_cap, B, 2), B, 0, s>>>(a);
-  CUBE_CUDA(c, cudaMemcpyAsync(&c->sout->upd, c->dstats, sizeof(DevStats), cudaMemcpyDeviceToDevice, s));
   // sigma_vi_new and its codec tables beside the densities and transforms: the
   // fine kick is the first to need them (it waits for ev_codec)
   CUBE_CUDA(c, cudaEventRecord(c->ev_aux, s));
@@ -1255,6 +1264,7 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   a.vdense = c->vdense;
   a.vf_dense = vf_dense(c, c->np);
   const int B = 256;
+  a.zero_offc = c->opt_rank_walk == 0;
   cube_phase_begin(c, PH_UPD_DEST);
   if (c->xv_pending && c->up_np == c->np) {
     // a pending cube_upload_begin: take xp and vp piece by piece as they land
@@ -1262,8 +1272,9 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
       UpdArgs ap = a;
       ap.p_lo = c->np * i / c->up_pieces;
       ap.np = c->np * (i + 1) / c->up_pieces;
+      ap.zero_offc = a.zero_offc && i == 0;
       CUBE_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_xv[i], 0));
-      if (ap.np > ap.p_lo) k_dest<<<cube_grid(ap.np - ap.p_lo, B), B, 0, c->stream>>>(ap);
+      if (ap.np > ap.p_lo || ap.zero_offc) k_dest<<<cube_grid(ap.np - ap.p_lo, B), B, 0, c->stream>>>(ap);
     }
     c->xv_pending = false;  // pid (the last piece) is joined before the scatter
   } else {
@@ -1320,7 +1331,6 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
     // particle is lost to a second frame and the new count is at most the old)
     a.spec = 1;
     cube_phase_begin(c, PH_UPD_RANK);
-    CUBE_CUDA(c, cudaMemsetAsync(c->offc, 0, sizeof(uint16_t) * NOFF * (size_t)c->ncells, c->stream));
     k_rank_local<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(a);
     k_rank_dense<<<cube_grid((int64_t)1 << 40, 1, 4), RD_THREADS, 0, c->stream>>>(a);
     k_rank_base<<<cube_grid(c->ncells, 256), 256, 0, c->stream>>>(a);
