@@ -47,7 +47,7 @@ struct DevStats {
   unsigned long long pp_active;           // PP prefilter: particles with a neighbour besides themselves
   double sums[3];                         // update_x: the sigma_v sums (update_particle.f90:172-196)
   long long np_new;                       // update_x: particles of the new state
-  int pp_nlist[11];  // PP: lengths of the levels' lists (5), then each level's next-item counter (6)
+  int pp_nlist[12];  // PP: lengths of the levels' lists (5), each level's next-item counter (6), level 4's blocks done
 };
 
 // share of the last step's vmax above which the coarse kick evaluates a

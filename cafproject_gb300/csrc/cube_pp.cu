@@ -89,7 +89,7 @@ struct PPArgs {
   int nb;        // bricks per dimension
   int* list[5];    // work of levels 1..5: bricks, bricks, cells, cells, cells
   int* lpart[5];   // per listed item: parts (low 8 bits), parts claimed (above)
-  int* nlist;      // their lengths (5), then each level's next-item counter (6)
+  int* nlist;      // their lengths (5), then each level's next-item counter (6) and level 4's blocks done
   float4* scr_pts;     // global staging of levels 4-5 (scr_cap entries each)
   unsigned* scr_kinfo;
   unsigned* scr_order;
@@ -685,12 +685,9 @@ __global__ void __launch_bounds__(NT, NT <= 128 ? 8 : (NT <= 256 ? 4 : 1)) k_pp_
 // hold is counted as an overflow and its particles keep no PP force (the
 // call reports it).
 template <int kLevel>
-__global__ void __launch_bounds__(PP_THREADS1) k_pp_global(PPArgs a) {
-  __shared__ PPSmem sm;
-  __shared__ unsigned bins[PNF1 + 2];
-  __shared__ int s3[3];
+__device__ void pp_scratch_level(const PPArgs& a, PPSmem& sm, unsigned* bins, int* s3, PPAcc& acc) {
   const Geo& g = a.g;
-  const int n = a.nlist[kLevel - 1];
+  const int n = *(volatile int*)&a.nlist[kLevel - 1];
   const int64_t share = kLevel == 4 ? a.scr_cap / gridDim.x : a.scr_cap;
   const int64_t off = kLevel == 4 ? share * blockIdx.x : 0;
   PPBuf<unsigned, 8> buf;
@@ -699,7 +696,6 @@ __global__ void __launch_bounds__(PP_THREADS1) k_pp_global(PPArgs a) {
   buf.order = a.scr_order + off;
   buf.bins = bins;
   buf.cap = (int)share;
-  PPAcc acc;
   int it, part, np;
   while (pp_next_part(a.nlist + 5 + kLevel, n, a.lpart[kLevel - 1], s3, it, part, np)) {
     const int item = a.list[kLevel - 1][it];
@@ -714,6 +710,24 @@ __global__ void __launch_bounds__(PP_THREADS1) k_pp_global(PPArgs a) {
       __syncthreads();
     }
   }
+}
+// (the block that ends level 4 last takes level 5: a launch less)
+__global__ void __launch_bounds__(PP_THREADS1) k_pp_global(PPArgs a) {
+  __shared__ PPSmem sm;
+  __shared__ unsigned bins[PNF1 + 2];
+  __shared__ int s3[3];
+  PPAcc acc;
+  pp_scratch_level<4>(a, sm, bins, s3, acc);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s3[0] = atomicAdd(&a.nlist[11], 1) == (int)gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  const bool last = s3[0] != 0;
+  __syncthreads();
+  if (last) pp_scratch_level<5>(a, sm, bins, s3, acc);
   pp_reduce(a, acc.npairs, acc.nwork, acc.f2max);
 }
 
@@ -881,20 +895,19 @@ __device__ __forceinline__ int64_t act_prefix(const PPFilter& f, int64_t q) {
   return r == 0 ? __ldg(f.wstart + w) : __ldg(f.wstart + w) + __popc(__ldg(f.act + w) & ((1u << r) - 1u));
 }
 
-__global__ void __launch_bounds__(256) k_pp_acells(PPFilter f) {
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < f.ncells; c += (int64_t)gridDim.x * blockDim.x) {
+// the active particles' list, and each cell's part of it
+__global__ void __launch_bounds__(256) k_pp_alists(PPFilter f) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t p = t; p < f.np; p += stride) {
+    const unsigned w = __ldg(f.act + (p >> 5));
+    const int r = (int)(p & 31);
+    if ((w >> r) & 1u) f.aidx[__ldg(f.wstart + (p >> 5)) + __popc(w & ((1u << r) - 1u))] = (int32_t)p;
+  }
+  for (int64_t c = t; c < f.ncells; c += stride) {
     const int64_t s0 = __ldg(f.cstart + c);
     const int64_t a0 = act_prefix(f, s0);
     f.acstart[c] = a0;
     f.arhoc[c] = (int32_t)(act_prefix(f, s0 + __ldg(f.rhoc + c)) - a0);
-  }
-}
-
-__global__ void __launch_bounds__(256) k_pp_aidx(PPFilter f) {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < f.np; p += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned w = __ldg(f.act + (p >> 5));
-    const int r = (int)(p & 31);
-    if ((w >> r) & 1u) f.aidx[__ldg(f.wstart + (p >> 5)) + __popc(w & ((1u << r) - 1u))] = (int32_t)p;
   }
 }
 
@@ -985,11 +998,10 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
     if (c->np > 0) {
       r = cube_scan_counts(c, c->pp_wcnt, c->pp_wstart, nw);
       if (r) return r;
-      k_pp_aidx<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(f);
     } else {
       CUBE_CUDA(c, cudaMemsetAsync(c->pp_wstart, 0, 8, c->stream));
     }
-    k_pp_acells<<<cube_grid(c->ncells, 256), 256, 0, c->stream>>>(f);
+    k_pp_alists<<<cube_grid(std::max(c->np, c->ncells), 256), 256, 0, c->stream>>>(f);
     a.rhoc = c->pp_arhoc;
     a.cstart = c->pp_acstart;
     a.pidx = c->pp_aidx;
@@ -1017,8 +1029,7 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
   if (start <= 3) k3<<<one_per_sm, PP_THREADS1, PP_SMEM1, c->stream>>>(a);
   // level 4: a block per SM, each region at least twice level 3's room
   const int g4 = (int)std::max<int64_t>(1, std::min<int64_t>(one_per_sm, c->pp_scr_cap / (2 * PP_CAP1)));
-  if (start <= 4) k_pp_global<4><<<g4, PP_THREADS1, 0, c->stream>>>(a);
-  k_pp_global<5><<<1, PP_THREADS1, 0, c->stream>>>(a);
+  k_pp_global<<<start <= 4 ? g4 : 1, PP_THREADS1, 0, c->stream>>>(a);
   if (!defer_kick)
     k_pp_kick<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(a);
   else if (c->pp_act_valid)  // the fine kick gives the others their zero-kick codes
