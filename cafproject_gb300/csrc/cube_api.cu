@@ -229,7 +229,7 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
   ALLOC(c->enc_edge, 8 * (c->nvbin / 2));
   for (int k = 0; k < 2; k++) {
     ALLOC(c->codec[k].dec, 8 * c->nvbin);
-    ALLOC(c->codec[k].dech, 8 * c->nvbin);
+    ALLOC(c->codec[k].dech, 8 * (c->nvbin / 2 + 1));
     ALLOC(c->codec[k].bnd, 8 * (c->nvbin / 2 + 1));
     ALLOC(c->codec[k].decf, 4 * (c->nvbin / 2 + 1));
     ALLOC(c->codec[k].rt, 4 * (c->nvbin + 3));

@@ -402,11 +402,8 @@ __global__ void __launch_bounds__(CT_THREADS) k_codec_tables(const float* __rest
     const float lo = __double2float_rn(__dsub_rn(d, (double)hi));
     const bool two = m > 0 && m < half;
     dec[half - m] = d;
-    dech[half - m] = make_float2(hi, lo);
-    if (two) {
-      dec[half + m] = -d;
-      dech[half + m] = make_float2(-hi, __fsub_rn(0.f, lo));  // +0 stays +0
-    }
+    if (two) dec[half + m] = -d;
+    dech[m] = m > 0 ? make_float2(-hi, __fsub_rn(0.f, lo)) : make_float2(0.f, 0.f);
     if (decf) decf[m] = -hi;
     if (m < half) bnd[m] = m > 0 ? v_edge(edge[m], c) : 0;
     if (rt) {

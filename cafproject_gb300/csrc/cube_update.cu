@@ -1031,7 +1031,7 @@ struct SigmaArgs {
   int64_t np, ncells;
   const int64_t* npp;  // when set, the particle count on the device (at most np)
   const float2* dech;
-  int nvbin, izipv;
+  int izipv;
   double* part;      // 3 per block
   unsigned* count;   // blocks done; the last one leaves it at zero
   DevStats* st;      // eager: receives the sums
@@ -1090,7 +1090,7 @@ __global__ void __launch_bounds__(SG_THREADS) k_sigma(SigmaArgs a) {
     int64_t c = a.pcell[p];
     if (c < 0 || c >= ncells) continue;
     for (int d = 0; d < 3; d++) {
-      float2 v = __ldg(a.dech + load_code(a.vp, 3 * p + d, a.izipv) + a.nvbin / 2);
+      const float2 v = decode_ff(a.dech, load_code(a.vp, 3 * p + d, a.izipv));
       float p2 = __fmul_rn(v.x, v.x);
       ff_add(rh, rl, p2, __fmaf_rn(v.x, v.x, -p2) + 2.f * v.x * v.y);
       float w, ew;
@@ -1202,7 +1202,7 @@ static int update_x_graph(cube_ctx* c) {
   CUBE_CUDA(c, cudaEventRecord(c->ev_aux, s));
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_aux, c->ev_aux, 0));
   const double npg = (double)(c->npglobal > 0 ? c->npglobal : c->np);
-  const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, nullptr, cv.dech, c->nvbin,
+  const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], c->np, c->ncells, nullptr, cv.dech,
                      c->p.izipv, c->red_tmp, c->red_count, nullptr, false, npg, c->sd, c->sout};
   k_sigma<<<sigma_blocks(c, c->np), SG_THREADS, 0, c->stream_aux>>>(sg);
   CUBE_CUDA(c, cudaGetLastError());
@@ -1318,7 +1318,7 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   auto sigma = [&](int64_t np_most) -> int {
     cube_phase_begin(c, PH_UPD_SIGMA);
     const SigmaArgs sg{c->vp[kn], c->pcell[kn], c->vfield[kn], np_most, c->ncells, c->cstart[kn] + c->ncells, cv.dech,
-                       c->nvbin, c->p.izipv, c->red_tmp, c->red_count, c->dstats, a.spec != 0, 0.0, nullptr,
+                       c->p.izipv, c->red_tmp, c->red_count, c->dstats, a.spec != 0, 0.0, nullptr,
                        nullptr};
     k_sigma<<<sigma_blocks(c, np_most), SG_THREADS, 0, c->stream>>>(sg);
     cube_phase_end(c, PH_UPD_SIGMA);
