@@ -342,6 +342,11 @@ __device__ __forceinline__ float vfield_quotient(float acc, uint32_t cnt, int ex
 // bound for the same neighbour (storage order); the last of them also writes
 // that neighbour's count (the counts start at zero).  Cells denser than
 // RL_MAX particles are listed for k_rank_dense (a block per cell).
+// A warp holds 32 particles in storage order, so a cell's particles in it find
+// each other by one __match_any_sync over (cell, neighbour), and only those of
+// cells that cross the warp's ends look at the particles beyond them one by one.
+// (Every particle looking at all of its cell's took 289 us for 256^3 late
+// particles, 98 for 208^3 and 21 for 108^3; 139, 64 and 14 this way.)
 constexpr int RL_MAX = 128;
 constexpr int RD_THREADS = 256;
 
@@ -350,25 +355,41 @@ __global__ void k_rank_local(UpdArgs a) {
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&a.st->flags, 8);  // not eligible
     return;
   }
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.np; p += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t S = a.pcell[p];
-    const int64_t p0 = a.cstart[S], p1 = a.cstart[S + 1];
-    if (p1 - p0 > RL_MAX) {  // the cell's first particle lists it
-      if (p == p0) a.vdense[atomicAdd(&a.st->nrank_dense, 1u)] = (int32_t)S;
-      continue;
+  const int lane = threadIdx.x & 31;
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p - lane < a.np;
+       p += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t w0 = p - lane, w1 = w0 + 32;  // the warp's particles
+    int o = 255;
+    int32_t S = 0;
+    int64_t p0 = 0, p1 = 0;
+    if (p < a.np) {
+      S = a.pcell[p];
+      p0 = a.cstart[S];
+      p1 = a.cstart[S + 1];
+      if (p1 - p0 > RL_MAX) {  // the cell's first particle lists it
+        if (p == p0) a.vdense[atomicAdd(&a.st->nrank_dense, 1u)] = S;
+      } else {
+        o = a.doff[p];
+        if (o == 255 && a.dest[p] >= 0) atomicOr(&a.st->flags, 4);  // moved farther than one cell
+      }
     }
-    const int o = a.doff[p];
-    if (o == 255) {
-      if (a.dest[p] >= 0) atomicOr(&a.st->flags, 4);  // moved farther than one cell
-      continue;
-    }
+    // cells ascend in storage order; the first and last of a warp are the only ones
+    // that its ends can cut, and with 27 neighbours the key is the cell's distance
+    // from the warp's first in 26 bits (farther: not matched, looked for one by one)
+    const uint32_t rel = (uint32_t)(S - __shfl_sync(0xffffffffu, S, 0));
+    const bool by_key = o != 255 && rel < (1u << 26);
+    const unsigned key = by_key ? (rel << 5 | (unsigned)o) : (0x80000000u | (unsigned)lane);
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    if (o == 255) continue;
     int r = 0;
     bool last = true;
-    for (int64_t q = p0; q < p1; q++) {
-      if (a.doff[q] != o || q == p) continue;
-      if (q < p) r++;
-      else last = false;
+    const int64_t m0 = by_key ? w0 : p, m1 = by_key ? w1 : p + 1;  // [m0, m1) is matched
+    if (by_key) {
+      r = __popc(peers & ((1u << lane) - 1u));
+      last = (peers >> lane) == 1u;
     }
+    for (int64_t q = p0; q < m0; q++) r += a.doff[q] == o;
+    for (int64_t q = m1; last && q < p1; q++) last = a.doff[q] != o;
     a.lrank[p] = (uint16_t)r;
     if (last) a.offc[o * a.ncells + S] = (uint16_t)(r + 1);
   }
