@@ -203,10 +203,10 @@ def algorithmic_bytes(p, n):
         "fine_r2c": 4 * nf3 + 8 * hf,
         "fine_green": 8 * hf + 12 * hf + 3 * 8 * hf,
         "fine_c2r": 3 * (8 * hf + 4 * nf3),
-        "fine_f2max": 12 * nf3 + 12 * nf3,                 # maxima, then the kick factors written back
+        "fine_f2max": 12 * nf3,
         "fine_kick": n * (3 * p.izipx + 2 * 3 * p.izipv + 4) + 12 * nf3,
         "coarse_deposit": n * (3 * p.izipx + 4) + 4 * nc3,
-        "coarse_fft": (4 * nc3 + 8 * hc) + (8 * hc + 12 * hc + 24 * hc) + 3 * (8 * hc + 4 * nc3) + 24 * nc3,
+        "coarse_fft": (4 * nc3 + 8 * hc) + (8 * hc + 12 * hc + 24 * hc) + 3 * (8 * hc + 4 * nc3) + 12 * nc3,
         "coarse_kick": n * (3 * p.izipx + 2 * 3 * p.izipv + 4 + 12) + 12 * nc3,
     }
 
@@ -426,7 +426,8 @@ def run_gb300(args, ws, rank, lrank):
         cpu = cpu_baseline(p, g.download(), float(g.get_sigma()[0]), ts)
     g.close()
     return dict(value=value, ms=ms_max / args.steps, clocks=clk, phases=phases, roofline=roof, e2e=e2e,
-                cpu=cpu, n=int(ntot), p=p, t_ic=t_ic, gpu_launches=gpu_launches(p, args.steps))
+                cpu=cpu, n=int(ntot), p=p, t_ic=t_ic,
+                gpu_launches=gpu_launches(p, args.steps, conditional=False))
 
 
 def run_adjoint(args, lrank, reps=3):
@@ -632,18 +633,25 @@ def workload_config(p, n, z_init):
             "l2": "inputs larger than L2 (state %.1f GB, fine mesh %.1f GB)" % (state_gb, mesh_gb)}
 
 
-def gpu_launches(p, steps):
-    """Launches of this library's kernels per step (cuFFT kernels not counted)."""
-    upd = 1 + 3 + 3 + 3 + 1 + 1  # dest, counting ranks (3: local, dense cells, base), scan (3),
-    #                               place + two vfield passes, scatter, sigma
+def gpu_launches(p, steps, conditional=True):
+    """Launches of this library's kernels per step on the counting path of the
+    re-sort (cuFFT kernels not counted); with conditional, also those that a
+    step makes only when it needs them."""
+    def scan(n):
+        return 1 if n <= 1 << 17 else 3
+    upd = 1 + 3 + scan(p.nc ** 3) + 3 + 1 + 1  # dest, counting ranks (local, dense cells, base), scan,
+    #                                            place + two vfield passes, scatter, sigma
     # PP: the prefilter (occupancy, neighbour masks with the activity bits, a
-    # scan of 3, compaction, cell starts), six staging levels, the active
-    # particles' kick
-    pp = 7 + 6 + 1 if p.pp_on else 0
-    fine = 4                     # deposit, green, maxima + kick factors, kick (PP's zero kicks inside)
+    # scan of a count per 32 particles, active lists), four staging levels and
+    # the scratch levels, the active particles' kick
+    pp = 3 + scan(p.npglobal // 32) + 5 + 1 if p.pp_on else 0
+    fine = 4                     # deposit, green, maxima, kick (PP's zero kicks inside)
     coarse = 4
-    codec = 3                    # decode table, encode boundaries and zero-kick table for the new sigma
-    return steps * (upd + pp + fine + coarse + codec)
+    codec = 1                    # the new sigma's tables
+    # the exact-vmax rerun of the coarse kick, tables of a second sigma (after
+    # an upload), the visit-order walker and the extra copies behind it
+    cond = 4 if conditional else 0
+    return steps * (upd + pp + fine + coarse + codec + cond)
 
 
 def cpu_baseline(p, state, sigma, ts):
