@@ -162,23 +162,23 @@ class ClockSampler:
 # ------------------------------------------------------------------ gb300 arm
 
 
-# DRAM bytes (read + write) per particle of one launch, from the full ncu
+# DRAM bytes (read + write) per particle of one launch, from the ncu
 # capture of the 256^3 workload (profiles/step_kernels_cdm256.md); meshes and
 # particle counts scale together between 256^3 and 512^3, so per-particle
 # traffic carries over
 TRAFFIC_PER_PARTICLE = {
-    # one ncu capture per kernel at 256^3 (profiles/step_kernels_cdm256.md),
+    # the step's kernels in one ncu capture at 256^3 (profiles/step_kernels_cdm256.md),
     # DRAM read + write per launch over the particles; pp_force: the brick
     # kernel and the neighbour-mask pass that marks the active particles
     # (the prefilter's smaller passes uncaptured)
-    "pp_force": (93.1e6 + 34.2e6 + 113.5e6 + 4.5e6) / 16778347,
-    "fine_kick": (2194.1e6 + 114.8e6) / 16778347,
-    "coarse_kick": (325.2e6 + 89.9e6) / 16778347,
-    "fine_deposit": (83.7e6 + 476.4e6) / 16778347,
-    "update_dest": (243.8e6 + 77.9e6) / 16778347,
-    "update_scatter": (506.5e6 + 257.2e6) / 16778347,
-    "fine_green": (1347.5e6 + 1567.8e6) / 16778347,
-    "fine_f2max": (1617.1e6 + 1560.4e6) / 16778347,
+    "pp_force": (127.1e6 + 118.5e6) / 16778347,
+    "fine_kick": 2635.5e6 / 16778347,
+    "coarse_kick": 361.9e6 / 16778347,
+    "fine_deposit": 560.8e6 / 16778347,
+    "update_dest": 443.5e6 / 16778347,
+    "update_scatter": 958.0e6 / 16778347,
+    "fine_green": 2915.6e6 / 16778347,
+    "fine_f2max": 1620.8e6 / 16778347,
 }
 
 
