@@ -60,6 +60,7 @@ static void release(cube_ctx* c) {
   }
   if (c->ev_aux) cudaEventDestroy(c->ev_aux);
   if (c->ev_codec) cudaEventDestroy(c->ev_codec);
+  if (c->ev_coarse) cudaEventDestroy(c->ev_coarse);
   if (c->owner) {  // meshes, kernels, plans, work area and stream belong to the owner
     if (c->owner->linked == c) c->owner->linked = nullptr;
     c->rho_f = c->kern_f = c->kern_f_raw = c->rho_c = c->kern_c = nullptr;
@@ -131,13 +132,14 @@ static int make_plans(cube_ctx* c) {
   };
   if (int r = inverse(c->plan_f_c2r, nf, &c->f_c2r_batch, &wf2)) return r;
   if (int r = inverse(c->plan_c_c2r, nc, &c->c_c2r_batch, &wc2)) return r;
-  size_t w = wf1;
-  for (size_t x : {wf2, wc1, wc2})
-    if (x > w) w = x;
-  c->cufft_work_bytes = w;
-  ALLOC(c->cufft_work, w);
+  // coarse transforms that run beside the fine ones have their own part of it
+  const size_t wf = (std::max(wf1, wf2) + 255) / 256 * 256, wc = std::max(wc1, wc2);
+  const size_t off = coarse_area(c) ? wf : 0;
+  c->cufft_work_bytes = std::max(wf, off + wc);
+  ALLOC(c->cufft_work, c->cufft_work_bytes);
   for (cufftHandle h : {c->plan_f_r2c, c->plan_f_c2r, c->plan_c_r2c, c->plan_c_c2r}) {
-    CUBE_FFT(c, cufftSetWorkArea(h, c->cufft_work));
+    const bool coarse = h == c->plan_c_r2c || h == c->plan_c_c2r;
+    CUBE_FFT(c, cufftSetWorkArea(h, (char*)c->cufft_work + (coarse ? off : 0)));
     CUBE_FFT(c, cufftSetStream(h, c->stream));
   }
   return CUBE_OK;
@@ -198,6 +200,7 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
   CUBE_CUDA(c, cudaStreamCreateWithPriority(&c->stream_aux, cudaStreamNonBlocking, aux_hi));
   CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_aux, cudaEventDisableTiming));
   CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_codec, cudaEventDisableTiming));
+  CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_coarse, cudaEventDisableTiming));
   int64_t np = p->np_max;
   for (int k = 0; k < 2; k++) {
     ALLOC(c->xp[k], 3 * np * p->izipx);
@@ -458,11 +461,14 @@ extern "C" int cube_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_stats
   int r = check_ready(c);
   if (r) return r;
   // every stage is queued; the stats come back once, with the coarse kick's
-  if ((r = cube_fine_forces_impl(c, nullptr))) return r;
+  const bool beside = coarse_beside(c);
+  if (beside && (r = cube_forces_fork(c))) return r;
+  if ((r = cube_fine_forces_impl(c, nullptr, beside))) return r;
   cube_force_fused(c, 0, a_mid, dt);
+  if (beside && (r = cube_coarse_beside(c))) return r;
   if ((r = cube_fine_kick_impl(c, a_mid, dt))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
-  if ((r = cube_coarse_forces_impl(c, nullptr, true))) return r;
+  if ((r = beside ? cube_forces_join(c) : cube_coarse_forces_impl(c, nullptr, true))) return r;
   cube_force_fused(c, 1, a_mid, dt);
   if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true))) return r;
   if (st) cube_fine_stats(c, st);
@@ -480,12 +486,11 @@ extern "C" int cube_pp_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_st
   if (!c->stream_pp) return cube_fail(c, CUBE_ERR_ARG, "PP is off for this context (pp_on = 0)");
   CUBE_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_pp, c->ev_fork, 0));
-  // Queueing PP takes the host longer than a small mesh's deposit and transforms
-  // take the device, so those go first there (nc 24: a leg of four steps 1.51 ->
-  // 1.47 ms); on a larger mesh PP's blocks should find the chip free (nc 54 even,
-  // nc 128 late 36.2 against 36.4 ms, nc 256 174.9 against 175.1).
-  const bool pm_first = c->ncells <= (int64_t)1 << 17;
-  if (pm_first && (r = cube_fine_forces_impl(c, nullptr))) return r;
+  // The fine forces are queued first: queueing PP takes the host longer than a
+  // small mesh's deposit and transforms take the device, and on a large one PP,
+  // at the higher priority, takes its slots as the deposit's blocks leave them.
+  const bool beside = coarse_beside(c);
+  if (beside && ((r = cube_forces_fork(c)) || (r = cube_fine_forces_impl(c, nullptr, true)))) return r;
   {  // PP's launches go to its stream with its own stats
     cudaStream_t s0 = c->stream;
     DevStats *d0 = c->dstats, *h0 = c->hstats;
@@ -503,14 +508,15 @@ extern "C" int cube_pp_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_st
     c->hstats = h0;
     if (r) return r;
   }
-  if (!pm_first && (r = cube_fine_forces_impl(c, nullptr))) return r;
+  if (!beside && (r = cube_fine_forces_impl(c, nullptr))) return r;
   cube_force_fused(c, 0, a_mid, dt);
-  if ((r = cube_coarse_forces_impl(c, nullptr, true))) return r;
+  if ((r = beside ? cube_coarse_beside(c) : cube_coarse_forces_impl(c, nullptr, true))) return r;
   cube_force_fused(c, 1, a_mid, dt);
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_pp, 0));
   // the fine kick applies PP's kick first (ext_pp_force.f90:116-121), then its own
   if ((r = cube_fine_kick_impl(c, a_mid, dt, /*with_pp=*/true))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
+  if (beside && (r = cube_forces_join(c))) return r;
   if ((r = cube_coarse_kick_impl(c, a_mid, dt, st_pm, true))) return r;
   if (st_pm) cube_fine_stats(c, st_pm);
   // PP's stats are in their host copy: the kicks waited for its stream

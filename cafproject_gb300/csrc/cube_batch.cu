@@ -139,9 +139,12 @@ int box_step(cube_ctx* c, int ncell, const float2* sched, int nsteps) {
   c->dstats = &c->sout->pp;
   if (c->p.pp_on && (r = cube_pp_impl(c, 0.f, 0.f, nullptr))) return r;
   c->dstats = &c->sout->coarse;
+  const bool beside = coarse_beside(c);
+  if (beside && (r = cube_forces_fork(c))) return r;
   if ((r = cube_fine_forces_impl(c, nullptr))) return r;
+  if (beside && (r = cube_coarse_beside(c))) return r;
   if ((r = cube_fine_kick_impl(c, 0.f, 0.f))) return r;
-  if ((r = cube_coarse_forces_impl(c, nullptr, true))) return r;
+  if ((r = beside ? cube_forces_join(c) : cube_coarse_forces_impl(c, nullptr, true))) return r;
   return cube_coarse_kick_impl(c, 0.f, 0.f, nullptr, true);
 }
 

@@ -159,6 +159,7 @@ struct cube_ctx {
   // own (cube_codec_prefetch, and update_x of a captured step); slot, or -1
   int codec_ahead = -1;
   cudaStream_t stream_aux = nullptr;
+  cudaEvent_t ev_coarse = nullptr;  // coarse forces done there (cube_coarse_beside)
   cudaEvent_t ev_aux = nullptr, ev_codec = nullptr;
   float sigma_vi = 0.f, sigma_vi_new = 0.f;
   float vmax_prev[3] = {0.f, 0.f, 0.f};  // last coarse-kick vmax (0: unknown)
@@ -786,10 +787,26 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick = false);
 int cube_pp_init(cube_ctx* c);  // once per context: the staging kernels' shared-memory sizes
 int cube_pp_finish(cube_ctx* c, cube_stats* st, bool fetched = false);  // fetched: hstats holds the stats already
 // density deposits; accumulate: add to the mesh (the linked species) instead of writing it
-int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false);
-// fresh (the coarse stages): the stats were zeroed by this step's fine density
+int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false, bool fresh = false);
+// fresh: the stats were zeroed already (by cube_forces_fork, or by this step's fine density)
 int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = false, bool fresh = false);
-int cube_fine_forces_impl(cube_ctx* c, cube_stats* st);
+int cube_fine_forces_impl(cube_ctx* c, cube_stats* st, bool fresh = false);
+// Fused steps: the coarse forces beside the fine ones, on the auxiliary stream.
+// On a small box they fill a chip that the fine chain leaves idle, on a large one
+// the ends of its passes (one after the other -> beside, PP queued behind the fine
+// chain: 48^3 leg 1.53 -> 1.36 ms, 64^3 1.58 -> 1.44, 108^3 3.63 -> 3.41, 208^3
+// 19.28 -> 19.09, 256^3 late 36.4 -> 36.0, 512^3 177 -> 175).  The coarse
+// transforms then have a work area of their own; above 2^24 coarse cells, whose
+// area would be gigabytes, they stay behind the fine ones.  cube_forces_fork comes
+// before the fine forces, cube_coarse_beside after them, cube_forces_join before
+// the coarse kick.
+constexpr int64_t COARSE_BESIDE = (int64_t)1 << 24;  // coarse cells
+inline bool coarse_area(const cube_ctx* c) { return !c->owner && c->ncells <= COARSE_BESIDE; }
+// (under the phase timers one after the other, so that each phase's time is its own)
+inline bool coarse_beside(const cube_ctx* c) { return coarse_area(c) && !c->timers; }
+int cube_forces_fork(cube_ctx* c);
+int cube_coarse_beside(cube_ctx* c);
+int cube_forces_join(cube_ctx* c);
 // the force meshes' content as the fused step's caller finds it (ForcePre); and
 // that of other origin than the transforms'
 int cube_force_settle(cube_ctx* c, int coarse);

@@ -869,10 +869,11 @@ int cube_force_settle(cube_ctx* c, int coarse) {
 }
 
 // ----------------------------------------------------------------- fine
-int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate) {
+int cube_fine_density_impl(cube_ctx* c, cube_stats* st, bool accumulate, bool fresh) {
   cudaStream_t s = c->stream;
   Geo g = make_geo(c);
-  if (!c->graph_mode) CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), s));  // (zeroed at the step's head)
+  if (!c->graph_mode && !fresh)  // (a captured step's head zeroes them)
+    CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), s));
   const int sh = dep_shift(c->p.mass_p);
   DepArgs a{g, c->xp[c->cur], c->rhoc[c->cur], c->cstart[c->cur], c->p.mass_p, c->rho_f, &c->dstats->rhof_fix, 0, 0.f,
             std::ldexp(1.0f, sh), std::ldexp(1.0f, -sh), accumulate ? 1 : 0};
@@ -893,8 +894,32 @@ void cube_fine_stats(const cube_ctx* c, cube_stats* st) {
   st->testrhof = std::ldexp((double)c->hstats->rhof_fix, -dep_shift(c->p.mass_p));
 }
 
-int cube_fine_forces_impl(cube_ctx* c, cube_stats* st) {
-  int r0 = cube_fine_density_impl(c, nullptr, false);
+int cube_forces_fork(cube_ctx* c) {
+  if (!c->graph_mode) CUBE_CUDA(c, cudaMemsetAsync(c->dstats, 0, sizeof(DevStats), c->stream));
+  CUBE_CUDA(c, cudaEventRecord(c->ev_aux, c->stream));
+  return CUBE_OK;
+}
+
+int cube_coarse_beside(cube_ctx* c) {
+  cudaStream_t s = c->stream;
+  CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_aux, c->ev_aux, 0));
+  for (cufftHandle h : {c->plan_c_r2c, c->plan_c_c2r}) CUBE_FFT(c, cufftSetStream(h, c->stream_aux));
+  c->stream = c->stream_aux;
+  const int r = cube_coarse_forces_impl(c, nullptr, true);
+  c->stream = s;
+  for (cufftHandle h : {c->plan_c_r2c, c->plan_c_c2r}) CUBE_FFT(c, cufftSetStream(h, s));
+  if (r) return r;
+  CUBE_CUDA(c, cudaEventRecord(c->ev_coarse, c->stream_aux));
+  return CUBE_OK;
+}
+
+int cube_forces_join(cube_ctx* c) {
+  CUBE_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_coarse, 0));
+  return CUBE_OK;
+}
+
+int cube_fine_forces_impl(cube_ctx* c, cube_stats* st, bool fresh) {
+  int r0 = cube_fine_density_impl(c, nullptr, false, fresh);
   if (r0) return r0;
   return cube_fine_spectral_impl(c, st);
 }
