@@ -132,11 +132,19 @@ static int make_plans(cube_ctx* c) {
   };
   if (int r = inverse(c->plan_f_c2r, nf, &c->f_c2r_batch, &wf2)) return r;
   if (int r = inverse(c->plan_c_c2r, nc, &c->c_c2r_batch, &wc2)) return r;
-  // coarse transforms that run beside the fine ones have their own part of it
+  // coarse transforms that run beside the fine ones have their own part of it,
+  // where the memory is there
   const size_t wf = (std::max(wf1, wf2) + 255) / 256 * 256, wc = std::max(wc1, wc2);
-  const size_t off = coarse_area(c) ? wf : 0;
-  c->cufft_work_bytes = std::max(wf, off + wc);
-  ALLOC(c->cufft_work, c->cufft_work_bytes);
+  size_t off = 0;
+  if (c->ncells <= COARSE_BESIDE && cudaMalloc(&c->cufft_work, wf + wc + 16) == cudaSuccess) {
+    off = wf;
+    c->coarse_own_work = true;
+    c->cufft_work_bytes = wf + wc;
+  } else {
+    cudaGetLastError();  // a failed cudaMalloc is also the thread's last error: clear it
+    c->cufft_work_bytes = std::max(wf, wc);
+    ALLOC(c->cufft_work, c->cufft_work_bytes);
+  }
   for (cufftHandle h : {c->plan_f_r2c, c->plan_f_c2r, c->plan_c_r2c, c->plan_c_c2r}) {
     const bool coarse = h == c->plan_c_r2c || h == c->plan_c_c2r;
     CUBE_FFT(c, cufftSetWorkArea(h, (char*)c->cufft_work + (coarse ? off : 0)));

@@ -241,6 +241,7 @@ struct cube_ctx {
   DevStats* hstats = nullptr;   // pinned
   void* cufft_work = nullptr;
   size_t cufft_work_bytes = 0;
+  bool coarse_own_work = false;  // the coarse plans have a part of it to themselves (never set on a linked context)
 };
 
 // ------------------------------------------------------------------ errors
@@ -801,9 +802,8 @@ int cube_fine_forces_impl(cube_ctx* c, cube_stats* st, bool fresh = false);
 // before the fine forces, cube_coarse_beside after them, cube_forces_join before
 // the coarse kick.
 constexpr int64_t COARSE_BESIDE = (int64_t)1 << 24;  // coarse cells
-inline bool coarse_area(const cube_ctx* c) { return !c->owner && c->ncells <= COARSE_BESIDE; }
 // (under the phase timers one after the other, so that each phase's time is its own)
-inline bool coarse_beside(const cube_ctx* c) { return coarse_area(c) && !c->timers; }
+inline bool coarse_beside(const cube_ctx* c) { return c->coarse_own_work && !c->timers; }
 int cube_forces_fork(cube_ctx* c);
 int cube_coarse_beside(cube_ctx* c);
 int cube_forces_join(cube_ctx* c);
