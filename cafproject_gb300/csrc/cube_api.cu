@@ -60,6 +60,7 @@ static void release(cube_ctx* c) {
   }
   if (c->ev_aux) cudaEventDestroy(c->ev_aux);
   if (c->ev_codec) cudaEventDestroy(c->ev_codec);
+  if (c->ev_sums) cudaEventDestroy(c->ev_sums);
   if (c->ev_coarse) cudaEventDestroy(c->ev_coarse);
   if (c->owner) {  // meshes, kernels, plans, work area and stream belong to the owner
     if (c->owner->linked == c) c->owner->linked = nullptr;
@@ -208,6 +209,7 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
   CUBE_CUDA(c, cudaStreamCreateWithPriority(&c->stream_aux, cudaStreamNonBlocking, aux_hi));
   CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_aux, cudaEventDisableTiming));
   CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_codec, cudaEventDisableTiming));
+  CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_sums, cudaEventDisableTiming));
   CUBE_CUDA(c, cudaEventCreateWithFlags(&c->ev_coarse, cudaEventDisableTiming));
   int64_t np = p->np_max;
   for (int k = 0; k < 2; k++) {

@@ -161,6 +161,7 @@ struct cube_ctx {
   cudaStream_t stream_aux = nullptr;
   cudaEvent_t ev_coarse = nullptr;  // coarse forces done there (cube_coarse_beside)
   cudaEvent_t ev_aux = nullptr, ev_codec = nullptr;
+  cudaEvent_t ev_sums = nullptr;  // captured step: the velocity sums beside the step have read the codes
   float sigma_vi = 0.f, sigma_vi_new = 0.f;
   float vmax_prev[3] = {0.f, 0.f, 0.f};  // last coarse-kick vmax (0: unknown)
   // graph mode (cube_batch_*): step scalars on the device, codec slot

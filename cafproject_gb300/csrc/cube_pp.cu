@@ -1030,6 +1030,7 @@ int cube_pp_launch(cube_ctx* c, float a_mid, float dt, bool defer_kick) {
   // level 4: a block per SM, each region at least twice level 3's room
   const int g4 = (int)std::max<int64_t>(1, std::min<int64_t>(one_per_sm, c->pp_scr_cap / (2 * PP_CAP1)));
   k_pp_global<<<start <= 4 ? g4 : 1, PP_THREADS1, 0, c->stream>>>(a);
+  if (c->graph_mode) CUBE_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_sums, 0));  // update_x's sums read these codes
   if (!defer_kick)
     k_pp_kick<<<cube_grid(c->np, 256), 256, 0, c->stream>>>(a);
   else if (c->pp_act_valid)  // the fine kick gives the others their zero-kick codes

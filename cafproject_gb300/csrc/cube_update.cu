@@ -1244,8 +1244,10 @@ static int update_x_graph(cube_ctx* c) {
   k_vfield_new<<<cube_grid(c->ncells, 128, 32), 128, 0, s>>>(a);
   k_vfield_dense<<<cube_grid((int64_t)1 << 40, 1, 6), VF_BLOCK, 0, s>>>(a);
   k_scatter<<<cube_grid(c->np, B, MOVE_BLOCKS), B, 0, s>>>(a);
-  // sigma_vi_new and its codec tables beside the densities and transforms: the
-  // fine kick is the first to need them (it waits for ev_codec)
+  // sigma_vi_new and its codec tables beside PP's pairs, the densities and the
+  // transforms.  The sums read the codes, which PP's kick changes in place (it
+  // waits for ev_sums); the fine kick is the first to need the tables (it waits
+  // for ev_codec, so without PP the codes change no earlier either)
   CUBE_CUDA(c, cudaEventRecord(c->ev_aux, s));
   CUBE_CUDA(c, cudaStreamWaitEvent(c->stream_aux, c->ev_aux, 0));
   const double npg = (double)(c->npglobal > 0 ? c->npglobal : c->np);
@@ -1253,6 +1255,7 @@ static int update_x_graph(cube_ctx* c) {
                      c->p.izipv, c->red_tmp, c->red_count, nullptr, false, npg, c->sd, c->sout};
   k_sigma<<<sigma_blocks(c, c->np), SG_THREADS, 0, c->stream_aux>>>(sg);
   CUBE_CUDA(c, cudaGetLastError());
+  CUBE_CUDA(c, cudaEventRecord(c->ev_sums, c->stream_aux));
   c->stream = c->stream_aux;
   r = cube_codec_build_dev(c, 1 - c->graph_slot, &c->sd->sigma_new);
   c->stream = s;

@@ -1,0 +1,99 @@
+"""Which of a step's operations are ordered after which, checked on the CPU.
+
+The library runs with the CUDA runtime and cuFFT replaced by a stand-in
+(host/stream_log.c) that records launches, copies, events and waits and runs no
+kernel.  From the record each operation gets a vector clock over streams and the
+host, so "a is ordered before b" is a comparison, whatever a GPU's timing would
+have made of it."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+@pytest.fixture(scope="session")
+def standin(tmp_path_factory):
+    so = tmp_path_factory.mktemp("standin") / "libstream_log.so"
+    subprocess.run(["gcc", "-O1", "-w", "-shared", "-fPIC", "-o", str(so), os.path.join(HERE, "host", "stream_log.c")],
+                   check=True)
+    return so
+
+
+class Ops:
+    """The recorded operations with their vector clocks."""
+
+    def __init__(self, log):
+        clock, events, host = {}, {}, {}
+        self.ops = []
+
+        def join(a, b):
+            for k, v in b.items():
+                a[k] = max(a.get(k, 0), v)
+
+        for line in log.splitlines():
+            kind, s, x, name = line.split(" ", 3)
+            c = clock.setdefault(s, {})
+            if kind == "op":
+                join(c, host)
+                c[s] = c.get(s, 0) + 1
+                self.ops.append((name, s, c[s], dict(c)))
+            elif kind == "record":
+                events[x] = dict(c)
+            elif kind == "wait":
+                join(c, events.get(x, {}))
+            elif kind == "hostwait":
+                join(host, events.get(x, {}))
+            elif kind == "sync":
+                join(host, c)
+            elif kind == "syncall":
+                for k in clock.values():
+                    join(host, k)
+
+    def find(self, name):
+        return [o for o in self.ops if name in o[0]]
+
+    @staticmethod
+    def before(a, b):
+        return b[3].get(a[1], 0) >= a[2]
+
+
+def run(standin, tmp_path, lib, script):
+    log = tmp_path / "log"
+    env = dict(os.environ, LD_PRELOAD=str(standin), STREAM_LOG=str(log), PYTHONPATH=ROOT)
+    r = subprocess.run([sys.executable, "-c", script], env=env, cwd=ROOT, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr
+    return Ops(log.read_text())
+
+
+BATCH = """
+from cafproject_gb300 import batch as B
+from cafproject_gb300.cube import CubeError
+b = B.Batch([(B.box_params(32, pp_on=%r), 1)], z_init=19.0, mode=B.GRAPH)
+b.set_schedule(0.0, 4)
+try:
+    b.step(1)  # captures both parities; no kernel ran, so the check of the step's results fails
+except CubeError as e:
+    assert "box 0 step 1: " in str(e), e
+"""
+
+
+@pytest.mark.parametrize("pp_on", [True, False])
+def test_captured_sums_before_the_codes_change(standin, tmp_path, built_lib, pp_on):
+    """The captured step's velocity sums read the codes that the PP kick (in
+    place) and the kicks after it rewrite: none may start before they are done."""
+    o = run(standin, tmp_path, built_lib, BATCH % pp_on)
+    sums = o.find("k_sigma")
+    assert len(sums) == 2  # one per parity
+    after = [k for k in o.find("k_pp_kick") + o.find("k_kick")]
+    assert len(o.find("k_pp_kick")) == (2 if pp_on else 0) and len(o.find("k_kick")) == 6
+    for i, s in enumerate(sums):
+        end = sums[i + 1] if i + 1 < len(sums) else None
+        seq = o.ops[o.ops.index(s):o.ops.index(end) if end else None]
+        writers = [k for k in seq if k in after]
+        assert writers
+        for k in writers:
+            assert o.before(s, k), k[0]
