@@ -138,15 +138,17 @@ int cube_scan_counts(cube_ctx* c, const int32_t* counts, int64_t* starts, int64_
 
 // ---------------------------------------------------------- cell index
 // pcell[p] = cell of particle p, from the spine: one thread per cell; a
-// negative count is flagged (bit 16 of *flags) and writes nothing.
+// negative count is flagged (bit 16 of *flags) and writes nothing.  The counts
+// are the caller's and not yet checked: the spine may run below 0 or past np.
 __global__ void k_fill_pcell(const int32_t* __restrict__ rhoc, const int64_t* __restrict__ cstart, int64_t ncells,
-                             int32_t* __restrict__ pcell, int* flags) {
+                             int64_t np, int32_t* __restrict__ pcell, int* flags) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncells; c += (int64_t)gridDim.x * blockDim.x) {
     if (rhoc && rhoc[c] < 0) {
       atomicOr(flags, 1 << 16);
       continue;
     }
-    for (int64_t p = cstart[c]; p < cstart[c + 1]; p++) pcell[p] = (int32_t)c;
+    const int64_t p1 = min(cstart[c + 1], np);
+    for (int64_t p = max(cstart[c], (int64_t)0); p < p1; p++) pcell[p] = (int32_t)c;
   }
 }
 
@@ -199,7 +201,7 @@ int cube_state_in(cube_ctx* c, int64_t np, const void* xp, const void* vp, const
   r = cube_scan_counts(c, c->rhoc[k], c->cstart[k], c->ncells);
   if (r) return r;
   CUBE_CUDA(c, cudaMemsetAsync(&c->dstats->flags, 0, sizeof(int), c->stream));
-  k_fill_pcell<<<cube_grid(c->ncells, 256), 256, 0, c->stream>>>(c->rhoc[k], c->cstart[k], c->ncells, c->pcell[k],
+  k_fill_pcell<<<cube_grid(c->ncells, 256), 256, 0, c->stream>>>(c->rhoc[k], c->cstart[k], c->ncells, np, c->pcell[k],
                                                                  &c->dstats->flags);
   CUBE_CUDA(c, cudaGetLastError());
   int64_t tot = -1;

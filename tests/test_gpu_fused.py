@@ -71,6 +71,32 @@ def test_upload_rejects_inconsistent_counts():
         g.close()
 
 
+@pytest.mark.parametrize("begin", [False, True])
+def test_upload_rejects_counts_beyond_the_arrays(begin):
+    # counts whose cells would start far past the particle arrays, or (behind a
+    # negative count) before them, write nothing there: an error, and the
+    # context takes the next upload
+    from cafproject_gb300 import cube as C
+    from cafproject_gb300 import params as P
+    from cafproject_gb300 import synth
+    p = P.small(nc=24, nnt=2, pp_on=False)
+    st = synth.random_state(p, mean_per_cell=4, seed=3)
+    g = C.CubeGPU(p)
+    try:
+        for cell, count, code in ((5, 500000000, 6), (13823, 2147483647, 6), (0, -2000000000, 1)):
+            bad = st["rhoc"].copy()
+            bad.reshape(-1)[cell] = count
+            with pytest.raises(C.CubeError) as e:
+                (g.upload_begin if begin else g.upload)(st["xp"], st["vp"], st["pid"], bad, st["vfield"])
+            assert e.value.code == code
+        g.upload(st["xp"], st["vp"], st["pid"], st["rhoc"], st["vfield"])
+        out = g.download()
+        for k in ("xp", "vp", "pid", "rhoc"):
+            np.testing.assert_array_equal(out[k].reshape(-1), st[k].reshape(-1))
+    finally:
+        g.close()
+
+
 def test_split_download_matches_download():
     # xp, pid, rhoc and vfield copied beside PP+PM (cube_download_begin right
     # after update_x), vp behind the coarse kick's pieces: the same arrays as a
