@@ -71,15 +71,17 @@ __global__ void k_scan_sums(long long* __restrict__ bsum, int64_t nb) {
 // The chunk at base of the counts, scanned into starts from off on: counts and
 // results pass through shared memory so that the global accesses are
 // consecutive; a word of padding per thread's stretch keeps the stretches of
-// neighbouring threads in different banks (256^3 counts: 89 -> 35 us).  (Within a chunk offsets are 32-bit:
-// an image holds fewer than 2^31 particles.)
+// neighbouring threads in different banks (256^3 counts: 89 -> 35 us).  (Within a chunk
+// offsets are 32-bit: an image holds fewer than 2^31 particles.  The total is
+// 64-bit throughout: an upload compares it with the particle count while the
+// counts may still be anything.)
 __device__ __forceinline__ int scan_at(int i) { return i + i / SCAN_I; }
 __device__ __forceinline__ void scan_chunk(const int32_t* __restrict__ cnt, int64_t n, int64_t base,
                                            int64_t* __restrict__ starts, int32_t* tile, long long* s, long long off) {
   for (int i = threadIdx.x; i < SCAN_CHUNK; i += SCAN_T) tile[scan_at(i)] = base + i < n ? cnt[base + i] : 0;
   __syncthreads();
   int32_t* mine = tile + scan_at(threadIdx.x * SCAN_I);
-  int v = 0;
+  long long v = 0;
 #pragma unroll
   for (int i = 0; i < SCAN_I; i++) v += mine[i];
   long long tot;
