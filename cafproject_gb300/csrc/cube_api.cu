@@ -118,10 +118,9 @@ static int make_plans(cube_ctx* c) {
   // batched plan: a third of the launches, and more blocks in each (64: 37 ->
   // 19 us, 128: 62 -> 41, 200: 240 -> 222).  From 232 on the batch is no faster
   // and sometimes slower (232: 407 -> 425, 264: 518 -> 586).  The same bits for
-  // every size compared (16 to 640).  Odd extents keep the single plan, whose
-  // default in-place layout differs there.
+  // every size compared (16 to 640).
   auto inverse = [&](cufftHandle h, int n, int* batch, size_t* w) -> int {
-    if (n > 224 || n % 2) {
+    if (n > 224) {
       CUBE_FFT(c, cufftMakePlan3d(h, n, n, n, CUFFT_C2R, w));
       return CUBE_OK;
     }
@@ -171,6 +170,9 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
   // LRCKCORR rescales the coarse modes with |k|<=8 by 1/Im FFT(raw kernel)
   // (kernel_c.f90:111-113); below nc = 16 that sphere wraps past Nyquist
   if (p->nc < 16) return bad("nc must be at least 16 (coarse kernel correction needs |k|<=8 up to Nyquist)");
+  // the meshes' rows are nc + 2 values, which is the transforms' in-place layout
+  // for even sizes only, and the kernels read them in pairs
+  if (p->nc % 2) return bad("nc must be even");
   // the deposits keep a cell's coordinates in 16-bit fields; far beyond any mesh HBM holds
   if (p->nc > 16384) return bad("nc must be at most 16384");
   if (p->ncell != 4) return bad("ncell must be 4");
@@ -267,7 +269,7 @@ static int create_impl(const cube_params* p, const float* fine_table, const floa
     for (int d = 1; d < 3; d++) c->force_f[d] = c->force_f[0] + d * fpad;
     ALLOC(c->kern_f, 4 * 3 * nfh * c->nf * (int64_t)c->nf);
     int64_t nch = (int64_t)(p->nc / 2 + 1);
-    int64_t cpad = (int64_t)(p->nc + 2) * p->nc * (int64_t)p->nc;  // the kernels' row stride, for odd nc too
+    int64_t cpad = 2 * nch * p->nc * (int64_t)p->nc;
     ALLOC(c->rho_c, 4 * cpad);
     ALLOC(c->force_c[0], 3 * 4 * cpad);
     for (int d = 1; d < 3; d++) c->force_c[d] = c->force_c[0] + d * cpad;

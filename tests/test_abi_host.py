@@ -53,6 +53,21 @@ def test_cube_create_rejects_bad_sizes(built_lib, nc, msg):
     L.cube_destroy(h)
 
 
+@pytest.mark.parametrize("nc,nnt", [(17, 1), (45, 3), (255, 1)])
+def test_cube_create_rejects_odd_nc(built_lib, nc, nnt):
+    # the padded meshes are the transforms' in-place layout for even sizes only
+    from cafproject_gb300 import cube
+    L = cube.load_library()
+    bad = P.CubeParams(nc=nc, nnt=nnt).to_c()
+    fine, coarse = cube.force_tables()
+    h = ctypes.c_void_p()
+    rc = L.cube_create(ctypes.byref(bad), fine.ctypes.data_as(ctypes.c_void_p),
+                       coarse.ctypes.data_as(ctypes.c_void_p), 0, ctypes.byref(h))
+    assert rc == 1  # CUBE_ERR_ARG before any device call
+    assert b"nc must be even" in L.cube_last_error(h)
+    L.cube_destroy(h)
+
+
 def test_expansion_advances_scale_factor():
     a = np.float32(0.02)
     d1, d2 = cosmology.expansion(a, np.float32(0.1), 0.3, 0.7)
