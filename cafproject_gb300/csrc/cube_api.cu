@@ -469,11 +469,25 @@ extern "C" int cube_pm_coarse_kick(cube_ctx* c, float a_mid, float dt, cube_stat
   return cube_coarse_kick_impl(c, a_mid, dt, st);
 }
 
+// A fused step may end in an error (a sigma that is not positive, at the fine
+// kick) with the coarse forces queued beside it: what the context's stream gets
+// next then waits for them.
+namespace {
+struct JoinOnReturn {
+  cube_ctx* c;
+  bool on;
+  ~JoinOnReturn() {
+    if (on && cudaEventRecord(c->ev_coarse, c->stream_aux) == cudaSuccess) cube_forces_join(c);
+  }
+};
+}  // namespace
+
 extern "C" int cube_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_stats* st) {
   int r = check_ready(c);
   if (r) return r;
   // every stage is queued; the stats come back once, with the coarse kick's
   const bool beside = coarse_beside(c);
+  JoinOnReturn left{c, beside};
   if (beside && (r = cube_forces_fork(c))) return r;
   if ((r = cube_fine_forces_impl(c, nullptr, beside))) return r;
   cube_force_fused(c, 0, a_mid, dt);
@@ -481,6 +495,7 @@ extern "C" int cube_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_stats
   if ((r = cube_fine_kick_impl(c, a_mid, dt))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
   if ((r = beside ? cube_forces_join(c) : cube_coarse_forces_impl(c, nullptr, true))) return r;
+  left.on = false;
   cube_force_fused(c, 1, a_mid, dt);
   if ((r = cube_coarse_kick_impl(c, a_mid, dt, st, true))) return r;
   if (st) cube_fine_stats(c, st);
@@ -502,6 +517,7 @@ extern "C" int cube_pp_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_st
   // small mesh's deposit and transforms take the device, and on a large one PP,
   // at the higher priority, takes its slots as the deposit's blocks leave them.
   const bool beside = coarse_beside(c);
+  JoinOnReturn left{c, beside};
   if (beside && ((r = cube_forces_fork(c)) || (r = cube_fine_forces_impl(c, nullptr, true)))) return r;
   {  // PP's launches go to its stream with its own stats
     cudaStream_t s0 = c->stream;
@@ -529,6 +545,7 @@ extern "C" int cube_pp_particle_mesh(cube_ctx* c, float a_mid, float dt, cube_st
   if ((r = cube_fine_kick_impl(c, a_mid, dt, /*with_pp=*/true))) return r;
   c->sigma_vi = c->sigma_vi_new;  // pm.f90:193
   if (beside && (r = cube_forces_join(c))) return r;
+  left.on = false;
   if ((r = cube_coarse_kick_impl(c, a_mid, dt, st_pm, true))) return r;
   if (st_pm) cube_fine_stats(c, st_pm);
   // PP's stats are in their host copy: the kicks waited for its stream

@@ -97,3 +97,33 @@ def test_captured_sums_before_the_codes_change(standin, tmp_path, built_lib, pp_
         assert writers
         for k in writers:
             assert o.before(s, k), k[0]
+
+
+FAILED_KICK = """
+from cafproject_gb300 import cube as C
+from cafproject_gb300 import batch as B
+p = B.box_params(32, pp_on=%r)
+g = C.CubeGPU(p)
+g.ic_zeldovich(19.0, seed=1)
+g.set_sigma(g.get_sigma()[0], 0.0)  # what a re-sort of particles at rest leaves
+try:
+    (g.pp_particle_mesh if p.pp_on else g.particle_mesh)(0.4, 0.02)
+    raise SystemExit("a zero sigma went through")
+except C.CubeError as e:
+    assert "sigma_vi must be positive" in str(e), e
+g.get_field(C.FIELD_RHO_C)
+"""
+
+
+@pytest.mark.parametrize("pp_on", [True, False])
+def test_failed_step_leaves_nothing_beside(standin, tmp_path, built_lib, pp_on):
+    """A fused step that ends in an error while the coarse forces run beside it:
+    whatever the next call does on the context's stream comes after them."""
+    o = run(standin, tmp_path, built_lib, FAILED_KICK % pp_on)
+    main = o.find("k_ic_gather")[0][1]
+    read = o.find("memcpy2D")[-1]
+    assert read[1] == main and o.ops[-1] == read
+    beside = [k for k in o.ops if k[1] != main]
+    assert any("k_deposit" in k[0] for k in beside) and any("c2r" in k[0] for k in beside)
+    for k in beside:
+        assert o.before(k, read), k[0]
