@@ -454,7 +454,7 @@ extern "C" int cube_pm_fine_forces(cube_ctx* c, cube_stats* st) {
 extern "C" int cube_pm_fine_kick(cube_ctx* c, float a_mid, float dt) {
   int r = check_ready(c);
   if (r) return r;
-  if ((r = cube_force_settle(c, 0))) return r;
+  if ((r = cube_force_ready(c, 0))) return r;
   return cube_fine_kick_impl(c, a_mid, dt);
 }
 extern "C" int cube_pm_coarse_forces(cube_ctx* c, cube_stats* st) {
@@ -465,7 +465,7 @@ extern "C" int cube_pm_coarse_forces(cube_ctx* c, cube_stats* st) {
 extern "C" int cube_pm_coarse_kick(cube_ctx* c, float a_mid, float dt, cube_stats* st) {
   int r = check_ready(c);
   if (r) return r;
-  if ((r = cube_force_settle(c, 1))) return r;
+  if ((r = cube_force_ready(c, 1))) return r;
   return cube_coarse_kick_impl(c, a_mid, dt, st);
 }
 

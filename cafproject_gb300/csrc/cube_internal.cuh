@@ -134,9 +134,11 @@ struct cube_ctx {
   // velocity code tables
   // The kicks' look at the force meshes, beside them on their owner: the bits of
   // the maxima of force^2 (fine, coarse), NaN when the meshes' content is not
-  // the last transforms'.  force_pre: a fused step left the meshes as forces
-  // where its caller finds force*a_mid*dt/6/pi (get_field)
+  // the last transforms' and has not been looked over since (f2_known).
+  // force_pre: a fused step left the meshes as forces where its caller finds
+  // force*a_mid*dt/6/pi (get_field)
   unsigned* f2_kick = nullptr;
+  bool f2_known[2] = {false, false};
   struct ForcePre {
     bool on = false;
     float a_mid = 0.f, dt = 0.f;
@@ -812,6 +814,8 @@ int cube_forces_join(cube_ctx* c);
 // that of other origin than the transforms'
 int cube_force_settle(cube_ctx* c, int coarse);
 int cube_force_foreign(cube_ctx* c, int coarse);
+// before a kick of its own (not a fused step's): settled, and their maximum known
+int cube_force_ready(cube_ctx* c, int coarse);
 inline void cube_force_fused(cube_ctx* c, int coarse, float a_mid, float dt) {
   (c->owner ? c->owner : c)->force_pre[coarse] = {true, a_mid, dt};
 }

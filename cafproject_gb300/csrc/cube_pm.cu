@@ -850,8 +850,16 @@ __global__ void k_force_pre(float* __restrict__ f, int64_t n, float a_mid, float
 }
 }  // namespace
 
+// the meshes hold the transforms' forces, their maximum behind them
+static void force_transformed(cube_ctx* c, int coarse) {
+  cube_ctx* o = c->owner ? c->owner : c;
+  o->force_pre[coarse].on = false;
+  o->f2_known[coarse] = true;
+}
+
 int cube_force_foreign(cube_ctx* c, int coarse) {
-  (c->owner ? c->owner : c)->force_pre[coarse].on = false;
+  cube_ctx* o = c->owner ? c->owner : c;
+  o->force_pre[coarse].on = o->f2_known[coarse] = false;
   CUBE_CUDA(c, cudaMemsetAsync(c->f2_kick + coarse, 0xff, 4, c->stream));
   return CUBE_OK;
 }
@@ -866,6 +874,19 @@ int cube_force_settle(cube_ctx* c, int coarse) {
                                                                pre.dt);
   CUBE_CUDA(c, cudaGetLastError());
   return cube_force_foreign(c, coarse);
+}
+
+// (the pass over the mesh takes a fraction of the FP64 chain for every component,
+// which is the kick's way without the maximum)
+int cube_force_ready(cube_ctx* c, int coarse) {
+  if (int r = cube_force_settle(c, coarse)) return r;
+  cube_ctx* o = c->owner ? c->owner : c;
+  if (o->f2_known[coarse]) return CUBE_OK;
+  CUBE_CUDA(c, cudaMemsetAsync(c->f2_kick + coarse, 0, 4, c->stream));
+  launch_f2max(c, coarse ? c->force_c : c->force_f, coarse ? c->p.nc : c->nf, c->f2_kick + coarse, c->f2_kick + coarse);
+  CUBE_CUDA(c, cudaGetLastError());
+  o->f2_known[coarse] = true;
+  return CUBE_OK;
 }
 
 // ----------------------------------------------------------------- fine
@@ -942,7 +963,7 @@ int cube_fine_spectral_impl(cube_ctx* c, cube_stats* st) {
   cube_phase_end(c, PH_F_C2R);
   cube_phase_begin(c, PH_F_F2MAX);
   launch_f2max(c, c->force_f, c->nf, &c->dstats->f2_fine_bits, c->f2_kick);
-  (c->owner ? c->owner : c)->force_pre[0].on = false;
+  force_transformed(c, 0);
   cube_phase_end(c, PH_F_F2MAX);
   CUBE_CUDA(c, cudaGetLastError());
   if (st) {
@@ -1055,7 +1076,7 @@ int cube_coarse_spectral_impl(cube_ctx* c, cube_stats* st) {
   for (int d = 0; d < 3; d += c->c_c2r_batch)
     CUBE_FFT(c, cufftExecC2R(c->plan_c_c2r, (cufftComplex*)c->force_c[d], c->force_c[d]));
   launch_f2max(c, c->force_c, nc, &c->dstats->f2_coarse_bits, c->f2_kick + 1);
-  (c->owner ? c->owner : c)->force_pre[1].on = false;
+  force_transformed(c, 1);
   cube_phase_end(c, PH_C_FFT);
   CUBE_CUDA(c, cudaGetLastError());
   if (st) {

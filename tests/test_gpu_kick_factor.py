@@ -70,3 +70,25 @@ def test_fields_after_a_fused_step():
     np.testing.assert_array_equal(b.get_field(C.FIELD_FORCE_F), raw_f)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e13, 1e17, np.inf, np.nan])
+def test_written_forces_equal_fp64(scale):
+    """Stage kicks on force meshes that the caller wrote, and on those that a
+    fused step left, with and without the exact option."""
+    C, make = _state()
+    out = []
+    for exact in (0, 1):
+        g = make()
+        g.set_option(C.OPT_EXACT_KICKS, exact)
+        g.particle_mesh(0.4, 0.02)
+        g.fine_kick(0.4, 0.02)
+        g.coarse_kick(0.4, 0.02)
+        for field, kick in ((C.FIELD_FORCE_F, g.fine_kick), (C.FIELD_FORCE_C, g.coarse_kick)):
+            f = g.get_field(field)
+            f.reshape(-1)[::97] *= np.float32(scale)
+            g.set_field(field, f)
+            kick(0.3, 0.01)
+        out.append(g.download()["vp"])
+        g.close()
+    np.testing.assert_array_equal(out[0], out[1])

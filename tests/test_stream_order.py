@@ -127,3 +127,27 @@ def test_failed_step_leaves_nothing_beside(standin, tmp_path, built_lib, pp_on):
     assert any("k_deposit" in k[0] for k in beside) and any("c2r" in k[0] for k in beside)
     for k in beside:
         assert o.before(k, read), k[0]
+
+
+OWN_FORCES = """
+from cafproject_gb300 import cube as C
+from cafproject_gb300 import batch as B
+p = B.box_params(32, pp_on=False)
+g = C.CubeGPU(p)
+g.ic_zeldovich(19.0, seed=1)
+g.%s_forces()
+g.set_field(C.FIELD_FORCE_%s, g.get_field(C.FIELD_FORCE_%s))
+for _ in range(2):
+    g.%s_kick(0.4, 0.02)
+"""
+
+
+@pytest.mark.parametrize("level", ["fine", "coarse"])
+def test_written_forces_keep_the_fast_kick(standin, tmp_path, built_lib, level):
+    """The kick's fast path needs the maximum of the force mesh: after the
+    caller has written the mesh it is found once, before the first kick."""
+    F = level[0].upper()
+    o = run(standin, tmp_path, built_lib, OWN_FORCES % (level, F, F, level))
+    names = [k[0] for k in o.ops if "k_f2max" in k[0] or "k_kick" in k[0] or k[0] == "memcpy2D"]
+    tail = ["max" if "f2max" in n else "kick" for n in names[len(names) - 1 - names[::-1].index("memcpy2D"):]]
+    assert tail[1:3] == ["max", "kick"] and tail.count("max") == 1 and tail.count("kick") >= 2
