@@ -644,7 +644,8 @@ extern "C" int cube_set_option(cube_ctx* c, int option, int64_t value) {
       return CUBE_OK;
     case CUBE_OPT_DEPOSIT_FINE:
     case CUBE_OPT_DEPOSIT_COARSE:
-      if (value < 0 || value > 3) return cube_fail(c, CUBE_ERR_ARG, "deposit brick shape must be 0 to 3");
+      if (value < -1 || value > 3)
+        return cube_fail(c, CUBE_ERR_ARG, "deposit brick shape must be 0 to 3, or -1 (by the mesh)");
       (option == CUBE_OPT_DEPOSIT_FINE ? c->opt_dep_fine : c->opt_dep_coarse) = (int)value;
       return CUBE_OK;
     case CUBE_OPT_FAIL_ALLOC:

@@ -331,8 +331,8 @@ void* cube_stream(cube_ctx* ctx);
    CUBE_OPT_DEPOSIT_FINE=4 / CUBE_OPT_DEPOSIT_COARSE=5 pick the brick shape
    of the fine / coarse density deposit (0-3; fine: 8x4x4, 4x4x4, 8x4x2,
    4x4x2 coarse cells; coarse: 8x8x8, 16x8x8, 8x8x4, 4x4x4): a tile-size
-   choice for the autotuner, same exact sums for every shape; unless set, the
-   mesh size decides.
+   choice for the autotuner, same exact sums for every shape; -1, the
+   default, leaves it to the mesh size.
    CUBE_OPT_FAIL_ALLOC=6 is host-side fault injection for tests: value n > 0
    makes the n-th device allocation the library makes lazily (the general
    re-sort's key buffers, on first use) report failure, 0 turns it off.

@@ -151,3 +151,28 @@ def test_written_forces_keep_the_fast_kick(standin, tmp_path, built_lib, level):
     names = [k[0] for k in o.ops if "k_f2max" in k[0] or "k_kick" in k[0] or k[0] == "memcpy2D"]
     tail = ["max" if "f2max" in n else "kick" for n in names[len(names) - 1 - names[::-1].index("memcpy2D"):]]
     assert tail[1:3] == ["max", "kick"] and tail.count("max") == 1 and tail.count("kick") >= 2
+
+
+BRICKS = """
+from cafproject_gb300 import cube as C
+from cafproject_gb300 import batch as B
+g = C.CubeGPU(B.box_params(32, pp_on=False))
+g.ic_zeldovich(19.0, seed=1)
+for shape in (None, 0, -1):
+    if shape is not None:
+        g.set_option(C.OPT_DEPOSIT_%s, shape)
+    g.%s_density()
+for shape in (-2, 4):
+    try:
+        g.set_option(C.OPT_DEPOSIT_%s, shape)
+        raise SystemExit("shape %%d went through" %% shape)
+    except C.CubeError:
+        pass
+"""
+
+
+@pytest.mark.parametrize("level", ["fine", "coarse"])
+def test_default_brick_can_be_chosen_again(standin, tmp_path, built_lib, level):
+    o = run(standin, tmp_path, built_lib, BRICKS % (level.upper(), level, level.upper()))
+    names = [k[0] for k in o.find("k_deposit")]
+    assert len(names) == 3 and names[0] == names[2] != names[1]
