@@ -290,13 +290,14 @@ int launch_deposit(cube_ctx* c, const DepArgs& a) {
 // 4.53 against 4.58 ms); the coarse one takes it up to three bricks a
 // multiprocessor (nc 48: 52 against 72, nc 64: 76.5 against 78.6, nc 96: 189
 // against 173).
-int default_bricks(const cube_ctx* c, int bx, int by, int bz) {
-  const int nc = c->p.nc;
+int64_t default_bricks(const cube_ctx* c, int bx, int by, int bz) {
+  const int64_t nc = c->p.nc;
   return ((nc + bx - 1) / bx) * ((nc + by - 1) / by) * ((nc + bz - 1) / bz);
 }
+int sm_count() { return cube_grid((int64_t)1 << 40, 1, 1); }
 int launch_fine_deposit(cube_ctx* c, const DepArgs& a) {
   int shape = c->opt_dep_fine;
-  if (shape < 0) shape = default_bricks(c, 8, 4, 4) < 152 ? 3 : 2;
+  if (shape < 0) shape = default_bricks(c, 8, 4, 4) < sm_count() ? 3 : 2;
   switch (shape) {
     case 1: return launch_deposit<4, 4, 4, 4, 1, 0>(c, a);  // 16^3 fine cells, 32 KB
     case 2: return launch_deposit<4, 8, 4, 2, 1, 0>(c, a);  // 32x16x8, 32 KB
@@ -307,8 +308,8 @@ int launch_fine_deposit(cube_ctx* c, const DepArgs& a) {
 int launch_coarse_deposit(cube_ctx* c, const DepArgs& a) {
   int shape = c->opt_dep_coarse;
   if (shape < 0) {
-    const int nb = default_bricks(c, 8, 8, 8);
-    shape = nb < 152 ? 3 : (nb < 3 * 152 ? 2 : 0);
+    const int64_t nb = default_bricks(c, 8, 8, 8);
+    shape = nb < sm_count() ? 3 : (nb < 3 * sm_count() ? 2 : 0);
   }
   switch (shape) {
     case 1: return launch_deposit<1, 16, 8, 8, 1, 1>(c, a);

@@ -97,7 +97,10 @@ int cudaGraphExecDestroy(ptr x) { return 0; }
 int cudaSetDevice(int d) { return 0; }
 int cudaGetDevice(int* d) { return *d = 0, 0; }
 int cudaGetDeviceCount(int* n) { return *n = 1, 0; }
-int cudaDeviceGetAttribute(int* v, int a, int d) { return *v = 152, 0; }
+int cudaDeviceGetAttribute(int* v, int a, int d) { /* multiprocessors */
+  const char* n = getenv("STREAM_SMS");
+  return *v = n ? atoi(n) : 152, 0;
+}
 int cudaFuncGetAttributes(void* a, const void* f) { return memset(a, 0, 128), 0; }
 int cudaFuncSetAttribute(const void* f, int a, int v) { return 0; }
 int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int b, size_t s, unsigned fl) {

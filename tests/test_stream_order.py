@@ -61,9 +61,9 @@ class Ops:
         return b[3].get(a[1], 0) >= a[2]
 
 
-def run(standin, tmp_path, lib, script):
+def run(standin, tmp_path, lib, script, **env):
     log = tmp_path / "log"
-    env = dict(os.environ, LD_PRELOAD=str(standin), STREAM_LOG=str(log), PYTHONPATH=ROOT)
+    env = dict(os.environ, LD_PRELOAD=str(standin), STREAM_LOG=str(log), PYTHONPATH=ROOT, **env)
     r = subprocess.run([sys.executable, "-c", script], env=env, cwd=ROOT, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr
     return Ops(log.read_text())
@@ -176,3 +176,16 @@ def test_default_brick_can_be_chosen_again(standin, tmp_path, built_lib, level):
     o = run(standin, tmp_path, built_lib, BRICKS % (level.upper(), level, level.upper()))
     names = [k[0] for k in o.find("k_deposit")]
     assert len(names) == 3 and names[0] == names[2] != names[1]
+
+
+@pytest.mark.parametrize("level,fewest", [("fine", (8, 4, 4)), ("coarse", (8, 8, 8))])
+def test_default_brick_goes_by_multiprocessors(standin, tmp_path, built_lib, level, fewest):
+    """The smallest bricks while the default ones are fewer than the device's
+    multiprocessors, whatever their number."""
+    bricks = 1
+    for b in fewest:
+        bricks *= 16 // b
+    script = BRICKS % (level.upper(), level, level.upper())
+    first = [run(standin, tmp_path, built_lib, script, STREAM_SMS=str(n)).find("k_deposit")[0][0]
+             for n in (152, bricks + 1, bricks)]
+    assert first[0] == first[1] != first[2]
