@@ -408,8 +408,6 @@ struct KickArgs {
   const void* vp_in;
   void* vp_out;            // may equal vp_in (fine kick updates in place)
   const int32_t* pcell;
-  const int32_t* rhoc;     // staged kernels: cell counts and starts
-  const int64_t* cstart;
   const float* vfield;
   const float* f[3];
   const unsigned* f2;      // bits of the maximum of force^2 over these meshes, or NaN
@@ -1001,8 +999,6 @@ int cube_fine_kick_impl(cube_ctx* c, float a_mid, float dt, bool with_pp) {
   k.vp_in = c->vp[c->cur];
   k.vp_out = c->vp[c->cur];
   k.pcell = c->pcell[c->cur];
-  k.rhoc = c->rhoc[c->cur];
-  k.cstart = c->cstart[c->cur];
   k.vfield = c->vfield[c->cur];
   for (int d = 0; d < 3; d++) k.f[d] = c->force_f[d];
   k.f2 = c->f2_kick;
