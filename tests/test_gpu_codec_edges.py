@@ -45,3 +45,36 @@ def test_zero_kick_codes(izipv):
         direct, table = g.codec_check(s, v)
         np.testing.assert_array_equal(direct, table)
     g.close()
+
+
+@pytest.mark.parametrize("izipv", [1, 2])
+@pytest.mark.parametrize("fused", [False, True])
+def test_idle_particles_keep_their_codes(izipv, fused):
+    """Particles alone in their neighbourhood take their code from the table of
+    zero kicks: every code through it, in PP's own kick and in the fine kick of
+    a fused step without motion, against decode and encode in FP64."""
+    from cafproject_gb300 import cube as C
+
+    lim = 1 << (8 * izipv - 1)
+    p = P.CubeParams(nc=28, nnt=1, izipv=izipv, pp_on=True, rsoft=0.1)
+    n = p.nc ** 3  # one particle in the middle of every coarse cell
+    codes = np.resize(np.arange(-lim, lim), 3 * n)
+    assert 3 * n >= 2 * lim
+    nvm1 = np.float32(2 * lim - 1)
+    t = np.tan(np.float32(np.float32(PI_F * codes.astype(np.float32)) / nvm1).astype(np.float64)).astype(np.float32)
+    g = C.CubeGPU(p)
+    for s in np.float32([1e-30, 0.037, 12.0]):
+        c = synth.vcoef(s)
+        want = np.rint(np.float64(nvm1) * np.arctan(c * (t.astype(np.float64) / c)) / np.float64(PI_F)).astype(np.int64)
+        g.upload(np.zeros((n, 3), np.int8 if p.izipx == 1 else np.int16),
+                 codes.reshape(n, 3).astype(np.int8 if izipv == 1 else np.int16), np.arange(n, dtype=np.int32),
+                 np.ones(n, np.int32), np.zeros((n, 3), np.float32))
+        g.set_sigma(s, s)
+        g.set_option(C.OPT_PP_FILTER, 2)
+        if fused:
+            st = g.pp_particle_mesh(0.4, 0.0)[0]
+        else:
+            st = g.ext_pp_force(0.4, 0.02)
+        assert st["npairs"] == n  # each particle its own entry alone: none is active
+        np.testing.assert_array_equal(g.download()["vp"].reshape(-1), want)
+    g.close()
