@@ -134,6 +134,35 @@ def test_fast_division_is_exact():
             assert fdiv(n, d, m, l) == n // d, (n, d)
 
 
+def test_force_maxima_pair_index():
+    # the maxima pass walks a padded mesh as a flat array of value pairs and
+    # takes a pair's place in its row from the low and the high 32 bits of its
+    # index (cube_pm.cu, k_f2max), beyond 2^32 pairs too (n > 2046)
+    rng = np.random.default_rng(1)
+    for n in (64, 1024, 2046, 2048, 4096, 16384, 65536):
+        row = n // 2 + 1
+        wrap = (1 << 32) % row
+        pairs = row * n * n
+        ks = [0, row - 2, row - 1, row, pairs - 2, (1 << 32) - 2, 1 << 32, (1 << 32) + 2 * row]
+        for k in ks + [int(k) for k in rng.integers(0, pairs, 2000)]:
+            if k >= pairs:
+                continue
+            r = (k & 0xFFFFFFFF) % row
+            if k >> 32:
+                t = (k >> 32) * wrap
+                assert r + t < 1 << 32  # no carry is lost
+                r = (r + t) % row
+            assert r == k % row
+
+
+def test_bench_counts_the_unconditional_launches():
+    import bench
+    p = P.WORKLOADS["cdm512"]()
+    # re-sort: destinations, ranks 3, scan 3, place and means 3, scatter, sums;
+    # PP: filter 3, scan 3, levels 5, kick; fine 4; coarse 4; tables
+    assert bench.gpu_launches(p, 1, conditional=False) == 12 + 12 + 4 + 4 + 1
+
+
 def test_sim_header_matches_reference_layout():
     # sim_header (parameters.f90:136-160) in Fortran stream I/O: 17 int64 then 22 real(4)
     from cafproject_gb300.cube import SimHeader

@@ -57,3 +57,33 @@ def test_boxes_evolve(serial):
         assert hs[4][i]["vmax"][0] > hs[0][i]["vmax"][0] > 0  # growth of structure
         assert hs[4][i]["f2_max_fine"] > 0 and hs[4][i]["npairs"] > 0
         assert ss[i]["rhoc"].sum() == ss[i]["xp"].shape[0]
+
+
+def test_eager_calls_between_graph_steps(serial):
+    """Calls on a box's own context between captured steps may replace both of
+    its code tables; the next step's are those of its state again."""
+    from cafproject_gb300 import batch as B
+    from cafproject_gb300 import cube as C
+    hs, ss, _, _ = serial
+    b = B.Batch(boxes(), z_init=19.0, mode=0)
+    b.set_schedule(0.0, 50)
+    for n in (1, 1, 2, 1):
+        b.step(n)
+        done = b.time()["steps_done"]
+        for i in range(b.nbox):
+            g = b.box(i)
+            sigma = float(g.get_sigma()[0])
+            for s in (0.5 * sigma, 3.0 * sigma)[:1 + done % 2]:
+                direct, table = g.codec_check(s, np.linspace(-4 * s, 4 * s, 33))
+                assert np.array_equal(direct, table)
+            g.get_field(C.FIELD_FORCE_C)
+    hist = [b.history(k) for k in range(5)]
+    states = [b.box(i).download() for i in range(b.nbox)]
+    b.close()
+    for k in range(5):
+        for i in range(4):
+            for key in ("sigma_vi_new", "f2_max_fine", "f2_max_coarse", "f2_max_pp", "npairs", "vmax"):
+                assert hs[k][i][key] == hist[k][i][key], (k, i, key)
+    for i in range(4):
+        for key in ("xp", "vp", "pid", "rhoc", "vfield"):
+            assert np.array_equal(ss[i][key], states[i][key]), (i, key)

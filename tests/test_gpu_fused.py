@@ -40,6 +40,39 @@ def test_fused_pp_and_pm_match_the_two_calls():
     assert ta[-1][2] > 0  # pairs were found
 
 
+@pytest.mark.parametrize("nc", [24, 40])
+@pytest.mark.parametrize("pp_on", [False, True])
+def test_coarse_forces_beside_or_behind_the_fine_ones(nc, pp_on):
+    # with the phase timers on, the coarse chain follows the fine one on the
+    # context's stream instead of running beside it: the same state and maxima
+    from cafproject_gb300 import cube as C
+    from cafproject_gb300 import params as P
+    from cafproject_gb300 import synth
+    p = P.small(nc=nc, nnt=2, pp_on=pp_on)
+    st = synth.random_state(p, mean_per_cell=4, seed=nc, vsig=0.03, clump=10)
+    outs = []
+    for behind in (False, True):
+        g = C.CubeGPU(p)
+        try:
+            g.upload(st["xp"], st["vp"], st["pid"], st["rhoc"], st["vfield"])
+            g.set_sigma(st["sigma_vi"])
+            g.timing(behind)
+            stats = []
+            for _ in range(3):
+                g.update_x(20.0, 30.0, st["vz_max"])
+                pm = g.pp_particle_mesh(0.4, 0.02)[1] if pp_on else g.particle_mesh(0.4, 0.02)
+                stats.append((pm["f2_max_fine"], pm["f2_max_coarse"], pm["testrhof"], pm["testrhoc"],
+                              tuple(pm["vmax"])))
+            outs.append((g.download(), stats, g.get_field(C.FIELD_RHO_C), g.get_field(C.FIELD_FORCE_C)))
+        finally:
+            g.close()
+    a, b = outs
+    assert a[1] == b[1]
+    for key in a[0]:
+        assert np.array_equal(a[0][key], b[0][key]), key
+    assert np.array_equal(a[2], b[2]) and np.array_equal(a[3], b[3])
+
+
 def test_upload_rejects_inconsistent_counts():
     # the counts are checked on the device after the copies: a sum that is
     # not nplocal, or a negative count, is an error and leaves no state; a
