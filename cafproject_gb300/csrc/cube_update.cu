@@ -28,6 +28,7 @@ constexpr int NOFF = 27;  // the counting path: a cell's neighbours and itself
 struct UpdArgs {
   Geo g;
   int64_t np, ncells;
+  int64_t np_max;     // what the particle arrays hold
   float dt_mid;
   int nlayer;
   const void* xp;
@@ -897,9 +898,11 @@ __device__ __forceinline__ void recode_rest(const UpdArgs& a, RecodeQueue& rq) {
   if ((int)(threadIdx.x & 31) < rq.n) recode_entry(a, rq.q[threadIdx.x & 31]);
 }
 
-// rank r of a landing in D checked before anything is written
+// rank r of a landing in D checked before anything is written.  (Extra copies
+// may bring the new count above np_max: the eager path's host has looked before
+// it comes here, a captured step has not.)
 __device__ __forceinline__ bool rank_ok(const UpdArgs& a, int32_t D, uint32_t r) {
-  if (D >= 0 && (int64_t)D < a.ncells && r < (uint32_t)a.cnt_new[D]) return true;
+  if (D >= 0 && (int64_t)D < a.ncells && r < (uint32_t)a.cnt_new[D] && a.cstart_new[D] + r < a.np_max) return true;
   atomicOr(&a.st->flags, 2);  // rank not assigned: never write outside the new arrays
   return false;
 }
@@ -1196,6 +1199,7 @@ static int update_x_graph(cube_ctx* c) {
   a.g = g;
   a.np = c->np;
   a.ncells = c->ncells;
+  a.np_max = c->p.np_max;
   a.dt_mid = 0.f;
   a.nlayer = 1;
   a.sd = c->sd;
@@ -1284,6 +1288,7 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
   a.g = g;
   a.np = c->np;
   a.ncells = c->ncells;
+  a.np_max = c->p.np_max;
   a.dt_mid = dt_mid;
   a.nlayer = nlayer;
   a.xp = c->xp[k];
@@ -1432,7 +1437,7 @@ int cube_update_x_impl(cube_ctx* c, float dt_old, float dt, float vz_max, cube_s
       CUBE_CUDA(c, cudaMemsetAsync(&c->dstats->flags, 0, sizeof(int), c->stream));
       path = WALK;
       if ((r = walk()) || (r = scan())) return r;
-    } else {
+    } else if (np_new <= c->p.np_max) {
       cube_phase_begin(c, PH_UPD_PLACE);
       k_sort_place<<<cube_grid(np_new, 256), 256, 0, c->stream>>>(a, vals, np_new);
       cube_phase_end(c, PH_UPD_PLACE);

@@ -101,7 +101,10 @@ int cudaDeviceGetAttribute(int* v, int a, int d) { /* multiprocessors */
   const char* n = getenv("STREAM_SMS");
   return *v = n ? atoi(n) : 152, 0;
 }
-int cudaFuncGetAttributes(void* a, const void* f) { return memset(a, 0, 128), 0; }
+int cudaFuncGetAttributes(void* a, const void* f) { /* sizes, then threads, registers, PTX and binary version */
+  const int v[4] = {1024, 32, 103, 103};
+  return memset(a, 0, 128), memcpy((char*)a + 3 * sizeof(size_t), v, sizeof v), 0;
+}
 int cudaFuncSetAttribute(const void* f, int a, int v) { return 0; }
 int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int b, size_t s, unsigned fl) {
   return *n = 1, 0;

@@ -189,3 +189,22 @@ def test_default_brick_goes_by_multiprocessors(standin, tmp_path, built_lib, lev
     first = [run(standin, tmp_path, built_lib, script, STREAM_SMS=str(n)).find("k_deposit")[0][0]
              for n in (152, bricks + 1, bricks)]
     assert first[0] == first[1] != first[2]
+
+
+OVERFULL = """
+from cafproject_gb300 import cube as C
+from cafproject_gb300 import batch as B
+g = C.CubeGPU(B.box_params(32, pp_on=False))
+g.ic_zeldovich(19.0, seed=1)
+g.set_option(C.OPT_RANK_WALK, 2)
+try:  # the stand-in's count of the new state is far above np_max
+    g.update_x(1.0, 1.0, 0.1)
+    raise SystemExit("an overfull state went through")
+except C.CubeError as e:
+    assert "np_max" in str(e), e
+"""
+
+
+def test_overfull_state_is_refused_before_its_order_is_written(standin, tmp_path, built_lib):
+    o = run(standin, tmp_path, built_lib, OVERFULL)
+    assert o.find("k_sort_keys") and not o.find("k_sort_place") and not o.find("k_sort_gather")
