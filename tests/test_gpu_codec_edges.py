@@ -57,7 +57,7 @@ def test_idle_particles_keep_their_codes(izipv, fused):
 
     lim = 1 << (8 * izipv - 1)
     p = P.CubeParams(nc=28, nnt=1, izipv=izipv, pp_on=True, rsoft=0.1)
-    n = p.nc ** 3  # one particle in the middle of every coarse cell
+    n = p.nc ** 3  # one particle to a coarse cell
     codes = np.resize(np.arange(-lim, lim), 3 * n)
     assert 3 * n >= 2 * lim
     nvm1 = np.float32(2 * lim - 1)

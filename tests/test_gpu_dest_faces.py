@@ -64,7 +64,7 @@ def test_one_particle_lands_in_two_tiles(room, path):
     rhoc = np.zeros(p.nc ** 3, np.int32)
     rhoc[11] = n  # tile 0, cell (12, 1, 1): the last along x
     xp, vp = np.zeros((n, 3), p.xdtype), np.zeros((n, 3), p.vdtype)
-    xp[7, 0], vp[7, 0] = 127, code
+    xp[7, 0], vp[7, 0] = -1, code  # the last of the 256 positions in a cell
     st = dict(xp=xp, vp=vp, pid=np.arange(1, n + 1, dtype=np.int32), rhoc=rhoc,
               vfield=np.zeros((p.nc ** 3, 3), np.float32))
     g = C.CubeGPU(p)
