@@ -693,13 +693,16 @@ __global__ void __launch_bounds__(256, 4) k_kick(KickArgs a) {
 }
 
 // The blocks that an SM holds, once: every block ends in its warps' part-filled
-// queues, which cost as much as full ones, so fewer blocks are better (256^3
-// particles, coarse: 0.96 ms with 4 a SM, 1.13 with 16, 2.05 with a particle a
-// thread; 108^3: 0.18, 0.26, 0.31).  Above 2^26 particles the queues' share is
-// small and the balance of more blocks gives more (512^3, fine: 13.3 against 12.9).
+// queues, which cost as much as full ones, so fewer blocks are better.  Above 2^25
+// particles the queues' share is small and the balance of more blocks gives more.
+// Fine / coarse kick in ms with 4 and with 16 blocks an SM, uniform states (at
+// z = 3 the same within 1 %): 256^3 particles 0.541 / 0.463 and 0.559 / 0.468,
+// 320^3 1.042 / 0.898 and 1.064 / 0.895, 352^3 1.384 / 1.191 and 1.402 / 1.163,
+// 384^3 1.818 / 1.570 and 1.814 / 1.532, 448^3 2.856 / 2.482 and 2.847 / 2.412,
+// 512^3 4.320 / 3.696 and 4.286 / 3.595.
 template <bool kFine>
 void launch_kick(cube_ctx* c, const KickArgs& k) {
-  k_kick<kFine><<<cube_grid(k.np, 256, k.np > (int64_t)1 << 26 ? 16 : 4), 256, 0, c->stream>>>(k);
+  k_kick<kFine><<<cube_grid(k.np, 256, k.np > (int64_t)1 << 25 ? 16 : 4), 256, 0, c->stream>>>(k);
 }
 
 }  // namespace
