@@ -797,9 +797,9 @@ int cube_coarse_density_impl(cube_ctx* c, cube_stats* st, bool accumulate = fals
 int cube_fine_forces_impl(cube_ctx* c, cube_stats* st, bool fresh = false);
 // Fused steps: the coarse forces beside the fine ones, on the auxiliary stream.
 // On a small box they fill a chip that the fine chain leaves idle, on a large one
-// the ends of its passes (one after the other -> beside, PP queued behind the fine
-// chain: 48^3 leg 1.53 -> 1.36 ms, 64^3 1.58 -> 1.44, 108^3 3.63 -> 3.41, 208^3
-// 19.28 -> 19.09, 256^3 late 36.4 -> 36.0, 512^3 177 -> 175).  The coarse
+// the ends of its passes (one after the other -> beside, legs of two to four steps:
+// 48^3 particles 1.45 -> 1.27 ms, 64^3 1.47 -> 1.29, 108^3 3.54 -> 3.35, 208^3
+// 19.70 -> 19.56; 256^3 late and 512^3 the same within 0.3 %).  The coarse
 // transforms then have a work area of their own; above 2^24 coarse cells, whose
 // area would be gigabytes, they stay behind the fine ones.  cube_forces_fork comes
 // before the fine forces, cube_coarse_beside after them, cube_forces_join before

@@ -407,9 +407,11 @@ __device__ bool pp_block(const PPArgs& a, const int C0[3], const int B[3], PPSme
   // walks the block's particles [i0, i1) in bin order (slots differ from one
   // staging to the next; bin order does not).  From PP_BIN_ORDER staged
   // particles a sparse block too takes them in bin order: neighbours' lists are
-  // about as long, so fewer lanes wait (256^3 particles at z = 0: PP 9.76 ->
-  // 9.45 ms; at 500 the bin search cost blocks of a state at z = 5 more than
-  // that, 1.05 -> 1.11 ms).
+  // about as long, so fewer lanes wait, and below that the bin search costs more.
+  // PP in ms from 500, 1000, 1500 staged particles on: 96^3 particles at z = 0.1
+  // 2.16, 2.17, 2.26; 128^3 2.58, 2.59, 2.67; 192^3 4.65, 4.69, 4.84, at z = 1
+  // 1.91, 1.92, 2.03; 256^3 at z = 0.1 9.48, 9.57, 9.98, but at z = 3 2.29, 2.22,
+  // 2.22.
   const bool crowded = 4 * nst >= NF;
   const bool by_bin = crowded || nparts > 1 || nst >= PP_BIN_ORDER;
   const int RX = 4 * B[1], nrc = RX * 4 * B[2];

@@ -610,8 +610,8 @@ extern "C" int cube_arith_check(cube_ctx* c, int64_t* mismatches) {
 // cudaFree synchronises the whole device, which stalls every other stream.
 // The array holds CUBE_CODEC_STATIC_MAX doubles of input, two
 // CUBE_CODEC_STATIC_MAX int32 outputs and one set of codec tables for the
-// largest velocity format (izipv = 2: 65536 decode values as double and as a
-// float pair, 32769 encode bounds), 1.25 MiB + 256 KiB in all.  The tables
+// largest velocity format (izipv = 2: 65536 decode values, 32769 float pairs in
+// room for 65536, 32769 encode bounds), 1.25 MiB + 256 KiB in all.  The tables
 // are rebuilt by every call for its sigma, so the context's own two codec
 // slots (the step's sigma_vi and sigma_vi_new) are never touched.  Nothing in
 // the array needs to start at zero: each call writes every value it reads.
